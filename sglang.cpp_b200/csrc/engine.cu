@@ -194,6 +194,19 @@ bool fold_supported(const b200_engine* e, int phase, int T) {
     return e->ssq != nullptr && phase == B200_PHASE_DECODE && T <= b200_engine::kSsqStride;
 }
 
+// Can this step run on the projections for a handful of rows, which carry the norms, the residual and the head operations
+// themselves?  A dense, unsharded model; where the norms of the other path read the sum before it is rounded, only if that
+// path would be the folded one, which does not either.  Every CTA normalises x for itself: beside the weights of a wide
+// model's projections that is too much (one layer of hidden 4096, 4 requests, in a step: 173 us against 120).
+bool narrow_supported(const b200_engine* e, int phase, int T) {
+    const int H = e->m.hidden_size, D = e->m.head_dim;
+    auto takes = [&](int N, int K, int epilogue) { return narrow_gemm_takes(nullptr, nullptr, T, N, K, K, epilogue); };
+    return e->use_fold && !e->use_chain && phase == B200_PHASE_DECODE && e->c.tp_size == 1 && e->m.num_experts == 0 && D == 128 &&
+           H <= 2048 && (e->m.fused_residual == 0 || e->ssq != nullptr) && takes(e->qkv_dim, H, B200_EPILOGUE_NONE) &&
+           takes(H, e->hq * D, B200_EPILOGUE_NONE) && takes(2 * e->inter, H, B200_EPILOGUE_SWIGLU) &&
+           takes(H, e->inter, B200_EPILOGUE_NONE);
+}
+
 // Rebuilds the folded weight copies after a weight was loaded.  Enqueued on the engine's stream, never
 // inside a graph capture (the callers run it first).
 int ensure_folded(b200_engine* e) {
@@ -228,7 +241,7 @@ bool logits_f32(const b200_engine* e) { return e->stack && stack_dtype(e) == B20
 int output_head(b200_engine* e, const void* rows, int count) {
     if (e->stack) return layer_stack_head(e, e->logits, rows, count);
     return launch_linear(e->logits, rows, e->lm_head, nullptr, count, e->m.vocab_size, e->m.hidden_size,
-                         e->m.hidden_size, B200_EPILOGUE_NONE, e->status, e->stream);
+                         e->m.hidden_size, B200_EPILOGUE_NONE, e->status, e->stream, nullptr, 0.f, e->use_fold);
 }
 
 // Last part of every step: each request's last row, the head, token selection and write-back.
@@ -300,7 +313,8 @@ int enqueue_forward(b200_engine* e, int phase, int B, int Bp, int T, int max_ext
     const uint64_t launches_before = kernel_launch_count();
     const int32_t* meta_table_idx = e->meta_dev;
     const int32_t* meta_qo = e->meta_dev + 2 * Bp;
-    const bool fold = fold_supported(e, phase, T);
+    const bool narrow = narrow_supported(e, phase, T);
+    const bool fold = narrow || fold_supported(e, phase, T);
     // The residual stream starts at zero, so the first fused add+norm leaves residual = embedding
     // (what the reference's layer 0 does with `residual = x`).  With the norms folded into the GEMMs
     // the embedding is written into the residual directly.
@@ -319,8 +333,8 @@ int enqueue_forward(b200_engine* e, int phase, int B, int Bp, int T, int max_ext
     // of the step can then rely on seq_lens / positions / out_loc being complete even in code it
     // runs ahead of griddepcontrol.wait (a kernel can only start after the embedding has).
     if (fold)
-        B200_TRY(launch_embedding(e->residual, e->embed, e->input_ids, T, hidden, m.vocab_size, e->status, s, e->ssq,
-                                  2 * m.num_layers + 1, b200_engine::kSsqStride));
+        B200_TRY(launch_embedding(e->residual, e->embed, e->input_ids, T, hidden, m.vocab_size, e->status, s,
+                                  narrow ? nullptr : e->ssq, 2 * m.num_layers + 1, b200_engine::kSsqStride));
     else
         B200_TRY(launch_embedding(e->x, e->embed, e->input_ids, T, hidden, m.vocab_size, e->status, s));
     set_pdl_launches(e->use_pdl && !(e->profile_attention && !e->capturing));
@@ -361,6 +375,18 @@ int enqueue_forward(b200_engine* e, int phase, int B, int Bp, int T, int max_ext
         return launch_fused_add_rmsnorm(e->x, e->residual, w, T, hidden, m.rms_norm_eps, round_first, s);
     };
     const int epi = m.hidden_act == 1 ? B200_EPILOGUE_GEGLU : B200_EPILOGUE_SWIGLU;
+    // Events around the attention launch of a layer, where they are asked for.
+    auto time_attention = [&](int l, int end) -> int {
+        if (!e->profile_attention || e->capturing) return B200_OK;
+        while (static_cast<int>(e->prof_events.size()) < 2 * m.num_layers) {
+            cudaEvent_t ev = nullptr;
+            B200_CHECK_CUDA(cudaEventCreate(&ev));
+            e->prof_events.push_back(ev);
+        }
+        B200_CHECK_CUDA(cudaEventRecord(e->prof_events[2 * l + end], s));
+        if (end) e->prof_pairs_recorded = l + 1;
+        return B200_OK;
+    };
     // The head epilogue of the qkv projection wants the split-K form of the small-batch kernel; beyond
     // two exchange rounds (128 tokens) the separate kernel is the faster of the two, and on a sharded
     // engine (few heads per rank) it is no gain: Llama-3-8B at batch 128 ran 7.21 against 7.44 ms with it
@@ -446,7 +472,62 @@ int enqueue_forward(b200_engine* e, int phase, int B, int Bp, int T, int max_ext
         }
     }
 
-    for (int l = 0; l < (fold ? m.num_layers : 0); ++l) {
+    auto fill_heads = [&](HeadEpilogue& he, int l) {
+        LayerWeights& L = e->layers[l];
+        he.q_norm_w = L.q_norm;
+        he.k_norm_w = L.k_norm;
+        he.cos_t = e->rope_cos;
+        he.sin_t = e->rope_sin;
+        he.positions = e->positions;
+        he.out_loc = e->out_loc;
+        __nv_bfloat16* k_cache = e->kv_cache + static_cast<int64_t>(l) * e->num_slots * e->hkv * d;
+        he.k_cache = k_cache;
+        he.v_cache = k_cache + static_cast<int64_t>(m.num_layers) * e->num_slots * e->hkv * d;
+        he.q_heads = e->hq;
+        he.kv_heads = e->hkv;
+        he.max_pos = m.max_position;
+        he.num_slots = e->num_slots;
+        he.eps = m.rms_norm_eps;
+    };
+    // (B200_FOLD_NORM=0, the path of one kernel per operator, keeps to one kind of projection)
+    auto linear = [&](void* y, const void* x, const void* w, const void* bias, int N, int K, int epilogue) {
+        return launch_linear(y, x, w, bias, T, N, K, K, epilogue, e->status, s, nullptr, 0.f, e->use_fold);
+    };
+    // Head norms, rotation and K/V store behind a plain projection.
+    auto norm_and_store = [&](const HeadEpilogue& he) -> int {
+        return launch_qknorm_rope_store(e->qkv, he.q_norm_w, he.k_norm_w, he.cos_t, he.sin_t, e->positions, e->out_loc, he.k_cache,
+                                        he.v_cache, T, e->hq, e->hkv, d, m.max_position, e->num_slots, m.rms_norm_eps, 0,
+                                        e->status, s);
+    };
+    for (int l = 0; l < (narrow ? m.num_layers : 0); ++l) {
+        LayerWeights& L = e->layers[l];
+        HeadEpilogue he;
+        fill_heads(he, l);
+        NarrowFusion from_residual, into_residual;
+        into_residual.residual = e->residual;
+        from_residual.eps = m.rms_norm_eps;
+        from_residual.norm_w = L.input_norm;
+        from_residual.heads = e->use_fold_heads ? &he : nullptr;
+        B200_TRY(launch_narrow_gemm(e->qkv, e->residual, L.qkv, L.qkv_bias, T, e->qkv_dim, hidden, hidden, B200_EPILOGUE_NONE,
+                                    e->status, s, &from_residual));
+        if (!e->use_fold_heads) B200_TRY(norm_and_store(he));
+        B200_TRY(time_attention(l, 0));
+        B200_TRY(launch_attention_decode(e->attn_out, e->qkv, e->qkv_dim, d, L.tmap_k, L.tmap_v, e->num_slots,
+                                         e->page_table, e->pt_cols, meta_table_idx, e->seq_lens, Bp, e->hq, e->hkv,
+                                         e->c.page_size, e->sm_scale, e->attn_ws, e->attn_ws_bytes, e->status, s,
+                                         e->kv_evict_first));
+        B200_TRY(time_attention(l, 1));
+        B200_TRY(launch_narrow_gemm(nullptr, e->attn_out, L.o, nullptr, T, hidden, e->hq * d, e->hq * d, B200_EPILOGUE_NONE,
+                                    e->status, s, &into_residual));
+        from_residual.norm_w = L.post_norm;
+        from_residual.heads = nullptr;
+        B200_TRY(launch_narrow_gemm(e->h, e->residual, L.gate_up, nullptr, T, 2 * e->inter, hidden, hidden, epi, e->status, s,
+                                    &from_residual));
+        B200_TRY(launch_narrow_gemm(nullptr, e->h, L.down, nullptr, T, hidden, e->inter, e->inter, B200_EPILOGUE_NONE,
+                                    e->status, s, &into_residual));
+    }
+
+    for (int l = 0; l < (fold && !narrow ? m.num_layers : 0); ++l) {
         LayerWeights& L = e->layers[l];
         unsigned long long* ssq_l = e->ssq + static_cast<int64_t>(2 * l) * b200_engine::kSsqStride;
         SkinnyFusion normed, into_residual;
@@ -460,19 +541,7 @@ int enqueue_forward(b200_engine* e, int phase, int B, int Bp, int T, int max_ext
         if (heads_in_qkv) {
             // ... and the QK-norm, the rotation and the K/V store ride in the qkv projection's epilogue
             HeadEpilogue he;
-            he.q_norm_w = L.q_norm;
-            he.k_norm_w = L.k_norm;
-            he.cos_t = e->rope_cos;
-            he.sin_t = e->rope_sin;
-            he.positions = e->positions;
-            he.out_loc = e->out_loc;
-            he.k_cache = k_cache;
-            he.v_cache = v_cache;
-            he.q_heads = e->hq;
-            he.kv_heads = e->hkv;
-            he.max_pos = m.max_position;
-            he.num_slots = e->num_slots;
-            he.eps = m.rms_norm_eps;
+            fill_heads(he, l);
             normed.heads = &he;
             B200_TRY(launch_linear(e->qkv, e->residual, L.qkv_folded, L.qkv_bias, T, e->qkv_dim, hidden, hidden,
                                    B200_EPILOGUE_NONE, e->status, s, &normed));
@@ -484,23 +553,12 @@ int enqueue_forward(b200_engine* e, int phase, int B, int Bp, int T, int max_ext
                                               e->out_loc, k_cache, v_cache, T, e->hq, e->hkv, d, m.max_position,
                                               e->num_slots, m.rms_norm_eps, 0, e->status, s));
         }
-        const bool timed = e->profile_attention && !e->capturing;
-        if (timed) {
-            while (static_cast<int>(e->prof_events.size()) < 2 * m.num_layers) {
-                cudaEvent_t ev = nullptr;
-                B200_CHECK_CUDA(cudaEventCreate(&ev));
-                e->prof_events.push_back(ev);
-            }
-            B200_CHECK_CUDA(cudaEventRecord(e->prof_events[2 * l], s));
-        }
+        B200_TRY(time_attention(l, 0));
         B200_TRY(launch_attention_decode(e->attn_out, e->qkv, e->qkv_dim, d, L.tmap_k, L.tmap_v, e->num_slots,
                                          e->page_table, e->pt_cols, meta_table_idx, e->seq_lens, Bp, e->hq, e->hkv,
                                          e->c.page_size, e->sm_scale, e->attn_ws, e->attn_ws_bytes, e->status, s,
                                          e->kv_evict_first));
-        if (timed) {
-            B200_CHECK_CUDA(cudaEventRecord(e->prof_events[2 * l + 1], s));
-            e->prof_pairs_recorded = l + 1;
-        }
+        B200_TRY(time_attention(l, 1));
         into_residual.ssq_out = ssq_l + b200_engine::kSsqStride;
         B200_TRY(launch_linear(nullptr, e->attn_out, L.o, nullptr, T, hidden, e->hq * d, e->hq * d,
                                B200_EPILOGUE_NONE, e->status, s, &into_residual));
@@ -515,76 +573,44 @@ int enqueue_forward(b200_engine* e, int phase, int B, int Bp, int T, int max_ext
     for (int l = 0; l < (chain || fold ? 0 : m.num_layers); ++l) {
         LayerWeights& L = e->layers[l];
         B200_TRY(add_norm(L.input_norm));
-        __nv_bfloat16* k_cache = e->kv_cache + static_cast<int64_t>(l) * e->num_slots * e->hkv * d;
-        __nv_bfloat16* v_cache = k_cache + static_cast<int64_t>(m.num_layers) * e->num_slots * e->hkv * d;
+        HeadEpilogue he;
+        fill_heads(he, l);
         if (heads_in_qkv) {
             // (sharded and MoE engines, short prefill batches: the head epilogue alone, on normalised rows)
-            HeadEpilogue he;
-            he.q_norm_w = L.q_norm;
-            he.k_norm_w = L.k_norm;
-            he.cos_t = e->rope_cos;
-            he.sin_t = e->rope_sin;
-            he.positions = e->positions;
-            he.out_loc = e->out_loc;
-            he.k_cache = k_cache;
-            he.v_cache = v_cache;
-            he.q_heads = e->hq;
-            he.kv_heads = e->hkv;
-            he.max_pos = m.max_position;
-            he.num_slots = e->num_slots;
-            he.eps = m.rms_norm_eps;
             SkinnyFusion with_heads;
             with_heads.heads = &he;
             B200_TRY(launch_linear(e->qkv, e->x, L.qkv, L.qkv_bias, T, e->qkv_dim, hidden, hidden, B200_EPILOGUE_NONE,
                                    e->status, s, &with_heads));
         } else {
-            B200_TRY(launch_linear(e->qkv, e->x, L.qkv, L.qkv_bias, T, e->qkv_dim, hidden, hidden,
-                                   B200_EPILOGUE_NONE, e->status, s));
-            B200_TRY(launch_qknorm_rope_store(e->qkv, L.q_norm, L.k_norm, e->rope_cos, e->rope_sin,
-                                              e->positions, e->out_loc, k_cache, v_cache, T, e->hq, e->hkv,
-                                              d, m.max_position, e->num_slots, m.rms_norm_eps, 0, e->status, s));
+            B200_TRY(linear(e->qkv, e->x, L.qkv, L.qkv_bias, e->qkv_dim, hidden, B200_EPILOGUE_NONE));
+            B200_TRY(norm_and_store(he));
         }
-        const bool timed = e->profile_attention && !e->capturing;
-        if (timed) {
-            while (static_cast<int>(e->prof_events.size()) < 2 * m.num_layers) {
-                cudaEvent_t ev = nullptr;
-                B200_CHECK_CUDA(cudaEventCreate(&ev));
-                e->prof_events.push_back(ev);
-            }
-            B200_CHECK_CUDA(cudaEventRecord(e->prof_events[2 * l], s));
-        }
+        B200_TRY(time_attention(l, 0));
         if (phase == B200_PHASE_DECODE) {
             B200_TRY(launch_attention_decode(e->attn_out, e->qkv, e->qkv_dim, d, L.tmap_k, L.tmap_v,
                                              e->num_slots, e->page_table, e->pt_cols, meta_table_idx,
                                              e->seq_lens, Bp, e->hq, e->hkv, e->c.page_size, e->sm_scale,
                                              e->attn_ws, e->attn_ws_bytes, e->status, s, e->kv_evict_first));
         } else {
-            B200_TRY(launch_attention_prefill(e->attn_out, e->qkv, e->qkv_dim, d, k_cache, v_cache,
+            B200_TRY(launch_attention_prefill(e->attn_out, e->qkv, e->qkv_dim, d, he.k_cache, he.v_cache,
                                               e->num_slots, e->page_table, e->pt_cols, meta_table_idx,
                                               e->seq_lens, meta_qo, Bp, max_extend, e->hq, e->hkv,
                                               e->c.page_size, e->sm_scale, e->status, s));
         }
-        if (timed) {
-            B200_CHECK_CUDA(cudaEventRecord(e->prof_events[2 * l + 1], s));
-            e->prof_pairs_recorded = l + 1;
-        }
-        B200_TRY(launch_linear(proj_out(), e->attn_out, L.o, nullptr, T, hidden, e->hq * d, e->hq * d,
-                                   B200_EPILOGUE_NONE, e->status, s));
+        B200_TRY(time_attention(l, 1));
+        B200_TRY(linear(proj_out(), e->attn_out, L.o, nullptr, hidden, e->hq * d, B200_EPILOGUE_NONE));
         B200_TRY(add_norm(L.post_norm));
         if (m.num_experts > 0) {
             // MoEMLP::forward (src/models/utils.cc:82-91): router logits, then the expert layer.
-            B200_TRY(launch_linear(e->router_logits, e->x, L.router, nullptr, T, m.num_experts, hidden, hidden,
-                                   B200_EPILOGUE_NONE, e->status, s));
+            B200_TRY(linear(e->router_logits, e->x, L.router, nullptr, m.num_experts, hidden, B200_EPILOGUE_NONE));
             B200_TRY(launch_moe_forward(proj_out(), e->x, e->router_logits, L.experts_gate_up, L.experts_down, T,
                                         m.num_experts, m.num_experts_per_tok, hidden, e->moe_inter,
                                         m.norm_topk_prob, m.hidden_act == 1 ? 1 : 0, e->expert_begin,
                                         e->experts_local, e->moe_ws, e->status, s));
             continue;
         }
-        B200_TRY(launch_linear(e->h, e->x, L.gate_up, nullptr, T, 2 * e->inter, hidden, hidden, epi,
-                                   e->status, s));
-        B200_TRY(launch_linear(proj_out(), e->h, L.down, nullptr, T, hidden, e->inter, e->inter,
-                                   B200_EPILOGUE_NONE, e->status, s));
+        B200_TRY(linear(e->h, e->x, L.gate_up, nullptr, 2 * e->inter, hidden, epi));
+        B200_TRY(linear(proj_out(), e->h, L.down, nullptr, hidden, e->inter, B200_EPILOGUE_NONE));
     }
     if (fold)
         B200_TRY(launch_rmsnorm(e->x, e->residual, e->final_norm, T, hidden, m.rms_norm_eps, s));

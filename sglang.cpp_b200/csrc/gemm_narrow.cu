@@ -1,0 +1,381 @@
+// y = x W^T for a handful of rows (decode steps of a few requests): weights go from memory to registers.
+//
+// Such a call reads W once and computes next to nothing, and a decode step is a chain of them.  What bounds a small
+// one is not bandwidth but what happens between the end of the kernel before it and its own end, so that part is
+// kept short, and everything else is moved in front of it:
+//   * 16 rows of W per CTA and the whole of K, dealt to its warps: no exchange between CTAs.  A lane loads 16
+//     contiguous bytes of a row; which of the k of a 32-wide step these are does not matter, because x is loaded
+//     the same way, so the bytes are the operands of two m16n8k16 products as they are (weights as the left one,
+//     8 tokens as the right one).  No shared memory, no barrier before the sums meet.
+//   * the weights that fit in registers are requested before griddepcontrol.wait.  CTAs are small (8 warps, a few
+//     KB of shared memory), so those of the next kernels of the chain become resident beside the running one.
+//   * behind the wait: x (from L2), the products, one exchange through shared memory, the epilogue.
+// tcgen05 has no place here: its operands would have to pass through shared memory, and 128 x 64 tiles of W leave
+// most SMs without one.
+//
+// The rows of W of a CTA's tile are two groups of 8, g and g + 8 of the product: neighbours in plain projections, the
+// same features' gate and up rows, or the two halves of an attention head, so that what an epilogue has to bring
+// together is in one thread.  Head norms need the whole head: 8 CTAs of a cluster exchange sums of squares.
+//
+// One layer's projections of hidden 1024, one request (us; the split-K clusters of gemm_skinny.cu before): 4096 x 1024 3.5 (6.3),
+// 1024 x 2048 3.5 (5.9), 6144 x 1024 with SwiGLU 4.2 (8.8), 1024 x 3072 4.8 (6.9); their weights take 0.6 to 1.9 at the copy
+// bandwidth.  151936 x 1024: 47 (57), which is the bandwidth.
+//
+// "Normalised input": x is an un-normalised residual row.  Each CTA reads whole rows anyway, so it sums their squares
+// itself; the products run on bf16(x * weight of the norm), and the result is scaled by the row's 1 / rms.
+#include "common.cuh"
+#include "kernels.h"
+
+namespace b200 {
+namespace {
+
+constexpr int kSteps = 4;        // k-steps of 32 per register buffer
+constexpr int kTokenPitch = 20;  // floats: 16 features of a token, padded so that a warp's stores hit 32 banks
+constexpr int kHeadRanks = 8;    // CTAs that share an attention head
+enum Kind { kPlain, kResidual, kHeads };
+
+struct NarrowParams {
+    __nv_bfloat16* y;            // [M, y_pitch]
+    const __nv_bfloat16 *x, *w, *bias, *norm_w;
+    int M, n_out, n_rows, up_row_offset, steps, epilogue;
+    int64_t ldx, K, y_pitch;
+    float norm_eps, act_limit;
+    __nv_bfloat16* residual;
+    // attention heads (see HeadEpilogue)
+    const __nv_bfloat16 *q_norm_w, *k_norm_w;
+    const float *cos_t, *sin_t;
+    const int32_t *positions, *out_loc;
+    __nv_bfloat16 *k_cache, *v_cache;
+    int q_heads, kv_heads, max_pos;
+    long long num_slots;
+    float qk_eps;
+    int* status;
+};
+
+// Weights are read once: past L1.
+__device__ __forceinline__ uint4 load_weights(const uint4* p) {
+    uint4 v;
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void store_in_cluster(const float* mine, uint32_t rank, float v) {
+    uint32_t remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(mine)), "r"(rank));
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
+}
+
+__device__ float activate_pair(int epilogue, float g, float u, float limit) {
+    switch (epilogue) {
+        case B200_EPILOGUE_SWIGLU: return __fdividef(g, 1.0f + __expf(-g)) * u;
+        case B200_EPILOGUE_GEGLU_ERF: return 0.5f * g * (1.0f + erff(g * 0.70710678118654752f)) * u;
+        case B200_EPILOGUE_CLAMPED_SWIGLU: return clamped_swiglu<false>(g, u, limit);
+        default: return 0.5f * g * (1.0f + tanhf(0.7978845608f * (g + 0.044715f * g * g * g))) * u;
+    }
+}
+
+// BUFS register buffers of kSteps steps: with one, a warp's whole share of K is requested ahead of the wait.
+template <int KIND, bool NORM, int NT, int WARPS, int BUFS>
+__global__ void __launch_bounds__(WARPS * 32)
+narrow_gemm_kernel(const NarrowParams p) {
+    __shared__ float s_part[WARPS][NT * 8 * kTokenPitch];
+    __shared__ float s_ssq[WARPS][NT * 8];
+    __shared__ float s_head[kHeadRanks][NT * 8];
+    pdl_launch_dependents();
+    if (KIND == kHeads) cluster_arrive();   // (waited for before the first store to another CTA of the cluster)
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const bool gated = KIND == kPlain && p.up_row_offset > 0;
+    const int tile = static_cast<int>(blockIdx.x);
+    int row_a, row_b;
+    if (KIND == kHeads) {
+        row_a = (tile >> 3) * 128 + (tile & 7) * 8 + g;
+        row_b = row_a + 64;
+    } else if (gated) {
+        row_a = tile * 8 + g;
+        row_b = row_a + p.up_row_offset;
+    } else {
+        row_a = tile * 16 + g;
+        row_b = min(row_a + 8, p.n_rows - 1);   // (n_out may be an odd multiple of 8)
+    }
+    const uint4* wa = reinterpret_cast<const uint4*>(p.w + row_a * p.K) + t;
+    const uint4* wb = reinterpret_cast<const uint4*>(p.w + row_b * p.K) + t;
+    const int first = warp * p.steps / WARPS, last = (warp + 1) * p.steps / WARPS;
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    uint4 a[BUFS][kSteps], b[BUFS][kSteps];
+    auto fetch = [&](int buf, int at) {
+#pragma unroll
+        for (int u = 0; u < kSteps; ++u) {
+            const bool there = at + u < last;
+            a[buf][u] = there ? load_weights(wa + (at + u) * 4) : zero;
+            b[buf][u] = there ? load_weights(wb + (at + u) * 4) : zero;
+        }
+    };
+#pragma unroll
+    for (int i = 0; i < BUFS; ++i) fetch(i, first + i * kSteps);
+    // what the epilogue needs and no kernel of the chain writes: one thread per token and pair of features
+    const int m = static_cast<int>(threadIdx.x) >> 3, f = static_cast<int>(threadIdx.x) & 7;
+    const bool finishes = threadIdx.x < NT * 64;
+    const bool live = finishes && m < p.M;
+    const int head = tile >> 3, rank = tile & 7;
+    const int head_kind = head < p.q_heads ? 0 : head < p.q_heads + p.kv_heads ? 1 : 2;   // q, k, v
+    const __nv_bfloat16* head_w = head_kind == 0 ? p.q_norm_w : head_kind == 1 ? p.k_norm_w : nullptr;
+    float cs = 1.f, sn = 0.f, w0 = 1.f, w1 = 1.f, bias0 = 0.f, bias1 = 0.f;
+    int slot = -1;
+    const int n0 = KIND == kHeads ? head * 128 + rank * 8 + f : gated ? tile * 8 + f : tile * 16 + f;
+    const int n1 = n0 + (KIND == kHeads ? 64 : 8);
+    if (live) {
+        if (KIND != kResidual && !gated && p.bias != nullptr) {
+            bias0 = __bfloat162float(p.bias[n0]);
+            if (n1 < p.n_out) bias1 = __bfloat162float(p.bias[n1]);
+        }
+        if (KIND == kHeads) {
+            if (head_kind < 2) {
+                int pos = p.positions[m];
+                if (pos < 0 || pos >= p.max_pos) {
+                    if (rank == 0 && f == 0) atomicExch(&p.status[kStatusBadIndex], pos + 1);
+                    pos = min(max(pos, 0), p.max_pos - 1);
+                }
+                cs = p.cos_t[static_cast<int64_t>(pos) * 64 + rank * 8 + f];
+                sn = p.sin_t[static_cast<int64_t>(pos) * 64 + rank * 8 + f];
+                if (head_w != nullptr) {
+                    w0 = __bfloat162float(head_w[rank * 8 + f]);
+                    w1 = __bfloat162float(head_w[64 + rank * 8 + f]);
+                }
+            }
+            if (head_kind > 0) {
+                slot = p.out_loc[m];
+                if (slot < 0 || slot >= p.num_slots) {
+                    if (rank == 0 && f == 0) atomicExch(&p.status[kStatusBadIndex], slot + 1);
+                    slot = -1;
+                }
+            }
+        }
+    }
+    pdl_wait_prior();
+
+    float acc[NT][4] = {}, ss[NT] = {};
+    const uint4* xr[NT];
+#pragma unroll
+    for (int n = 0; n < NT; ++n) xr[n] = reinterpret_cast<const uint4*>(p.x + (n * 8 + g) * p.ldx) + t;
+    auto multiply = [&](int buf, int at) {
+        uint4 x[kSteps][NT], nw[kSteps];
+#pragma unroll
+        for (int u = 0; u < kSteps; ++u) {
+#pragma unroll
+            for (int n = 0; n < NT; ++n) x[u][n] = at + u < last && n * 8 + g < p.M ? xr[n][(at + u) * 4] : zero;
+            if (NORM) nw[u] = at + u < last ? *(reinterpret_cast<const uint4*>(p.norm_w) + (at + u) * 4 + t) : zero;
+        }
+#pragma unroll
+        for (int u = 0; u < kSteps; ++u) {
+#pragma unroll
+            for (int n = 0; n < NT; ++n) {
+                uint32_t v[4] = {x[u][n].x, x[u][n].y, x[u][n].z, x[u][n].w};
+                if (NORM) {
+                    const uint32_t w4[4] = {nw[u].x, nw[u].y, nw[u].z, nw[u].w};
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float lo = bf16_lo(v[e]), hi = bf16_hi(v[e]);
+                        ss[n] = fmaf(lo, lo, fmaf(hi, hi, ss[n]));
+                        v[e] = pack_bf16(lo * bf16_lo(w4[e]), hi * bf16_hi(w4[e]));
+                    }
+                }
+                mma_bf16_16816(acc[n], {a[buf][u].x, b[buf][u].x, a[buf][u].y, b[buf][u].y}, v[0], v[1]);
+                mma_bf16_16816(acc[n], {a[buf][u].z, b[buf][u].z, a[buf][u].w, b[buf][u].w}, v[2], v[3]);
+            }
+        }
+    };
+    if (BUFS == 1) {
+        multiply(0, first);
+    } else {
+        for (int at = first; at < last; at += BUFS * kSteps) {
+#pragma unroll
+            for (int i = 0; i < BUFS; ++i) {
+                multiply(i, at + i * kSteps);
+                fetch(i, at + (BUFS + i) * kSteps);
+            }
+        }
+    }
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+        float* part = &s_part[warp][(n * 8 + 2 * t) * kTokenPitch + g];
+        part[0] = acc[n][0];
+        part[kTokenPitch] = acc[n][1];
+        part[8] = acc[n][2];
+        part[kTokenPitch + 8] = acc[n][3];
+        if (NORM) {
+            ss[n] += __shfl_xor_sync(0xffffffffu, ss[n], 1);
+            ss[n] += __shfl_xor_sync(0xffffffffu, ss[n], 2);
+            if (t == 0) s_ssq[warp][n * 8 + g] = ss[n];
+        }
+    }
+    __syncthreads();
+
+    float v0 = 0.f, v1 = 0.f;
+    if (finishes) {
+#pragma unroll
+        for (int i = 0; i < WARPS; ++i) {
+            v0 += s_part[i][m * kTokenPitch + f];
+            v1 += s_part[i][m * kTokenPitch + 8 + f];
+        }
+        if (NORM) {
+            float sum = 0.f;
+#pragma unroll
+            for (int i = 0; i < WARPS; ++i) sum += s_ssq[i][m];
+            const float rstd = rsqrtf(sum / static_cast<float>(p.K) + p.norm_eps);
+            v0 *= rstd;
+            v1 *= rstd;
+        }
+        v0 += bias0;
+        v1 += bias1;
+    }
+    if (KIND == kHeads) {
+        // the projection's own output, as it would be stored; then head norm, rotation, store
+        v0 = round_bf16(v0);
+        v1 = round_bf16(v1);
+        cluster_wait();
+        if (head_w != nullptr) {   // (the same for a whole cluster)
+            float sq = v0 * v0 + v1 * v1;
+            sq += __shfl_xor_sync(0xffffffffu, sq, 4);
+            sq += __shfl_xor_sync(0xffffffffu, sq, 2);
+            sq += __shfl_xor_sync(0xffffffffu, sq, 1);
+            if (finishes) store_in_cluster(&s_head[rank][m], f, sq);   // thread f tells rank f
+            cluster_arrive();
+            cluster_wait();
+            if (finishes) {
+                float sum = 0.f;
+#pragma unroll
+                for (int i = 0; i < kHeadRanks; ++i) sum += s_head[i][m];
+                const float scale = rsqrtf(sum / 128.f + p.qk_eps);
+                v0 = round_bf16(v0 * scale * w0);
+                v1 = round_bf16(v1 * scale * w1);
+            }
+        }
+        if (!live) return;
+        const float r0 = v0 * cs - v1 * sn, r1 = v1 * cs + v0 * sn;
+        __nv_bfloat16* dst = nullptr;
+        if (head_kind == 0)
+            dst = p.y + m * p.y_pitch + head * 128;
+        else if (slot >= 0)
+            dst = (head_kind == 1 ? p.k_cache : p.v_cache) +
+                  (static_cast<int64_t>(slot) * p.kv_heads + head - p.q_heads - (head_kind == 2 ? p.kv_heads : 0)) * 128;
+        if (dst != nullptr) {
+            dst[rank * 8 + f] = __float2bfloat16_rn(r0);
+            dst[64 + rank * 8 + f] = __float2bfloat16_rn(r1);
+        }
+        return;
+    }
+    if (!live) return;
+    if (KIND == kResidual) {
+        __nv_bfloat16* r = p.residual + static_cast<int64_t>(m) * p.n_out;
+        r[n0] = __float2bfloat16_rn(round_bf16(v0) + __bfloat162float(r[n0]));
+        if (n1 < p.n_out) r[n1] = __float2bfloat16_rn(round_bf16(v1) + __bfloat162float(r[n1]));
+        return;
+    }
+    const int64_t at = m * p.y_pitch + n0;
+    if (gated) {
+        p.y[at] = __float2bfloat16_rn(activate_pair(p.epilogue, round_bf16(v0), round_bf16(v1), p.act_limit));
+        return;
+    }
+    if (p.epilogue == B200_EPILOGUE_RELU2) {
+        v0 = fmaxf(v0, 0.f) * fmaxf(v0, 0.f);
+        v1 = fmaxf(v1, 0.f) * fmaxf(v1, 0.f);
+    } else if (p.epilogue == B200_EPILOGUE_GELU_ERF) {
+        v0 = 0.5f * v0 * (1.0f + erff(v0 * 0.70710678118654752f));
+        v1 = 0.5f * v1 * (1.0f + erff(v1 * 0.70710678118654752f));
+    }
+    if (p.epilogue == B200_EPILOGUE_F32) {
+        float* y = reinterpret_cast<float*>(p.y) + at;
+        y[0] = v0;
+        if (n1 < p.n_out) y[8] = v1;
+        return;
+    }
+    p.y[at] = __float2bfloat16_rn(v0);
+    if (n1 < p.n_out) p.y[at + 8] = __float2bfloat16_rn(v1);
+}
+
+template <int KIND, bool NORM, int NT>
+cudaError_t launch(const NarrowParams& p, int tiles, cudaStream_t stream) {
+    const dim3 cluster(KIND == kHeads ? kHeadRanks : 1, 1, 1);
+    auto go = [&](auto kernel, int warps) {
+        return launch_kernel(kernel, dim3(tiles), dim3(warps * 32), 0, stream, cluster, p);
+    };
+    // Few tiles: more warps each.  A share of K that one buffer holds needs fewer registers.
+    if (tiles <= sm_count() && p.steps > 8 * kSteps) {
+        if (p.steps <= 16 * kSteps) return go(narrow_gemm_kernel<KIND, NORM, NT, 16, 1>, 16);
+        if constexpr (KIND != kHeads && !NORM) return go(narrow_gemm_kernel<KIND, NORM, NT, 16, 2>, 16);
+    }
+    return p.steps <= 8 * kSteps ? go(narrow_gemm_kernel<KIND, NORM, NT, 8, 1>, 8) : go(narrow_gemm_kernel<KIND, NORM, NT, 8, 2>, 8);
+}
+
+template <int KIND, bool NORM>
+cudaError_t launch(const NarrowParams& p, int tiles, cudaStream_t stream) {
+    return p.M <= 8 ? launch<KIND, NORM, 1>(p, tiles, stream) : launch<KIND, NORM, 2>(p, tiles, stream);
+}
+
+}  // namespace
+
+// Two tiles of tokens double a warp's operands and products, and a long K is walked a buffer at a time behind the wait,
+// where the TMA ring of gemm_skinny.cu keeps more bytes in flight (us, this against that, 16 rows: 6144 x 1024 5.0 and 8.7,
+// 2048 x 6144 8.8 and 14.4, 12288 x 2048 18.6 and 16.1; 4 rows of 28672 x 4096 43 and 45, but 57 and 44 with the norm).
+bool narrow_gemm_takes(const void* x, const void* w, int M, int N, int K, int64_t ldx, int epilogue) {
+    const int64_t bytes = static_cast<int64_t>(N) * K * 2;
+    const int n_out = epilogue_is_gated(epilogue) ? N / 2 : N;
+    const bool faster = (M <= 8 && K <= 2048) || (M <= kNarrowRows && bytes <= (26ll << 20));
+    return M >= 1 && faster && n_out % 8 == 0 && K % 32 == 0 && ldx % 8 == 0 &&
+           ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
+}
+
+int launch_narrow_gemm(void* y, const void* x, const void* w, const void* bias, int M, int N, int K, int64_t ldx, int epilogue,
+                       int* status, cudaStream_t stream, const NarrowFusion* fuse, float act_limit) {
+    const bool gated = epilogue_is_gated(epilogue);
+    const HeadEpilogue* h = fuse ? fuse->heads : nullptr;
+    NarrowParams p = {};
+    p.y = static_cast<__nv_bfloat16*>(y);
+    p.x = static_cast<const __nv_bfloat16*>(x);
+    p.w = static_cast<const __nv_bfloat16*>(w);
+    p.bias = static_cast<const __nv_bfloat16*>(bias);
+    p.norm_w = fuse ? static_cast<const __nv_bfloat16*>(fuse->norm_w) : nullptr;
+    p.norm_eps = fuse ? fuse->eps : 0.f;
+    p.residual = fuse ? static_cast<__nv_bfloat16*>(fuse->residual) : nullptr;
+    p.M = M;
+    p.n_rows = N;
+    p.n_out = gated ? N / 2 : N;
+    p.up_row_offset = gated ? N / 2 : 0;
+    p.steps = K / 32;
+    p.epilogue = epilogue;
+    p.ldx = ldx;
+    p.K = K;
+    p.y_pitch = p.n_out;
+    p.act_limit = act_limit;
+    p.status = status;
+    if (h != nullptr) {
+        B200_CHECK_ARG(!gated && N == (h->q_heads + 2 * h->kv_heads) * 128,
+                       "linear: the head epilogue wants a plain projection of (q_heads + 2 kv_heads) x 128 features");
+        p.q_norm_w = static_cast<const __nv_bfloat16*>(h->q_norm_w);
+        p.k_norm_w = static_cast<const __nv_bfloat16*>(h->k_norm_w);
+        p.cos_t = h->cos_t;
+        p.sin_t = h->sin_t;
+        p.positions = h->positions;
+        p.out_loc = h->out_loc;
+        p.k_cache = static_cast<__nv_bfloat16*>(h->k_cache);
+        p.v_cache = static_cast<__nv_bfloat16*>(h->v_cache);
+        p.q_heads = h->q_heads;
+        p.kv_heads = h->kv_heads;
+        p.max_pos = h->max_pos;
+        p.num_slots = h->num_slots;
+        p.qk_eps = h->eps;
+    }
+    const int tiles = gated ? div_ceil(p.n_out, 8) : div_ceil(N, 16);
+    cudaError_t err;
+    if (h != nullptr)
+        err = p.norm_w ? launch<kHeads, true>(p, tiles, stream) : launch<kHeads, false>(p, tiles, stream);
+    else if (p.residual != nullptr)
+        err = launch<kResidual, false>(p, tiles, stream);
+    else
+        err = p.norm_w ? launch<kPlain, true>(p, tiles, stream) : launch<kPlain, false>(p, tiles, stream);
+    B200_CHECK_CUDA(err);
+    return B200_OK;
+}
+
+}  // namespace b200

@@ -936,7 +936,10 @@ int launch_linear_heads(void* y, const void* x, const void* w, int M, int heads,
 
 int launch_linear(void* y, const void* x, const void* w, const void* bias, int M, int N, int K,
                   int64_t ldx, int epilogue, int* status, cudaStream_t stream, const SkinnyFusion* fuse,
-                  float act_limit) {
+                  float act_limit, bool narrow) {
+    // A handful of rows: weights straight into registers.
+    if (narrow && fuse == nullptr && narrow_gemm_takes(x, w, M, N, K, ldx, epilogue))
+        return launch_narrow_gemm(y, x, w, bias, M, N, K, ldx, epilogue, status, stream, nullptr, act_limit);
     // Few rows: stream the weights once (swap-AB, split-K).  Many rows: tensor-bound tiles.
     if (M >= env_int("B200_GEMM_TILE_MIN_M", 257)) {
         if (fuse != nullptr) {

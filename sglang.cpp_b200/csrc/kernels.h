@@ -103,13 +103,28 @@ struct SkinnyFusion {
     bool ssq_of_rounded = false;
     const HeadEpilogue* heads = nullptr;
 };
+// The same calls with at most kNarrowRows rows (gemm_narrow.cu), with fusions of its own:
+//  - norm_w: the rows of x are un-normalised; they enter as bf16(x * norm_w), and the result is scaled by the row's 1 / rms;
+//  - residual, heads: as above (without statistics for the projection that follows).
+constexpr int kNarrowRows = 16;
+struct NarrowFusion {
+    const void* norm_w = nullptr;
+    float eps = 0.f;
+    void* residual = nullptr;
+    const HeadEpilogue* heads = nullptr;
+};
+// Is that kernel possible, and the faster one?
+bool narrow_gemm_takes(const void* x, const void* w, int M, int N, int K, int64_t ldx, int epilogue);
+int launch_narrow_gemm(void* y, const void* x, const void* w, const void* bias, int M, int N, int K, int64_t ldx, int epilogue,
+                       int* status, cudaStream_t stream, const NarrowFusion* fuse = nullptr, float act_limit = 0.f);
 // The K split launch_linear picks for a slab of this shape (the fusions need it above 1).
 int skinny_gemm_split(int M, int N, int K, int epilogue);
 
-// y[M, n_out] = x[M, K] w[N, K]^T (+bias / gated epilogue); any M (slabs of 256 rows).
+// y[M, n_out] = x[M, K] w[N, K]^T (+bias / gated epilogue); any M (slabs of 256 rows).  narrow: a handful of rows may take
+// launch_narrow_gemm (another order of the same sums).
 int launch_linear(void* y, const void* x, const void* w, const void* bias, int M, int N, int K,
                   int64_t ldx, int epilogue, int* status, cudaStream_t stream,
-                  const SkinnyFusion* fuse = nullptr, float act_limit = 0.f);
+                  const SkinnyFusion* fuse = nullptr, float act_limit = 0.f, bool narrow = true);
 
 int launch_grouped_gemm(void* y, const void* x, const void* w, const int32_t* counts,
                         const int32_t* offsets, int num_groups, int max_rows_per_group,

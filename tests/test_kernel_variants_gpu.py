@@ -1,0 +1,37 @@
+"""Kernels that a rule on sizes picks, at the sizes where each can go wrong, against the oracle.
+
+Tolerances are those of the operators' own tests: the variants differ from one another in the order of fp32 sums only."""
+import pytest
+import torch
+
+from oracle import token_loop_oracle as O
+from tests.parity_cases import assert_close_bf16, decode_attention_case, prefill_attention_case, randn_bf16
+from tests.test_engine_gpu import test_decode_with_norms_folded_into_the_gemms as folded_decode
+from tests.test_moe_gpu import test_moe_forward_matches_oracle as moe_forward
+from tests.test_ops_gpu import test_fused_add_rmsnorm as fused_add
+from tests.test_saluzen_ops_gpu import DELTA, SSD, Recurrence, call, close  # noqa: F401  (call is a fixture)
+from tests.test_saluzen_ops_gpu import BF16
+
+pytestmark = pytest.mark.gpu
+RTOL = 2 ** -7
+BIG = (2e-3, 1e-3)   # absolute: sqrt(K / 1024) of the first, plus the second (as in test_linear_gpu.py)
+
+
+@pytest.mark.parametrize("M", [1, 7, 8, 9, 16])
+@pytest.mark.parametrize("N,K", [(8, 64), (24, 64), (1000, 192), (520, 2048), (1024, 3072), (4096, 1024), (128, 5632)])
+def test_linear_of_few_rows(L, pkg, M, N, K):
+    """One and two tiles of tokens, features behind the last whole tile of 16, K within a register buffer and beyond two."""
+    gen = torch.Generator().manual_seed(M + N + K)
+    buf, w, b = randn_bf16(gen, M, K + 64), randn_bf16(gen, N, K, std=0.05), randn_bf16(gen, N)
+    atol = BIG[0] * (K / 1024) ** 0.5 + BIG[1]
+    x = buf[:, 64:]
+    assert_close_bf16(L.linear(buf.cuda()[:, 64:], w.cuda(), b.cuda()), O.linear(x, w, b), 2 * atol, RTOL, "bias, strided rows")
+    if N % 16 == 0:
+        y = L.linear(x.contiguous().cuda(), w.cuda(), epilogue=pkg.EPILOGUE_SWIGLU)
+        assert_close_bf16(y, O.silu_and_mul(O.linear(x, w)), 2 * atol, 3 * RTOL, "SwiGLU")
+    assert L.read_device_status() == (0, 0)
+
+
+@pytest.mark.parametrize("kind,nreq", [("qwen3", 12), ("llama", 9), ("qwen2", 16)])
+def test_decode_of_two_token_tiles(pkg, monkeypatch, kind, nreq):
+    folded_decode(pkg, monkeypatch, kind, nreq, "1")
