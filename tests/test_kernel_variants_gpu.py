@@ -35,3 +35,11 @@ def test_linear_of_few_rows(L, pkg, M, N, K):
 @pytest.mark.parametrize("kind,nreq", [("qwen3", 12), ("llama", 9), ("qwen2", 16)])
 def test_decode_of_two_token_tiles(pkg, monkeypatch, kind, nreq):
     folded_decode(pkg, monkeypatch, kind, nreq, "1")
+
+
+@pytest.mark.parametrize("seq_lens,page_size,hq,hkv", [([700], 16, 16, 8), ([33], 16, 16, 8), ([5000, 2], 16, 16, 8), ([3000], 1, 8, 1),
+                                                       ([900] * 5, 64, 32, 4)])
+def test_decode_of_few_requests_with_many_partials(L, seq_lens, page_size, hq, hkv):
+    got, want, _ = decode_attention_case(L, seq_lens, page_size, hq, hkv, seed=len(seq_lens))
+    assert_close_bf16(got, want, 2e-2, 2e-2, "decode attention")
+    assert L.read_device_status() == (0, 0)
