@@ -43,3 +43,25 @@ def test_decode_of_few_requests_with_many_partials(L, seq_lens, page_size, hq, h
     got, want, _ = decode_attention_case(L, seq_lens, page_size, hq, hkv, seed=len(seq_lens))
     assert_close_bf16(got, want, 2e-2, 2e-2, "decode attention")
     assert L.read_device_status() == (0, 0)
+
+
+@pytest.mark.parametrize("tile", [0, 64, 128, 192, 256])
+@pytest.mark.parametrize("M,N,K", [(257, 72, 64), (300, 1000, 192), (129, 520, 640), (1025, 384, 1024), (2600, 2064, 128)])
+def test_tiles_of_every_width(L, pkg, monkeypatch, tile, M, N, K):
+    """Rows behind a tile's first and second half, features behind its last, K from one block to more than the ring holds, and
+    (2600 x 2064 with tiles of 64) more tiles than pairs of CTAs."""
+    monkeypatch.setenv("B200_TILE_TN", str(tile))
+    gen = torch.Generator().manual_seed(M + N)
+    x, w, b = randn_bf16(gen, M, K), randn_bf16(gen, N, K, std=0.05), randn_bf16(gen, N)
+    atol = BIG[0] * (K / 1024) ** 0.5 + BIG[1]
+    assert_close_bf16(L.linear(x.cuda(), w.cuda(), b.cuda()), O.linear(x, w, b), 2 * atol, RTOL, "bias")
+    if N % 16 == 0:
+        y = L.linear(x.cuda(), w.cuda(), epilogue=pkg.EPILOGUE_SWIGLU)
+        assert_close_bf16(y, O.silu_and_mul(O.linear(x, w)), 2 * atol, 3 * RTOL, "SwiGLU")
+    assert L.read_device_status() == (0, 0)
+
+
+@pytest.mark.parametrize("T,E,k", [(380, 4, 2), (450, 3, 1), (1030, 8, 1)])
+def test_experts_of_one_pair_tile(L, T, E, k):
+    """Between 128 and 256 rows per expert on average: pairs of CTAs."""
+    moe_forward(L, T, E, k, 128, 192, True, "silu")
