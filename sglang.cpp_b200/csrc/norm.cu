@@ -148,6 +148,63 @@ rmsnorm_kernel(__nv_bfloat16* out, const __nv_bfloat16* x_in,
     }
 }
 
+// The same with a warp per row, for many rows of VECS * 256 elements: no barrier, and a lane's loads of a whole row in flight
+// at once (8192 x 1024, sum and norm, 67 MB: 10.0 us against 16.3 with a CTA of 128 threads per row).
+constexpr int kRowWarps = 4;
+
+template <bool FUSED_ADD, bool ROUND_FIRST, int VECS>
+__global__ void __launch_bounds__(kRowWarps * 32)
+rmsnorm_rows_kernel(__nv_bfloat16* out, const __nv_bfloat16* x_in, __nv_bfloat16* residual,
+                    const __nv_bfloat16* __restrict__ weight, int rows, float eps) {
+    const int lane = threadIdx.x & 31;
+    const int64_t row = static_cast<int64_t>(blockIdx.x) * kRowWarps + (threadIdx.x >> 5);
+    pdl_launch_dependents();
+    uint4 w[VECS];
+#pragma unroll
+    for (int i = 0; i < VECS; ++i) w[i] = __ldg(reinterpret_cast<const uint4*>(weight) + i * 32 + lane);
+    pdl_wait_prior();
+    if (row >= rows) return;
+    const uint4* xv = reinterpret_cast<const uint4*>(x_in + row * VECS * 256) + lane;
+    uint4* rv = FUSED_ADD ? reinterpret_cast<uint4*>(residual + row * VECS * 256) + lane : nullptr;
+    uint4* ov = reinterpret_cast<uint4*>(out + row * VECS * 256) + lane;
+    uint4 a[VECS], r[VECS];
+#pragma unroll
+    for (int i = 0; i < VECS; ++i) {
+        a[i] = xv[i * 32];
+        if (FUSED_ADD) r[i] = rv[i * 32];
+    }
+    float v[VECS][8], ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < VECS; ++i) {
+        const uint32_t aw[4] = {a[i].x, a[i].y, a[i].z, a[i].w}, rw[4] = {r[i].x, r[i].y, r[i].z, r[i].w};
+        uint32_t packed[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            float lo = bf16_lo(aw[j]), hi = bf16_hi(aw[j]);
+            if (FUSED_ADD) {
+                lo += bf16_lo(rw[j]);
+                hi += bf16_hi(rw[j]);
+                packed[j] = pack_bf16(lo, hi);
+                if (ROUND_FIRST) lo = bf16_lo(packed[j]), hi = bf16_hi(packed[j]);
+            }
+            v[i][2 * j] = lo;
+            v[i][2 * j + 1] = hi;
+            ss += lo * lo + hi * hi;
+        }
+        if (FUSED_ADD) rv[i * 32] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+    }
+    const float scale = rsqrtf(warp_sum(ss) / static_cast<float>(VECS * 256) + eps);
+#pragma unroll
+    for (int i = 0; i < VECS; ++i) {
+        const uint32_t ww[4] = {w[i].x, w[i].y, w[i].z, w[i].w};
+        uint32_t packed[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            packed[j] = pack_bf16(v[i][2 * j] * scale * bf16_lo(ww[j]), v[i][2 * j + 1] * scale * bf16_hi(ww[j]));
+        ov[i * 32] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+    }
+}
+
 // One warp per (token, head) row of q or k; head_dim = 32 * EPL * 2 ... handled
 // generically: each lane walks the row in 4-byte (2 x bf16) steps.
 __global__ void __launch_bounds__(128)
@@ -190,10 +247,36 @@ qk_rmsnorm_kernel(__nv_bfloat16* q, __nv_bfloat16* k, const __nv_bfloat16* __res
 
 }  // namespace
 
+// Enough rows that a warp each fills the machine, of a width that has an instance.
+template <bool FUSED_ADD, bool ROUND_FIRST>
+bool launch_rows(cudaError_t* err, void* out, const void* x, void* residual, const void* weight, int rows, int hidden, float eps,
+                 cudaStream_t stream) {
+    if (rows < 1024) return false;
+    auto go = [&](auto kernel) {
+        *err = launch_kernel(kernel, dim3(div_ceil(rows, kRowWarps)), dim3(kRowWarps * 32), 0, stream, dim3(1, 1, 1),
+                             static_cast<__nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(x),
+                             static_cast<__nv_bfloat16*>(residual), static_cast<const __nv_bfloat16*>(weight), rows, eps);
+        return true;
+    };
+    switch (hidden) {
+        case 512: return go(rmsnorm_rows_kernel<FUSED_ADD, ROUND_FIRST, 2>);
+        case 768: return go(rmsnorm_rows_kernel<FUSED_ADD, ROUND_FIRST, 3>);
+        case 1024: return go(rmsnorm_rows_kernel<FUSED_ADD, ROUND_FIRST, 4>);
+        case 1536: return go(rmsnorm_rows_kernel<FUSED_ADD, ROUND_FIRST, 6>);
+        case 2048: return go(rmsnorm_rows_kernel<FUSED_ADD, ROUND_FIRST, 8>);
+        default: return false;
+    }
+}
+
 // Launch helpers shared with the model runner.
 int launch_rmsnorm(void* out, const void* x, const void* weight, int rows, int hidden, float eps,
                    cudaStream_t stream) {
     if (rows == 0) return B200_OK;
+    cudaError_t err = cudaSuccess;
+    if (launch_rows<false, false>(&err, out, x, nullptr, weight, rows, hidden, eps, stream)) {
+        B200_CHECK_CUDA(err);
+        return B200_OK;
+    }
     const int threads = hidden >= 2048 ? 256 : 128;
     B200_CHECK_CUDA(launch_kernel(rmsnorm_kernel<false, false>, dim3(rows), dim3(threads), 0, stream, dim3(1, 1, 1),
                                   static_cast<__nv_bfloat16*>(out), static_cast<const __nv_bfloat16*>(x),
@@ -205,6 +288,12 @@ int launch_rmsnorm(void* out, const void* x, const void* weight, int rows, int h
 int launch_fused_add_rmsnorm(void* x, void* residual, const void* weight, int rows, int hidden,
                              float eps, bool round_sum_first, cudaStream_t stream) {
     if (rows == 0) return B200_OK;
+    cudaError_t err = cudaSuccess;
+    if (round_sum_first ? launch_rows<true, true>(&err, x, x, residual, weight, rows, hidden, eps, stream)
+                        : launch_rows<true, false>(&err, x, x, residual, weight, rows, hidden, eps, stream)) {
+        B200_CHECK_CUDA(err);
+        return B200_OK;
+    }
     const int threads = hidden >= 2048 ? 256 : 128;
     auto kernel = round_sum_first ? rmsnorm_kernel<true, true> : rmsnorm_kernel<true, false>;
     B200_CHECK_CUDA(launch_kernel(kernel, dim3(rows), dim3(threads), 0, stream, dim3(1, 1, 1),

@@ -226,6 +226,105 @@ qknorm_rope_store_kernel(__nv_bfloat16* qkv, const __nv_bfloat16* __restrict__ q
     }
 }
 
+// The same for many tokens with heads of 128: a warp per token, four rows (heads) at a time and sixteen in flight.  A token's
+// rotation is read once, and no row number has to be divided (8192 tokens of 32 rows, 134 MB: 26.8 us against 43.8 with rows
+// dealt to warps one after the other).
+constexpr int kTokenWarps = 4;
+
+__global__ void __launch_bounds__(kTokenWarps * 32)
+qknorm_rope_store_tokens_kernel(__nv_bfloat16* qkv, const __nv_bfloat16* __restrict__ qw, const __nv_bfloat16* __restrict__ kw,
+                                const float* __restrict__ cos_t, const float* __restrict__ sin_t,
+                                const int32_t* __restrict__ positions, const int32_t* __restrict__ out_loc,
+                                __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache, int tokens, int q_heads,
+                                int kv_heads, int max_pos, int64_t num_slots, float eps, int write_k_back, int* status) {
+    constexpr int D = 128, kAhead = 4;
+    const int lane = threadIdx.x & 31, sub = lane & 7, group = lane >> 3;
+    const int t = static_cast<int>(blockIdx.x) * kTokenWarps + (threadIdx.x >> 5);
+    pdl_launch_dependents();
+    int slot = -1;
+    Vec8 cs = {}, sn = {}, wq[2] = {}, wk[2] = {};
+    if (t < tokens) {
+        int pos = positions[t];
+        slot = out_loc[t];
+        if (lane == 0 && (pos < 0 || pos >= max_pos)) atomicExch(&status[kStatusBadIndex], pos + 1);
+        if (lane == 0 && (slot < 0 || slot >= num_slots)) atomicExch(&status[kStatusBadIndex], slot + 1);
+        pos = min(max(pos, 0), max_pos - 1);
+        if (slot >= num_slots) slot = -1;
+        cs = load8(cos_t + static_cast<int64_t>(pos) * (D / 2) + sub * 8);
+        sn = load8(sin_t + static_cast<int64_t>(pos) * (D / 2) + sub * 8);
+    }
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        if (qw != nullptr) wq[half] = load8(qw + half * (D / 2) + sub * 8);
+        if (kw != nullptr) wk[half] = load8(kw + half * (D / 2) + sub * 8);
+    }
+    pdl_wait_prior();
+    if (t >= tokens) return;
+    const int rows = q_heads + 2 * kv_heads;
+    __nv_bfloat16* base = qkv + static_cast<int64_t>(t) * rows * D + sub * 8;
+    for (int r0 = 0; r0 < rows; r0 += 4 * kAhead) {
+        uint4 a[kAhead], b[kAhead];
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) {
+            const int r = min(r0 + 4 * i + group, rows - 1);
+            a[i] = *reinterpret_cast<const uint4*>(base + r * D);
+            b[i] = *reinterpret_cast<const uint4*>(base + r * D + D / 2);
+        }
+#pragma unroll
+        for (int i = 0; i < kAhead; ++i) {
+            const int r = r0 + 4 * i + group;
+            const bool is_q = r < q_heads, is_k = !is_q && r < q_heads + kv_heads;
+            __nv_bfloat16* src = base + r * D;
+            __nv_bfloat16* pool = is_q || slot < 0 ? nullptr
+                                  : (is_k ? k_cache : v_cache) + (static_cast<int64_t>(slot) * kv_heads +
+                                                                   (r - q_heads - (is_k ? 0 : kv_heads))) * D + sub * 8;
+            if (r0 + 4 * i >= q_heads + kv_heads) {   // (the whole warp: values as they are)
+                if (r < rows && pool != nullptr) {
+                    *reinterpret_cast<uint4*>(pool) = a[i];
+                    *reinterpret_cast<uint4*>(pool + D / 2) = b[i];
+                }
+                continue;
+            }
+            Vec8 x = load8(reinterpret_cast<const __nv_bfloat16*>(&a[i])), y = load8(reinterpret_cast<const __nv_bfloat16*>(&b[i]));
+            if (qw != nullptr) {
+                float ss = 0.f;
+#pragma unroll
+                for (int e = 0; e < 8; ++e) ss += x.v[e] * x.v[e] + y.v[e] * y.v[e];
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+                const float scale = rsqrtf(ss / static_cast<float>(D) + eps);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    // bf16 rounding here is where the unfused norm kernel stores its result.
+                    x.v[e] = round_bf16(x.v[e] * scale * (is_q ? wq[0].v[e] : wk[0].v[e]));
+                    y.v[e] = round_bf16(y.v[e] * scale * (is_q ? wq[1].v[e] : wk[1].v[e]));
+                }
+            }
+            Vec8 u, v;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                u.v[e] = x.v[e] * cs.v[e] - y.v[e] * sn.v[e];
+                v.v[e] = y.v[e] * cs.v[e] + x.v[e] * sn.v[e];
+            }
+            if (!is_q && !is_k) {
+                if (r < rows && pool != nullptr) {
+                    *reinterpret_cast<uint4*>(pool) = a[i];
+                    *reinterpret_cast<uint4*>(pool + D / 2) = b[i];
+                }
+                continue;
+            }
+            if (is_q || write_k_back) {
+                store8(src, u);
+                store8(src + D / 2, v);
+            }
+            if (pool != nullptr) {
+                store8(pool, u);
+                store8(pool + D / 2, v);
+            }
+        }
+    }
+}
+
 }  // namespace
 
 int launch_qknorm_rope_store(void* qkv, const void* q_weight, const void* k_weight,
@@ -236,6 +335,16 @@ int launch_qknorm_rope_store(void* qkv, const void* q_weight, const void* k_weig
                              int* status, cudaStream_t stream) {
     const int64_t rows = static_cast<int64_t>(tokens) * (q_heads + 2 * kv_heads);
     if (rows == 0) return B200_OK;
+    const bool aligned = ((reinterpret_cast<uintptr_t>(cos_table) | reinterpret_cast<uintptr_t>(sin_table)) & 15) == 0;
+    if (rows >= 32768 && head_dim == 128 && aligned) {
+        B200_CHECK_CUDA(launch_kernel(qknorm_rope_store_tokens_kernel, dim3(div_ceil(tokens, kTokenWarps)), dim3(kTokenWarps * 32), 0,
+                                      stream, dim3(1, 1, 1), static_cast<__nv_bfloat16*>(qkv),
+                                      static_cast<const __nv_bfloat16*>(q_weight), static_cast<const __nv_bfloat16*>(k_weight),
+                                      cos_table, sin_table, positions, out_loc, static_cast<__nv_bfloat16*>(k_cache),
+                                      static_cast<__nv_bfloat16*>(v_cache), tokens, q_heads, kv_heads, max_pos, num_slots, eps,
+                                      write_k_back, status));
+        return B200_OK;
+    }
     // Few rows (decode): one row per warp for the most parallelism; many rows (prefill): four per
     // warp with the next row's loads in flight.
     const int rows_per_warp = rows >= 32768 ? 4 : 1;   // passes of 4 rows each

@@ -65,3 +65,39 @@ def test_tiles_of_every_width(L, pkg, monkeypatch, tile, M, N, K):
 def test_experts_of_one_pair_tile(L, T, E, k):
     """Between 128 and 256 rows per expert on average: pairs of CTAs."""
     moe_forward(L, T, E, k, 128, 192, True, "silu")
+
+
+@pytest.mark.parametrize("rows", [1023, 1024, 1027])
+@pytest.mark.parametrize("hidden", [512, 768, 1024, 1536, 2048, 2560])
+def test_norms_of_many_rows(L, rows, hidden):
+    fused_add(L, rows, hidden)
+    gen = torch.Generator().manual_seed(hidden)
+    norm, x = L.RMSNorm(hidden, 1e-6), randn_bf16(gen, rows, hidden)
+    norm.weight = randn_bf16(gen, hidden).cuda()
+    assert_close_bf16(norm.forward(x.cuda()), O.rmsnorm(x, norm.weight.cpu(), 1e-6), 1e-6, RTOL, "norm")
+
+
+@pytest.mark.parametrize("tokens,hq,hkv,qk_norm", [(4700, 5, 1, True), (1025, 16, 8, False), (2341, 6, 4, True)])
+def test_head_pass_of_many_tokens(L, tokens, hq, hkv, qk_norm):
+    """Rows per token that are not a multiple of the four a warp takes at a time, keys beginning inside such a group: the same
+    bits as in pieces that are few enough rows for the other kernel (which has its own test against the oracle)."""
+    gen = torch.Generator().manual_seed(tokens)
+    width = (hq + 2 * hkv) * 128
+    qkv = randn_bf16(gen, tokens, width)
+    pos = torch.randint(0, 2048, (tokens,), generator=gen, dtype=torch.int32).cuda()
+    rot, qn, kn = L.RotaryEmbedding(128, 128, 2048, 1e6), None, None
+    if qk_norm:
+        qn, kn = L.RMSNorm(128, 1e-6), L.RMSNorm(128, 1e-6)
+        qn.weight, kn.weight = randn_bf16(gen, 128).cuda(), randn_bf16(gen, 128).cuda()
+    results = []
+    for piece in (tokens, 500):
+        cache = L.MHAKVCache(hkv, 1, 128, tokens // 16 + 2, 16)
+        loc = torch.randperm(cache.total_slots, generator=torch.Generator().manual_seed(3))[:tokens].to(torch.int32).cuda()
+        x = qkv.cuda()
+        for t in range(0, tokens, piece):
+            part = slice(t, min(t + piece, tokens))
+            L.qknorm_rope_store(x[part], qn, kn, rot, pos[part], loc[part], cache, 0, hq, hkv, write_k_back=piece == tokens)
+        results.append((x[:, :hq * 128].clone(), cache.k_cache(0).clone(), cache.v_cache(0).clone()))
+        if piece == tokens:
+            assert torch.equal(x[:, hq * 128:(hq + hkv) * 128].view(tokens, hkv, 128), cache.k_cache(0)[loc.long()])
+    assert all(torch.equal(a, b) for a, b in zip(*results))
