@@ -975,19 +975,18 @@ __device__ __forceinline__ uint32_t transpose_8x8(uint32_t x) {
     return y;
 }
 
-constexpr int kWalkThreads = 256;
-constexpr int kSlice = 64;            // value columns per CTA, 16 per pair of warps
+constexpr int kSlice = 64;            // value columns per CTA at most, 16 per pair of warps
 
-template <int DK, int RULE>
+template <int DK, int RULE, int SLICE>
 struct WalkSmem {
-    static constexpr int kRow = DK + kPad, kVRow = kSlice + kPad;
+    static constexpr int kRow = DK + kPad, kVRow = SLICE + kPad;
     __nv_bfloat16 k[2][kChunk * kRow], q[2][kChunk * kRow], v[2][kChunk * kVRow];   // this chunk's and the next one's
     uint4 m[2][(RULE == kDelta ? 2 : 1) * kMatrixVecs];   // P and inverse
     // what the warps of a pair hand to one another as left operands, per 16 tokens upper and lower parts:
     // beta (V - G K S), U, U as it enters the state
-    uint4 hand[RULE == kDelta ? 3 : 1][kSlice / 16][RULE == kDelta ? 4 : 1][2][32];
+    uint4 hand[RULE == kDelta ? 3 : 1][SLICE / 16][RULE == kDelta ? 4 : 1][2][32];
     // and what a warp's state rows add to the other one's tokens: [pair][warp][token tile][Q S, K S][8 tokens]
-    float4 sums[kSlice / 16][2][2][RULE == kDelta ? 2 : 1][2][32];
+    float4 sums[SLICE / 16][2][2][RULE == kDelta ? 2 : 1][2][32];
     float out[2][kChunk];      // G_t times q's factor
     float beta[2][kChunk], read[2][kChunk];   // beta_t; beta_t G_t times k's factor
     float write[2][kChunk];    // exp(B_n - B_t) times k's factor (or times dt)
@@ -997,20 +996,25 @@ struct WalkSmem {
     float n[RULE == kMemory ? DK : 4], over[RULE == kMemory ? kChunk : 4];
 };
 
-// Grid: slices of 64 value columns, heads, requests.  All products are formed transposed, 16 value columns by tokens (or
+// Grid: slices of SLICE value columns, heads, requests.  Pairs of warps have nothing to do with one another, so where few
+// requests and heads leave SMs idle a CTA takes fewer columns: a pair alone does not wait for the tensor pipe behind three
+// others (a prompt of 3001 tokens, 16 heads of 128 by 128: 214 us with 64 columns on 32 CTAs, 186 with 16 on 128; 32 heads of
+// 128 by 64 of the state space: 153 and 137).  All products are formed transposed, 16 value columns by tokens (or
 // by state rows), so that what one leaves in a warp's accumulators is the next one's left operand where it is.  Two
 // warps share 16 columns: each keeps half of the state rows and works out the results of half of the tokens (tiles 0
 // and 3, tiles 1 and 2).
-template <int DK, int RULE>
-__global__ void __launch_bounds__(kWalkThreads, 1)
+template <int DK, int RULE, int SLICE>
+__global__ void __launch_bounds__(SLICE * 4, 1)
 chunk_kernel(const Recurrence a) {
-    using Smem = WalkSmem<DK, RULE>;
+    using Smem = WalkSmem<DK, RULE, SLICE>;
+    static_assert(RULE != kMemory || SLICE == kSlice, "a CTA keeps its own n and m");
+    constexpr int kWalkThreads = SLICE * 4;
     constexpr int ROW = Smem::kRow, VROW = Smem::kVRow, kMatrices = RULE == kDelta ? 2 : 1;
     extern __shared__ __align__(16) uint8_t smem_raw[];
     Smem& S = *reinterpret_cast<Smem*>(smem_raw);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int g = lane >> 2, tq = lane & 3, mi = lane >> 3, r8 = lane & 7;
-    const int h = blockIdx.y, req = blockIdx.z, v0 = blockIdx.x * kSlice, pair = warp >> 1, half = warp & 1, col0 = pair * 16;
+    const int h = blockIdx.y, req = blockIdx.z, v0 = blockIdx.x * SLICE, pair = warp >> 1, half = warp & 1, col0 = pair * 16;
     const int vp = a.padded_value_dim, kvh = h / (a.heads / a.kv_heads);
     const int own[4] = {half, 3 - half, 1 - half, 2 + half};   // this warp's 16-token tiles, then the other one's
     constexpr int kRows = DK / 2;                              // state rows per warp
@@ -1031,8 +1035,8 @@ chunk_kernel(const Recurrence a) {
             cp_async16(smem_u32(&S.k[buf][t * ROW + c]), row, t < n);
             cp_async16(smem_u32(&S.q[buf][t * ROW + c]), row + to_q, t < n);
         }
-        for (int i = threadIdx.x; i < kChunk * (kSlice / 8); i += kWalkThreads) {
-            const int t = i / (kSlice / 8), c = (i % (kSlice / 8)) * 8;
+        for (int i = threadIdx.x; i < kChunk * (SLICE / 8); i += kWalkThreads) {
+            const int t = i / (SLICE / 8), c = (i % (SLICE / 8)) * 8;
             cp_async16(smem_u32(&S.v[buf][t * VROW + c]), mixed + static_cast<int64_t>(t < n ? s0 + t : s0) * nc + at_v + c, t < n);
         }
     };
@@ -1188,7 +1192,7 @@ chunk_kernel(const Recurrence a) {
             if ((threadIdx.x & 3) == 0)
                 S.over[t] = 1.f / (fmaxf(fabsf(fmaf(S.out[buf][t], dot, S.own[buf][t] * S.row_sum[buf][t])), S.floor[buf][t]) + kMemoryEps);
             __syncthreads();
-            constexpr int kParts = kWalkThreads / DK;
+            constexpr int kParts = 256 / DK;
             const int i = threadIdx.x / kParts, part = threadIdx.x % kParts;
             float sum = 0.f;
 #pragma unroll 8
@@ -1395,7 +1399,7 @@ chunk_kernel(const Recurrence a) {
     }
     if constexpr (RULE == kMemory) {
         __syncthreads();
-        for (int at = v0; at < v0 + kSlice; at += memory_columns(DK)) {
+        for (int at = v0; at < v0 + SLICE; at += memory_columns(DK)) {
             float* memory = memory_of(a, a.table_idx[req], h, at);
             for (int i = threadIdx.x; i < DK; i += kWalkThreads) memory[i] = S.n[i];
             if (threadIdx.x == 0) memory[DK] = top;
@@ -1428,6 +1432,17 @@ int launch_mix(const Recurrence& a, cudaStream_t stream) {
     return B200_OK;
 }
 
+template <int RULE, int SLICE>
+int launch_walk(const Recurrence& a, cudaStream_t stream) {
+    auto kernel = a.padded_dim == 64 ? chunk_kernel<64, RULE, SLICE> : chunk_kernel<128, RULE, SLICE>;
+    const size_t smem = a.padded_dim == 64 ? sizeof(WalkSmem<64, RULE, SLICE>) : sizeof(WalkSmem<128, RULE, SLICE>);
+    const int err = max_smem(reinterpret_cast<const void*>(kernel), smem);
+    if (err != B200_OK) return err;
+    B200_CHECK_CUDA(launch_kernel(kernel, dim3(a.padded_value_dim / SLICE, a.heads, a.batch), dim3(SLICE * 4), smem, stream,
+                                  dim3(1, 1, 1), a));
+    return B200_OK;
+}
+
 template <int RULE>
 int launch_chunked(const Recurrence& a, cudaStream_t stream) {
     auto prepare = prepare_kernel<RULE>;
@@ -1436,12 +1451,12 @@ int launch_chunked(const Recurrence& a, cudaStream_t stream) {
     const int parts = div_ceil(a.heads / a.kv_heads, kPrepareHeads);
     B200_CHECK_CUDA(launch_kernel(prepare, dim3(div_ceil(a.max_extend, kChunk), a.kv_heads * parts, a.batch), dim3(kPrepareThreads),
                                   sizeof(PrepareSmem), stream, dim3(1, 1, 1), a, parts));
-    auto kernel = a.padded_dim == 64 ? chunk_kernel<64, RULE> : chunk_kernel<128, RULE>;
-    const size_t smem = a.padded_dim == 64 ? sizeof(WalkSmem<64, RULE>) : sizeof(WalkSmem<128, RULE>);
-    err = max_smem(reinterpret_cast<const void*>(kernel), smem);
-    if (err != B200_OK) return err;
-    B200_CHECK_CUDA(launch_kernel(kernel, dim3(a.padded_value_dim / kSlice, a.heads, a.batch), dim3(kWalkThreads), smem, stream,
-                                  dim3(1, 1, 1), a));
+    // the narrowest slices whose CTAs still run at once
+    const int units = a.heads * a.batch;
+    int slice = kSlice;
+    while (RULE != kMemory && slice > 16 && static_cast<int64_t>(units) * (a.padded_value_dim / slice) * 2 <= sm_count()) slice /= 2;
+    if (slice == 64) return launch_walk<RULE, 64>(a, stream);
+    if constexpr (RULE != kMemory) return slice == 32 ? launch_walk<RULE, 32>(a, stream) : launch_walk<RULE, 16>(a, stream);
     return B200_OK;
 }
 

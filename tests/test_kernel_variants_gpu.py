@@ -101,3 +101,17 @@ def test_head_pass_of_many_tokens(L, tokens, hq, hkv, qk_norm):
         if piece == tokens:
             assert torch.equal(x[:, hq * 128:(hq + hkv) * 128].view(tokens, hkv, 128), cache.k_cache(0)[loc.long()])
     assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
+@pytest.mark.parametrize("rule", [SSD, DELTA])
+@pytest.mark.parametrize("heads", [4, 12, 20])
+@pytest.mark.parametrize("dv", [64, 128])
+def test_recurrence_in_slices_of_every_width(call, rule, heads, dv):  # noqa: F811
+    """Two requests, one of whole chunks; 4 to 20 heads are dealt in 16, 32 and 64 value columns per CTA."""
+    r = Recurrence(rule, [192, 65], heads, heads // 2, 128, dv, 4, BF16, 1)
+    states = r.states(3)
+    got = r.run(call, states, [0, 0], [2, 0])
+    outs, last = r.want()
+    close(got, torch.cat(outs), BF16)
+    for i, row in enumerate([2, 0]):
+        close(states[0][row, :, :128, :dv], last[i], BF16)
