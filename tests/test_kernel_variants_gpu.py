@@ -115,3 +115,12 @@ def test_recurrence_in_slices_of_every_width(call, rule, heads, dv):  # noqa: F8
     close(got, torch.cat(outs), BF16)
     for i, row in enumerate([2, 0]):
         close(states[0][row, :, :128, :dv], last[i], BF16)
+
+
+@pytest.mark.parametrize("seq_lens,extend_lens,page_size,hq,hkv", [([128], [128], 16, 16, 8), ([129, 257], [129, 257], 16, 16, 8),
+                                                                   ([640], [130], 1, 16, 8), ([385, 900], [200, 900], 64, 32, 4)])
+def test_prefill_at_the_edges_of_tiles(L, seq_lens, extend_lens, page_size, hq, hkv):
+    """Last tiles that are whole, of one key, in a slot of the ring that was in use and in one that was not."""
+    got, want = prefill_attention_case(L, seq_lens, extend_lens, page_size, hq, hkv, seed=sum(seq_lens))
+    assert_close_bf16(got, want, 2e-2, 2e-2, "prefill attention")
+    assert L.read_device_status() == (0, 0)
