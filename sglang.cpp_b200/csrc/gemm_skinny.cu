@@ -930,6 +930,13 @@ int launch_linear_heads(void* y, const void* x, const void* w, int M, int heads,
     return B200_OK;
 }
 
+// About how many microseconds the weight-streaming kernel takes on at most 256 rows: its weights, a start, and for every 64
+// rows an exchange (twice as much with a gated epilogue), which is what tiles do not have: 181 x 6144 x 1024 with SwiGLU
+// took 19.7 us against 10.4 on tiles, 64 rows of it 10.4 against 9.9, 181 x 1024 x 2048 10.3 against 11.3.
+static float skinny_gemm_us(int M, int N, int K, int epilogue) {
+    return static_cast<float>(N) * K * 2e-6f / 5.7f + 5.f + (epilogue_is_gated(epilogue) ? 4.2f : 1.9f) * div_ceil(M, kRoundCols);
+}
+
 int launch_linear(void* y, const void* x, const void* w, const void* bias, int M, int N, int K,
                   int64_t ldx, int epilogue, int* status, cudaStream_t stream, const SkinnyFusion* fuse,
                   float act_limit, bool narrow) {
@@ -937,7 +944,12 @@ int launch_linear(void* y, const void* x, const void* w, const void* bias, int M
     if (narrow && fuse == nullptr && narrow_gemm_takes(x, w, M, N, K, ldx, epilogue))
         return launch_narrow_gemm(y, x, w, bias, M, N, K, ldx, epilogue, status, stream, nullptr, act_limit);
     // Few rows: stream the weights once (swap-AB, split-K).  Many rows: tensor-bound tiles.
-    if (M >= env_int("B200_GEMM_TILE_MIN_M", 257)) {
+    const int tile_min = env_int("B200_GEMM_TILE_MIN_M", 257);
+    // (tiles are stored 16 bytes at a time)
+    const bool whole_vectors = (epilogue_is_gated(epilogue) ? N / 2 : N) % 8 == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0;
+    const bool tiles_faster = tile_min == 257 && fuse == nullptr && M > kRoundCols && whole_vectors &&
+                              tile_gemm_us(M, N, K, epilogue) < 0.9f * skinny_gemm_us(M, N, K, epilogue);
+    if (M >= tile_min || tiles_faster) {
         if (fuse != nullptr) {
             set_last_error("linear: the residual-stream fusions need at most 256 rows");
             return B200_ERR_UNSUPPORTED;

@@ -67,6 +67,9 @@ int cached_tmap(CUtensorMap* out, const void* base, uint64_t inner, uint64_t out
 int launch_tile_gemm(void* y, const void* x, const void* w, const void* bias, int M, int N, int K,
                      int64_t ldx, int epilogue, int* status, cudaStream_t stream, float act_limit = 0.f);
 
+// About how many microseconds that takes, for batches that the small-batch kernel could run too.
+float tile_gemm_us(int M, int N, int K, int epilogue);
+
 int launch_grouped_tile_gemm(void* y, const void* x, const void* w, const int32_t* counts,
                              const int32_t* offsets, int num_groups, int64_t total_rows, int N, int K,
                              int epilogue, int* status, cudaStream_t stream, float act_limit = 0.f);

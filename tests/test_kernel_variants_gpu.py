@@ -61,6 +61,16 @@ def test_tiles_of_every_width(L, pkg, monkeypatch, tile, M, N, K):
     assert L.read_device_status() == (0, 0)
 
 
+@pytest.mark.parametrize("M,N,K,gated", [(65, 6144, 1024, True), (100, 4096, 1024, False), (181, 6144, 1024, True), (256, 1024, 2048, False)])
+def test_batches_that_either_kernel_takes(L, pkg, monkeypatch, M, N, K, gated):
+    gen = torch.Generator().manual_seed(M)
+    x, w = randn_bf16(gen, M, K).cuda(), randn_bf16(gen, N, K, std=0.05).cuda()
+    epilogue = pkg.EPILOGUE_SWIGLU if gated else pkg.EPILOGUE_NONE
+    y = L.linear(x, w, epilogue=epilogue)
+    monkeypatch.setenv("B200_GEMM_TILE_MIN_M", "1000000")
+    assert_close_bf16(y, L.linear(x, w, epilogue=epilogue), 4e-3, 3 * RTOL, "tiles against slabs")
+
+
 @pytest.mark.parametrize("T,E,k", [(380, 4, 2), (450, 3, 1), (1030, 8, 1)])
 def test_experts_of_one_pair_tile(L, T, E, k):
     """Between 128 and 256 rows per expert on average: pairs of CTAs."""
