@@ -75,6 +75,30 @@ __device__ float activate_pair(int epilogue, float g, float u, float limit) {
     }
 }
 
+// Activation and store of a row's features n0 and n1 (gated: of the one feature that they are the gate and up part of).
+__device__ __forceinline__ void store_plain(const NarrowParams& p, bool gated, int64_t row, int n0, int n1, float v0, float v1) {
+    const int64_t at = row * p.y_pitch + n0;
+    if (gated) {
+        p.y[at] = __float2bfloat16_rn(activate_pair(p.epilogue, round_bf16(v0), round_bf16(v1), p.act_limit));
+        return;
+    }
+    if (p.epilogue == B200_EPILOGUE_RELU2) {
+        v0 = fmaxf(v0, 0.f) * fmaxf(v0, 0.f);
+        v1 = fmaxf(v1, 0.f) * fmaxf(v1, 0.f);
+    } else if (p.epilogue == B200_EPILOGUE_GELU_ERF) {
+        v0 = 0.5f * v0 * (1.0f + erff(v0 * 0.70710678118654752f));
+        v1 = 0.5f * v1 * (1.0f + erff(v1 * 0.70710678118654752f));
+    }
+    if (p.epilogue == B200_EPILOGUE_F32) {
+        float* y = reinterpret_cast<float*>(p.y) + at;
+        y[0] = v0;
+        if (n1 < p.n_out) y[8] = v1;
+        return;
+    }
+    p.y[at] = __float2bfloat16_rn(v0);
+    if (n1 < p.n_out) p.y[at + 8] = __float2bfloat16_rn(v1);
+}
+
 // BUFS register buffers of kSteps steps: with one, a warp's whole share of K is requested ahead of the wait.
 template <int KIND, bool NORM, int NT, int WARPS, int BUFS>
 __global__ void __launch_bounds__(WARPS * 32)
@@ -272,26 +296,71 @@ narrow_gemm_kernel(const NarrowParams p) {
         if (n1 < p.n_out) r[n1] = __float2bfloat16_rn(round_bf16(v1) + __bfloat162float(r[n1]));
         return;
     }
-    const int64_t at = m * p.y_pitch + n0;
-    if (gated) {
-        p.y[at] = __float2bfloat16_rn(activate_pair(p.epilogue, round_bf16(v0), round_bf16(v1), p.act_limit));
-        return;
+    store_plain(p, gated, m, n0, n1, v0, v1);
+}
+
+// Experts: group g multiplies rows [offsets[g], offsets[g] + counts[g]) of x by its own n_rows rows of w.  A handful of rows
+// per group: a CTA keeps its 16 rows of W in registers (BUFS buffers hold a warp's whole share of K) and takes the group's
+// rows 8 at a time.  The group table comes from the kernel before, so nothing is requested ahead of the wait.  No tiles of 128
+// rows of W and 32 of x to fill, and no ring to drain between a CTA's few k-blocks: 64 experts of 3 x 1024 x 2048, 32 tokens
+// with 4 experts each, 12 layers: 2.37 ms per decode step against 2.61.
+template <int BUFS>
+__global__ void __launch_bounds__(256)
+narrow_grouped_kernel(const NarrowParams p, const int32_t* __restrict__ counts, const int32_t* __restrict__ offsets) {
+    constexpr int WARPS = 8;
+    __shared__ float s_part[WARPS][8 * kTokenPitch];
+    pdl_launch_dependents();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int tile = static_cast<int>(blockIdx.x), group = static_cast<int>(blockIdx.y);
+    const bool gated = p.up_row_offset > 0;
+    const int row_a = gated ? tile * 8 + g : tile * 16 + g;
+    const int row_b = gated ? row_a + p.up_row_offset : min(row_a + 8, p.n_rows - 1);
+    const __nv_bfloat16* w = p.w + static_cast<int64_t>(group) * p.n_rows * p.K;
+    const uint4* wa = reinterpret_cast<const uint4*>(w + row_a * p.K) + t;
+    const uint4* wb = reinterpret_cast<const uint4*>(w + row_b * p.K) + t;
+    const int first = warp * p.steps / WARPS, last = (warp + 1) * p.steps / WARPS;
+    pdl_wait_prior();
+    const int count = counts[group];
+    if (count <= 0) return;
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    uint4 a[BUFS * kSteps], b[BUFS * kSteps];
+#pragma unroll
+    for (int u = 0; u < BUFS * kSteps; ++u) {
+        const bool there = first + u < last;
+        a[u] = there ? load_weights(wa + (first + u) * 4) : zero;
+        b[u] = there ? load_weights(wb + (first + u) * 4) : zero;
     }
-    if (p.epilogue == B200_EPILOGUE_RELU2) {
-        v0 = fmaxf(v0, 0.f) * fmaxf(v0, 0.f);
-        v1 = fmaxf(v1, 0.f) * fmaxf(v1, 0.f);
-    } else if (p.epilogue == B200_EPILOGUE_GELU_ERF) {
-        v0 = 0.5f * v0 * (1.0f + erff(v0 * 0.70710678118654752f));
-        v1 = 0.5f * v1 * (1.0f + erff(v1 * 0.70710678118654752f));
+    const int64_t row0 = offsets[group];
+    const int m = static_cast<int>(threadIdx.x) >> 3, f = static_cast<int>(threadIdx.x) & 7;
+    const int n0 = gated ? tile * 8 + f : tile * 16 + f;
+    for (int m0 = 0; m0 < count; m0 += 8) {
+        const uint4* x = reinterpret_cast<const uint4*>(p.x + (row0 + m0 + min(g, count - 1 - m0)) * p.ldx) + first * 4 + t;
+        float acc[4] = {};
+        uint4 v[BUFS * kSteps];
+#pragma unroll
+        for (int u = 0; u < BUFS * kSteps; ++u) v[u] = first + u < last ? x[u * 4] : zero;   // (columns of rows that are not there: unused)
+#pragma unroll
+        for (int u = 0; u < BUFS * kSteps; ++u) {
+            mma_bf16_16816(acc, {a[u].x, b[u].x, a[u].y, b[u].y}, v[u].x, v[u].y);
+            mma_bf16_16816(acc, {a[u].z, b[u].z, a[u].w, b[u].w}, v[u].z, v[u].w);
+        }
+        float* part = &s_part[warp][2 * t * kTokenPitch + g];
+        part[0] = acc[0];
+        part[kTokenPitch] = acc[1];
+        part[8] = acc[2];
+        part[kTokenPitch + 8] = acc[3];
+        __syncthreads();
+        if (threadIdx.x < 64 && m0 + m < count) {
+            float v0 = 0.f, v1 = 0.f;
+#pragma unroll
+            for (int i = 0; i < WARPS; ++i) {
+                v0 += s_part[i][m * kTokenPitch + f];
+                v1 += s_part[i][m * kTokenPitch + 8 + f];
+            }
+            store_plain(p, gated, row0 + m0 + m, n0, n0 + 8, v0, v1);
+        }
+        if (m0 + 8 < count) __syncthreads();
     }
-    if (p.epilogue == B200_EPILOGUE_F32) {
-        float* y = reinterpret_cast<float*>(p.y) + at;
-        y[0] = v0;
-        if (n1 < p.n_out) y[8] = v1;
-        return;
-    }
-    p.y[at] = __float2bfloat16_rn(v0);
-    if (n1 < p.n_out) p.y[at + 8] = __float2bfloat16_rn(v1);
 }
 
 template <int KIND, bool NORM, int NT>
@@ -324,6 +393,32 @@ bool narrow_gemm_takes(const void* x, const void* w, int M, int N, int K, int64_
     const bool faster = (M <= 8 && K <= 2048) || (M <= kNarrowRows && bytes <= (26ll << 20));
     return M >= 1 && faster && n_out % 8 == 0 && K % 32 == 0 && ldx % 8 == 0 &&
            ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
+}
+
+bool narrow_grouped_takes(const void* x, const void* w, int64_t total_rows, int num_groups, int n_out, int K) {
+    return total_rows <= 8ll * num_groups && num_groups <= 65535 && K <= 64 * 32 && K % 32 == 0 && n_out % 8 == 0 &&
+           ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
+}
+
+int launch_narrow_grouped(void* y, const void* x, const void* w, const int32_t* counts, const int32_t* offsets, int num_groups, int N,
+                          int K, int epilogue, cudaStream_t stream, float act_limit) {
+    const bool gated = epilogue_is_gated(epilogue);
+    NarrowParams p = {};
+    p.y = static_cast<__nv_bfloat16*>(y);
+    p.x = static_cast<const __nv_bfloat16*>(x);
+    p.w = static_cast<const __nv_bfloat16*>(w);
+    p.n_rows = N;
+    p.n_out = gated ? N / 2 : N;
+    p.up_row_offset = gated ? N / 2 : 0;
+    p.steps = K / 32;
+    p.epilogue = epilogue;
+    p.ldx = p.K = K;
+    p.y_pitch = p.n_out;
+    p.act_limit = act_limit;
+    const dim3 grid(gated ? div_ceil(p.n_out, 8) : div_ceil(N, 16), num_groups);
+    auto kernel = p.steps <= 8 * kSteps ? narrow_grouped_kernel<1> : narrow_grouped_kernel<2>;
+    B200_CHECK_CUDA(launch_kernel(kernel, grid, dim3(256), 0, stream, dim3(1, 1, 1), p, counts, offsets));
+    return B200_OK;
 }
 
 int launch_narrow_gemm(void* y, const void* x, const void* w, const void* bias, int M, int N, int K, int64_t ldx, int epilogue,

@@ -823,6 +823,9 @@ int launch_grouped_gemm(void* y, const void* x, const void* w, const int32_t* co
     const int n_tiles = div_ceil(n_out, kTileN);
     const int slabs = div_ceil(max_rows_per_group, 256);
     if (num_groups == 0 || slabs == 0 || total_rows == 0) return B200_OK;
+    // A handful of rows per group: weights straight into registers.
+    if (narrow_grouped_takes(x, w, total_rows, num_groups, n_out, K))
+        return launch_narrow_grouped(y, x, w, counts, offsets, num_groups, N, K, epilogue, stream, act_limit);
     // Many rows per group on average (prefill batches): tensor-bound, take the tile kernel.
     if (total_rows >= static_cast<int64_t>(num_groups) * env_int("B200_GROUPED_TILE_MIN_ROWS", 128) && num_groups <= 256)
         return launch_grouped_tile_gemm(y, x, w, counts, offsets, num_groups, total_rows, N, K, epilogue, status,

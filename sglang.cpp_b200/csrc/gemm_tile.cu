@@ -80,66 +80,66 @@ __device__ __forceinline__ void tile_coords(int t, int m_tiles, int n_tiles, int
 template <int EPI, int TN>
 __device__ __forceinline__ void store_tile(const TileParams& p, const TileAt& at, int q, int lane, uint32_t tmem_acc) {
     constexpr bool GATED = epilogue_is_gated(EPI);
-                const int m_local = q * 32 + lane;
-                const int m = at.row0 + m_local;
-                const uint32_t t0 = tmem_acc + (static_cast<uint32_t>(q * 32) << 16);
-                constexpr int kOutCols = GATED ? TN / 2 : TN;
-                const int n_base = at.n0;
-                __nv_bfloat16* yrow = p.y + static_cast<int64_t>(m) * p.n_out;
-    #pragma unroll 1
-                for (int c = 0; c < kOutCols / 32; ++c) {
-                    uint32_t g[32], u[32];
-                    tmem_ld_32x32b_x32(t0 + static_cast<uint32_t>(c * 32), g);
-                    if (GATED) tmem_ld_32x32b_x32(t0 + static_cast<uint32_t>(TN / 2 + c * 32), u);
-                    tmem_ld_wait();
-                    const int n = n_base + c * 32;
-                    if (m_local < at.valid && n < p.n_out) {
-                        float v[32];
-    #pragma unroll
-                        for (int j = 0; j < 32; ++j) {
-                            if (GATED) {
-                                const float gv = round_bf16(__uint_as_float(g[j]));
-                                const float uv = round_bf16(__uint_as_float(u[j]));
-                                v[j] = EPI == B200_EPILOGUE_CLAMPED_SWIGLU ? clamped_swiglu<false>(gv, uv, p.act_limit)
-                                                                           : gated_act_tile<EPI>(gv) * uv;
-                            } else {
-                                v[j] = __uint_as_float(g[j]);
-                            }
-                        }
-                        if (!GATED && p.bias) {
-    #pragma unroll
-                            for (int j = 0; j < 32; ++j)
-                                if (n + j < p.n_out) v[j] += __bfloat162float(p.bias[n + j]);
-                        }
-                        if (EPI == B200_EPILOGUE_RELU2) {
-    #pragma unroll
-                            for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.f) * fmaxf(v[j], 0.f);
-                        }
-                        if (EPI == B200_EPILOGUE_GELU_ERF) {
-    #pragma unroll
-                            for (int j = 0; j < 32; ++j) v[j] = 0.5f * v[j] * (1.0f + erff(v[j] * 0.70710678118654752f));
-                        }
-                        if (EPI == B200_EPILOGUE_F32) {
-                            float* frow = reinterpret_cast<float*>(p.y) + static_cast<int64_t>(m) * p.n_out;
-    #pragma unroll
-                            for (int j = 0; j < 32; j += 4)
-                                if (n + j < p.n_out)
-                                    *reinterpret_cast<float4*>(frow + n + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-                            continue;
-                        }
-    #pragma unroll
-                        for (int j = 0; j < 32; j += 8) {
-                            if (n + j < p.n_out) {  // n_out is a multiple of 8: whole 16-byte groups
-                                uint4 o;
-                                o.x = pack_bf16(v[j], v[j + 1]);
-                                o.y = pack_bf16(v[j + 2], v[j + 3]);
-                                o.z = pack_bf16(v[j + 4], v[j + 5]);
-                                o.w = pack_bf16(v[j + 6], v[j + 7]);
-                                *reinterpret_cast<uint4*>(yrow + n + j) = o;
-                            }
-                        }
-                    }
+    const int m_local = q * 32 + lane;
+    const int m = at.row0 + m_local;
+    const uint32_t t0 = tmem_acc + (static_cast<uint32_t>(q * 32) << 16);
+    constexpr int kOutCols = GATED ? TN / 2 : TN;
+    const int n_base = at.n0;
+    __nv_bfloat16* yrow = p.y + static_cast<int64_t>(m) * p.n_out;
+#pragma unroll 1
+    for (int c = 0; c < kOutCols / 32; ++c) {
+        uint32_t g[32], u[32];
+        tmem_ld_32x32b_x32(t0 + static_cast<uint32_t>(c * 32), g);
+        if (GATED) tmem_ld_32x32b_x32(t0 + static_cast<uint32_t>(TN / 2 + c * 32), u);
+        tmem_ld_wait();
+        const int n = n_base + c * 32;
+        if (m_local < at.valid && n < p.n_out) {
+            float v[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+                if (GATED) {
+                    const float gv = round_bf16(__uint_as_float(g[j]));
+                    const float uv = round_bf16(__uint_as_float(u[j]));
+                    v[j] = EPI == B200_EPILOGUE_CLAMPED_SWIGLU ? clamped_swiglu<false>(gv, uv, p.act_limit)
+                                                               : gated_act_tile<EPI>(gv) * uv;
+                } else {
+                    v[j] = __uint_as_float(g[j]);
                 }
+            }
+            if (!GATED && p.bias) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j)
+                    if (n + j < p.n_out) v[j] += __bfloat162float(p.bias[n + j]);
+            }
+            if (EPI == B200_EPILOGUE_RELU2) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.f) * fmaxf(v[j], 0.f);
+            }
+            if (EPI == B200_EPILOGUE_GELU_ERF) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = 0.5f * v[j] * (1.0f + erff(v[j] * 0.70710678118654752f));
+            }
+            if (EPI == B200_EPILOGUE_F32) {
+                float* frow = reinterpret_cast<float*>(p.y) + static_cast<int64_t>(m) * p.n_out;
+#pragma unroll
+                for (int j = 0; j < 32; j += 4)
+                    if (n + j < p.n_out)
+                        *reinterpret_cast<float4*>(frow + n + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                continue;
+            }
+#pragma unroll
+            for (int j = 0; j < 32; j += 8) {
+                if (n + j < p.n_out) {  // n_out is a multiple of 8: whole 16-byte groups
+                    uint4 o;
+                    o.x = pack_bf16(v[j], v[j + 1]);
+                    o.y = pack_bf16(v[j + 2], v[j + 3]);
+                    o.z = pack_bf16(v[j + 4], v[j + 5]);
+                    o.w = pack_bf16(v[j + 6], v[j + 7]);
+                    *reinterpret_cast<uint4*>(yrow + n + j) = o;
+                }
+            }
+        }
+    }
 }
 
 template <int EPI>

@@ -120,6 +120,10 @@ struct NarrowFusion {
 bool narrow_gemm_takes(const void* x, const void* w, int M, int N, int K, int64_t ldx, int epilogue);
 int launch_narrow_gemm(void* y, const void* x, const void* w, const void* bias, int M, int N, int K, int64_t ldx, int epilogue,
                        int* status, cudaStream_t stream, const NarrowFusion* fuse = nullptr, float act_limit = 0.f);
+// Expert GEMMs (launch_grouped_gemm) of about that many rows per expert.
+bool narrow_grouped_takes(const void* x, const void* w, int64_t total_rows, int num_groups, int n_out, int K);
+int launch_narrow_grouped(void* y, const void* x, const void* w, const int32_t* counts, const int32_t* offsets, int num_groups, int N,
+                          int K, int epilogue, cudaStream_t stream, float act_limit);
 // The K split launch_linear picks for a slab of this shape (the fusions need it above 1).
 int skinny_gemm_split(int M, int N, int K, int epilogue);
 

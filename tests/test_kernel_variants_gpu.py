@@ -77,6 +77,13 @@ def test_experts_of_one_pair_tile(L, T, E, k):
     moe_forward(L, T, E, k, 128, 192, True, "silu")
 
 
+@pytest.mark.parametrize("T,E,k,H,I,act", [(32, 16, 4, 2048, 1024, "silu"), (1, 64, 4, 1088, 64, "silu"), (9, 3, 1, 64, 192, "gelu"),
+                                           (24, 12, 4, 1024, 2048, "silu")])
+def test_experts_of_a_handful_of_rows(L, T, E, k, H, I, act):
+    """At most 8 rows per expert on average, some with more and some with none; K of one and of two register buffers."""
+    moe_forward(L, T, E, k, H, I, True, act)
+
+
 @pytest.mark.parametrize("rows", [1023, 1024, 1027])
 @pytest.mark.parametrize("hidden", [512, 768, 1024, 1536, 2048, 2560])
 def test_norms_of_many_rows(L, rows, hidden):
