@@ -394,6 +394,9 @@ int enqueue_forward(b200_engine* e, int phase, int B, int Bp, int T, int max_ext
     const bool heads_in_qkv = e->use_fold_heads && d == 128 && T <= 128 && !tp &&
                               skinny_gemm_split(T, e->qkv_dim, hidden, B200_EPILOGUE_NONE) > 1;
 
+    const bool heads_few = e->use_fold && e->use_fold_heads && d == 128 && !tp &&
+                           narrow_gemm_takes(nullptr, nullptr, T, e->qkv_dim, hidden, hidden, B200_EPILOGUE_NONE);
+
     // Decode batches of at most 64 tokens of a dense, unsharded model: everything between two attention
     // launches is one persistent kernel (decode_chain.cu) instead of seven launches.
     const bool chain = !fold && phase == B200_PHASE_DECODE && e->use_chain && !tp && m.num_experts == 0 &&
@@ -575,7 +578,13 @@ int enqueue_forward(b200_engine* e, int phase, int B, int Bp, int T, int max_ext
         B200_TRY(add_norm(L.input_norm));
         HeadEpilogue he;
         fill_heads(he, l);
-        if (heads_in_qkv) {
+        if (heads_few) {
+            // (MoE engines, a handful of requests: the same kernel as below, on normalised rows)
+            NarrowFusion with_heads;
+            with_heads.heads = &he;
+            B200_TRY(launch_narrow_gemm(e->qkv, e->x, L.qkv, L.qkv_bias, T, e->qkv_dim, hidden, hidden, B200_EPILOGUE_NONE, e->status,
+                                        s, &with_heads));
+        } else if (heads_in_qkv) {
             // (sharded and MoE engines, short prefill batches: the head epilogue alone, on normalised rows)
             SkinnyFusion with_heads;
             with_heads.heads = &he;

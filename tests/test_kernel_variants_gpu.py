@@ -78,7 +78,7 @@ def test_experts_of_one_pair_tile(L, T, E, k):
 
 
 @pytest.mark.parametrize("T,E,k,H,I,act", [(32, 16, 4, 2048, 1024, "silu"), (1, 64, 4, 1088, 64, "silu"), (9, 3, 1, 64, 192, "gelu"),
-                                           (24, 12, 4, 1024, 2048, "silu")])
+                                           (24, 16, 4, 1024, 2048, "silu")])
 def test_experts_of_a_handful_of_rows(L, T, E, k, H, I, act):
     """At most 8 rows per expert on average, some with more and some with none; K of one and of two register buffers."""
     moe_forward(L, T, E, k, H, I, True, act)
