@@ -545,7 +545,9 @@ struct TilePick {
 };
 TilePick pick_tile(int M, int n_out, bool gated, int kb) {
     const char* forced = getenv("B200_TILE_TN");
-    if (forced && *forced) return {atoi(forced), 0.f};
+    if (forced && *forced)
+        for (int tn : {0, 64, 128, 192, 256})
+            if (atoi(forced) == tn) return {tn, 0.f};
     const int sms = sm_count(), per = gated ? 2 : 1;
     auto cost = [&](int tm, int tn, int slots, float each, float once) {
         return static_cast<float>(div_ceil(div_ceil(M, tm) * div_ceil(n_out * per, tn), slots)) * kb * each + once;
