@@ -1,5 +1,5 @@
-// y = x W^T for few rows (decode batches, M <= 256): a weight-streaming GEMM on
-// the tcgen05 tensor cores.
+// y = x W^T for few rows (decode batches, M <= 256; a handful of them mostly in gemm_narrow.cu): a
+// weight-streaming GEMM on the tcgen05 tensor cores.
 //
 // The kernel is bound by reading W once from HBM, so the layout is chosen for
 // bytes in flight rather than for tensor-core occupancy:

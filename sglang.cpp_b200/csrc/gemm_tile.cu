@@ -11,6 +11,7 @@
 //   * gated epilogue (gate_up projection + SwiGLU): the B operand is 128 gate rows followed by
 //     the 128 matching up rows, so one thread holds gate[m][n] and up[m][n] in the same
 //     accumulator and writes act(gate) * up for 128 features.
+// Most batches run on pairs of CTAs instead (pair_gemm_kernel below); pick_tile has the line.
 #include <math.h>
 
 #include "common.cuh"
