@@ -456,6 +456,14 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
                     if (it >= early) tma_load_2d_pair(dst + kABytes, &tmap_w, kb * kBK, w_row, bar);
                 }
             }
+            // Neither CTA may end while something is under way to its memory: the last commits' arrivals at the "empty"
+            // barriers (nothing orders them before the accumulator's, which the epilogue waits for); or, where a wait ran
+            // out, the copies themselves, of both CTAs (the first one sees them all, and the second one waits for it below).
+            for (int i = it > STAGES ? it - STAGES : 0; i < it; ++i) {
+                const uint32_t par = static_cast<uint32_t>(i / STAGES) & 1u;
+                if (!failed && !mbar_wait_bounded(smem_u32(&empty_bar[i % STAGES]), par, p.status, 125)) failed = true;
+                if (failed && (rank > 0 || !mbar_wait_bounded(smem_u32(&full_bar[i % STAGES]), par, p.status, 126))) break;
+            }
         }
     } else if (warp == 1) {
         if (rank == 0 && elect_one()) {

@@ -61,6 +61,22 @@ def test_tiles_of_every_width(L, pkg, monkeypatch, tile, M, N, K):
     assert L.read_device_status() == (0, 0)
 
 
+@pytest.mark.parametrize("tile", [64, 128, 192, 256])
+@pytest.mark.parametrize("K", [64, 384, 832])
+def test_pairs_of_ctas_one_after_another(L, monkeypatch, tile, K):
+    """Launches that follow each other at once, with fewer k-blocks than the ring has stages, and more: a CTA of the next launch
+    takes the shared memory of one that has ended, which nothing may still be writing to."""
+    monkeypatch.setenv("B200_TILE_TN", str(tile))
+    gen = torch.Generator().manual_seed(K)
+    x, w = randn_bf16(gen, 700, K), randn_bf16(gen, 3, 1032, K, std=0.05)
+    xs, ws = x.cuda(), w.cuda()
+    ys = [L.linear(xs, ws[i % 3]) for i in range(60)]
+    for i in range(3):
+        assert_close_bf16(ys[i], O.linear(x, w[i]), BIG[0] * (K / 1024) ** 0.5 + BIG[1], RTOL, "first")
+        assert all(torch.equal(ys[i], y) for y in ys[i::3])
+    assert L.read_device_status() == (0, 0)
+
+
 @pytest.mark.parametrize("M,N,K,gated", [(65, 6144, 1024, True), (100, 4096, 1024, False), (181, 6144, 1024, True), (256, 1024, 2048, False)])
 def test_batches_that_either_kernel_takes(L, pkg, monkeypatch, M, N, K, gated):
     gen = torch.Generator().manual_seed(M)
