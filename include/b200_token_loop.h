@@ -372,6 +372,14 @@ B200_API int b200_linear_f32(float* y, const float* x, const float* w, int max_r
 B200_API int b200_linear_act(void* y, const void* x, const void* w, int M, int N, int K, int epilogue,
                              float act_limit, int dtype, b200_stream_t stream);
 
+/* The kernel that b200_linear (groups 0) or the expert projections (rows of all `groups` experts together, at most max_rows of
+ * them one expert's) run on for a shape with aligned operands; 0: no such shape.  Nothing is launched; needs no device. */
+#define B200_GEMM_NARROW 1   /* weights from memory to registers: a handful of rows */
+#define B200_GEMM_STREAM 2   /* weights through shared memory, split along K: a decode batch */
+#define B200_GEMM_TILE 3     /* tiles of single CTAs */
+#define B200_GEMM_PAIR 4     /* tiles of pairs of CTAs */
+B200_API int b200_gemm_kernel(int64_t rows, int N, int K, int epilogue, int groups, int max_rows);
+
 /* The wiring with the norm on what a block returned (layer_norm below: the same with layer norms):
  *   a = sum_k src_weights[t, k] src[src_rows[t, k], :] + src2[t, :]   (src_rows NULL: src[t, :]; weights NULL: 1),
  *   residual[t, :] += a / sqrt(mean(a^2) + eps) * add_weight          (add_weight NULL: += a; init: = instead of +=),

@@ -809,6 +809,10 @@ int launch_skinny_gemm(void* y, const void* x, const void* w, const void* bias, 
     return B200_OK;
 }
 
+static bool grouped_on_tiles(int64_t total_rows, int num_groups) {
+    return total_rows >= static_cast<int64_t>(num_groups) * env_int("B200_GROUPED_TILE_MIN_ROWS", 128) && num_groups <= 256;
+}
+
 // Grouped GEMM for expert layers: group g multiplies rows [offsets[g], offsets[g] + counts[g]) of
 // x [total_rows, K] by w[g] ([N, K], groups stacked) into the same rows of y.  counts / offsets
 // are device arrays (no host synchronisation); max_rows_per_group bounds any count.
@@ -824,10 +828,10 @@ int launch_grouped_gemm(void* y, const void* x, const void* w, const int32_t* co
     const int slabs = div_ceil(max_rows_per_group, 256);
     if (num_groups == 0 || slabs == 0 || total_rows == 0) return B200_OK;
     // A handful of rows per group: weights straight into registers.
-    if (narrow_grouped_takes(x, w, total_rows, num_groups, n_out, K))
+    if (narrow_grouped_takes(x, w, total_rows, max_rows_per_group, num_groups, n_out, K, epilogue))
         return launch_narrow_grouped(y, x, w, counts, offsets, num_groups, N, K, epilogue, stream, act_limit);
     // Many rows per group on average (prefill batches): tensor-bound, take the tile kernel.
-    if (total_rows >= static_cast<int64_t>(num_groups) * env_int("B200_GROUPED_TILE_MIN_ROWS", 128) && num_groups <= 256)
+    if (grouped_on_tiles(total_rows, num_groups))
         return launch_grouped_tile_gemm(y, x, w, counts, offsets, num_groups, total_rows, N, K, epilogue, status,
                                         stream, act_limit);
     int nt_max = 32;
@@ -940,6 +944,28 @@ static float skinny_gemm_us(int M, int N, int K, int epilogue) {
     return static_cast<float>(N) * K * 2e-6f / 5.7f + 5.f + (epilogue_is_gated(epilogue) ? 4.2f : 1.9f) * div_ceil(M, kRoundCols);
 }
 
+// Do tiles take this many rows?  (They are stored 16 bytes at a time.)
+static bool linear_on_tiles(const void* y, int M, int N, int K, int epilogue, bool fused) {
+    const int tile_min = env_int("B200_GEMM_TILE_MIN_M", 257);
+    const bool whole_vectors = (epilogue_is_gated(epilogue) ? N / 2 : N) % 8 == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0;
+    const bool tiles_faster = tile_min == 257 && !fused && M > kRoundCols && whole_vectors &&
+                              tile_gemm_us(M, N, K, epilogue) < 0.9f * skinny_gemm_us(M, N, K, epilogue);
+    return M >= tile_min || tiles_faster;
+}
+
+int gemm_kernel_of(int64_t rows, int N, int K, int epilogue, int groups, int max_rows) {
+    const int n_out = epilogue_is_gated(epilogue) ? N / 2 : N;
+    if (groups == 0) {
+        const int M = static_cast<int>(rows);
+        if (narrow_gemm_takes(nullptr, nullptr, M, N, K, K, epilogue)) return B200_GEMM_NARROW;
+        if (!linear_on_tiles(nullptr, M, N, K, epilogue, false)) return B200_GEMM_STREAM;
+        return tile_gemm_features(M, N, K, epilogue) > 0 ? B200_GEMM_PAIR : B200_GEMM_TILE;
+    }
+    if (narrow_grouped_takes(nullptr, nullptr, rows, max_rows, groups, n_out, K, epilogue)) return B200_GEMM_NARROW;
+    if (!grouped_on_tiles(rows, groups)) return B200_GEMM_STREAM;
+    return grouped_on_pairs(rows, groups) ? B200_GEMM_PAIR : B200_GEMM_TILE;
+}
+
 int launch_linear(void* y, const void* x, const void* w, const void* bias, int M, int N, int K,
                   int64_t ldx, int epilogue, int* status, cudaStream_t stream, const SkinnyFusion* fuse,
                   float act_limit, bool narrow) {
@@ -947,12 +973,7 @@ int launch_linear(void* y, const void* x, const void* w, const void* bias, int M
     if (narrow && fuse == nullptr && narrow_gemm_takes(x, w, M, N, K, ldx, epilogue))
         return launch_narrow_gemm(y, x, w, bias, M, N, K, ldx, epilogue, status, stream, nullptr, act_limit);
     // Few rows: stream the weights once (swap-AB, split-K).  Many rows: tensor-bound tiles.
-    const int tile_min = env_int("B200_GEMM_TILE_MIN_M", 257);
-    // (tiles are stored 16 bytes at a time)
-    const bool whole_vectors = (epilogue_is_gated(epilogue) ? N / 2 : N) % 8 == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0;
-    const bool tiles_faster = tile_min == 257 && fuse == nullptr && M > kRoundCols && whole_vectors &&
-                              tile_gemm_us(M, N, K, epilogue) < 0.9f * skinny_gemm_us(M, N, K, epilogue);
-    if (M >= tile_min || tiles_faster) {
+    if (linear_on_tiles(y, M, N, K, epilogue, fuse != nullptr)) {
         if (fuse != nullptr) {
             set_last_error("linear: the residual-stream fusions need at most 256 rows");
             return B200_ERR_UNSUPPORTED;
@@ -987,6 +1008,12 @@ int b200_linear_heads(void* y, const void* x, const void* w, int M, int heads, i
     int* status = b200::device_status_words(&err);
     if (err != B200_OK) return err;
     return b200::launch_linear_heads(y, x, w, M, heads, N, K, status, static_cast<cudaStream_t>(stream));
+}
+
+int b200_gemm_kernel(int64_t rows, int N, int K, int epilogue, int groups, int max_rows) {
+    const bool shape = rows > 0 && rows <= INT32_MAX && N > 0 && K > 0 && K % 64 == 0 && groups >= 0 && (groups == 0 || max_rows > 0);
+    const bool known = epilogue >= B200_EPILOGUE_NONE && epilogue <= B200_EPILOGUE_F32;
+    return shape && known ? b200::gemm_kernel_of(rows, N, K, epilogue, groups, max_rows) : 0;
 }
 
 int b200_linear_act(void* y, const void* x, const void* w, int M, int N, int K, int epilogue, float act_limit, int dtype,

@@ -596,6 +596,19 @@ float tile_gemm_us(int M, int N, int K, int epilogue) {
     return fmaxf(pick_tile(M, gated ? N / 2 : N, gated, K / kBK).us, static_cast<float>(N) * K * 2e-6f / 5.7f) + 1.f;
 }
 
+int tile_gemm_features(int M, int N, int K, int epilogue) {
+    const bool gated = epilogue_is_gated(epilogue);
+    return pick_tile(M, gated ? N / 2 : N, gated, K / kBK).tn;
+}
+
+// Blocks of 128 tokens on one CTA each, or of 256 on a pair: what a group's rows come to in either, where groups differ by a
+// seventh (64 groups of 189 rows, 2048 x 2048 and 1024 x 2048: a layer of 430 us against 456).
+bool grouped_on_pairs(int64_t total_rows, int num_groups) {
+    const float rows = static_cast<float>(total_rows) / num_groups;
+    auto blocks = [&](float per) { return ceilf(rows * 0.85f / per) + ceilf(rows * 1.15f / per); };
+    return 0.80f * blocks(kPairM) < 0.44f * blocks(kTM);
+}
+
 int launch_tile_gemm(void* y, const void* x, const void* w, const void* bias, int M, int N, int K,
                      int64_t ldx, int epilogue, int* status, cudaStream_t stream, float act_limit) {
     const bool gated = epilogue_is_gated(epilogue);
@@ -676,11 +689,7 @@ int launch_grouped_tile_gemm(void* y, const void* x, const void* w, const int32_
     p.num_groups = num_groups;
     p.w_rows_per_group = N;
     p.act_limit = act_limit;
-    // Blocks of 128 tokens on one CTA each, or of 256 on a pair: what a group's rows come to in either, where groups differ
-    // by a seventh (64 groups of 189 rows, 2048 x 2048 and 1024 x 2048: a layer of 430 us against 456).
-    const float rows = static_cast<float>(total_rows) / num_groups;
-    auto blocks = [&](float per) { return ceilf(rows * 0.85f / per) + ceilf(rows * 1.15f / per); };
-    if (0.80f * blocks(kPairM) < 0.44f * blocks(kTM))
+    if (grouped_on_pairs(total_rows, num_groups))
         return launch_pairs(p, kTN, x, w, total_rows, static_cast<int64_t>(num_groups) * N, K, K, sm_count() / 2, stream);
     CUtensorMap tmap_x, tmap_w;
     int err = cached_tmap(&tmap_x, x, static_cast<uint64_t>(K), static_cast<uint64_t>(total_rows),

@@ -1,0 +1,33 @@
+"""Which kernel a projection runs on: shapes on either side of each rule's line, where both kernels were timed."""
+import pytest
+
+NARROW, STREAM, TILE, PAIR = 1, 2, 3, 4
+PLAIN, SWIGLU = 0, 1
+
+
+def experts(lib, tokens, experts, per_token, hidden, inter):
+    """The kernels of an expert layer's two projections."""
+    return (lib.b200_gemm_kernel(tokens * per_token, 2 * inter, hidden, SWIGLU, experts, tokens),
+            lib.b200_gemm_kernel(tokens * per_token, hidden, inter, PLAIN, experts, tokens))
+
+
+@pytest.mark.parametrize("shape,hidden,inter,narrow,not_narrow", [
+    ((64, 4), 2048, 1024, (1, 8, 16, 32), (64, 96, 128)),
+    ((128, 8), 2048, 768, (1, 8), (24, 32, 64, 128)),
+    ((32, 2), 2048, 1024, (8, 32, 64), (128,)),
+    ((16, 4), 1024, 2048, (1, 8, 16, 32), (33, 64)),
+    ((8, 2), 1024, 1024, (4, 16, 32), (33,)),
+])
+def test_experts_whose_tokens_may_all_choose_alike(pkg, shape, hidden, inter, narrow, not_narrow):
+    """A CTA of the narrow kernel takes an expert's rows 8 at a time: it is left as soon as a batch in which every token chooses
+    the same experts would be slower on it."""
+    lib = pkg.load_library()
+    for tokens in narrow:
+        assert experts(lib, tokens, *shape, hidden, inter) == (NARROW, NARROW), tokens
+    for tokens in not_narrow:
+        assert NARROW not in experts(lib, tokens, *shape, hidden, inter), tokens
+
+
+def test_shapes_that_no_kernel_takes(pkg):
+    lib = pkg.load_library()
+    assert [lib.b200_gemm_kernel(*a) for a in [(0, 64, 64, 0, 0, 0), (4, 64, 96, 0, 0, 0), (4, 64, 64, 99, 0, 0), (4, 64, 64, 0, 2, 0)]] == [0] * 4
