@@ -196,15 +196,14 @@ bool fold_supported(const b200_engine* e, int phase, int T) {
 
 // Can this step run on the projections for a handful of rows, which carry the norms, the residual and the head operations
 // themselves?  A dense, unsharded model; where the norms of the other path read the sum before it is rounded, only if that
-// path would be the folded one, which does not either.  Every CTA normalises x for itself: beside the weights of a wide
-// model's projections that is too much (one layer of hidden 4096, 4 requests, in a step: 173 us against 120).
+// path would be the folded one, which does not either.
 bool narrow_supported(const b200_engine* e, int phase, int T) {
     const int H = e->m.hidden_size, D = e->m.head_dim;
-    auto takes = [&](int N, int K, int epilogue) { return narrow_gemm_takes(nullptr, nullptr, T, N, K, K, epilogue); };
+    auto takes = [&](int N, int K, int epilogue, bool normed) { return narrow_gemm_takes(nullptr, nullptr, T, N, K, K, epilogue, normed); };
     return e->use_fold && !e->use_chain && phase == B200_PHASE_DECODE && e->c.tp_size == 1 && e->m.num_experts == 0 && D == 128 &&
-           H <= 2048 && (e->m.fused_residual == 0 || e->ssq != nullptr) && takes(e->qkv_dim, H, B200_EPILOGUE_NONE) &&
-           takes(H, e->hq * D, B200_EPILOGUE_NONE) && takes(2 * e->inter, H, B200_EPILOGUE_SWIGLU) &&
-           takes(H, e->inter, B200_EPILOGUE_NONE);
+           (e->m.fused_residual == 0 || e->ssq != nullptr) && takes(e->qkv_dim, H, B200_EPILOGUE_NONE, true) &&
+           takes(H, e->hq * D, B200_EPILOGUE_NONE, false) && takes(2 * e->inter, H, B200_EPILOGUE_SWIGLU, true) &&
+           takes(H, e->inter, B200_EPILOGUE_NONE, false);
 }
 
 // Rebuilds the folded weight copies after a weight was loaded.  Enqueued on the engine's stream, never

@@ -392,8 +392,14 @@ cudaError_t launch(const NarrowParams& p, int tiles, cudaStream_t stream) {
 // Two tiles of tokens double a warp's operands and products, and a long K is walked a buffer at a time behind the wait,
 // where the TMA ring of gemm_skinny.cu keeps more bytes in flight (us, this against that, 16 rows: 6144 x 1024 5.0 and 8.7,
 // 2048 x 6144 8.8 and 14.4, 12288 x 2048 18.6 and 16.1; 4 rows of 28672 x 4096 43 and 45, but 57 and 44 with the norm).
-bool narrow_gemm_takes(const void* x, const void* w, int M, int N, int K, int64_t ldx, int epilogue) {
+// With the norm (and the chain of a decode step around it: the residual, the heads), every CTA computes it, which grows with K
+// and with the CTAs: a step of 12 layers against the split-K kernel with folded norms (us)
+//   hidden 768   1 request 254, 371   8: 279, 401   16: 312, 409     hidden 1024, gate and up of 16 MB   1: 330, 412   8: 356, 438   16: 428, 444
+//   hidden 1280  1 request 407, 475   8: 479, 491   16: 654, 498     ... of 32 MB   1: 414, 508   4: 502, 524   8: 564, 548
+//   hidden 2048  1 request 636, 650   4: 693, 675   8: 709, 695
+bool narrow_gemm_takes(const void* x, const void* w, int M, int N, int K, int64_t ldx, int epilogue, bool normed) {
     const int64_t bytes = static_cast<int64_t>(N) * K * 2;
+    if (normed && (K > (M <= 2 ? 2048 : 1024) || (M > 4 && bytes > (18ll << 20)))) return false;
     const int n_out = epilogue_is_gated(epilogue) ? N / 2 : N;
     const bool faster = (M <= 8 && K <= 2048) || (M <= kNarrowRows && bytes <= (26ll << 20));
     return M >= 1 && faster && n_out % 8 == 0 && K % 32 == 0 && ldx % 8 == 0 &&

@@ -953,11 +953,11 @@ static bool linear_on_tiles(const void* y, int M, int N, int K, int epilogue, bo
     return M >= tile_min || tiles_faster;
 }
 
-int gemm_kernel_of(int64_t rows, int N, int K, int epilogue, int groups, int max_rows) {
+int gemm_kernel_of(int64_t rows, int N, int K, int epilogue, int groups, int max_rows, bool normed) {
     const int n_out = epilogue_is_gated(epilogue) ? N / 2 : N;
     if (groups == 0) {
         const int M = static_cast<int>(rows);
-        if (narrow_gemm_takes(nullptr, nullptr, M, N, K, K, epilogue)) return B200_GEMM_NARROW;
+        if (narrow_gemm_takes(nullptr, nullptr, M, N, K, K, epilogue, normed)) return B200_GEMM_NARROW;
         if (!linear_on_tiles(nullptr, M, N, K, epilogue, false)) return B200_GEMM_STREAM;
         return tile_gemm_features(M, N, K, epilogue) > 0 ? B200_GEMM_PAIR : B200_GEMM_TILE;
     }
@@ -1010,10 +1010,10 @@ int b200_linear_heads(void* y, const void* x, const void* w, int M, int heads, i
     return b200::launch_linear_heads(y, x, w, M, heads, N, K, status, static_cast<cudaStream_t>(stream));
 }
 
-int b200_gemm_kernel(int64_t rows, int N, int K, int epilogue, int groups, int max_rows) {
+int b200_gemm_kernel(int64_t rows, int N, int K, int epilogue, int groups, int max_rows, int normed) {
     const bool shape = rows > 0 && rows <= INT32_MAX && N > 0 && K > 0 && K % 64 == 0 && groups >= 0 && (groups == 0 || max_rows > 0);
     const bool known = epilogue >= B200_EPILOGUE_NONE && epilogue <= B200_EPILOGUE_F32;
-    return shape && known ? b200::gemm_kernel_of(rows, N, K, epilogue, groups, max_rows) : 0;
+    return shape && known ? b200::gemm_kernel_of(rows, N, K, epilogue, groups, max_rows, normed != 0) : 0;
 }
 
 int b200_linear_act(void* y, const void* x, const void* w, int M, int N, int K, int epilogue, float act_limit, int dtype,

@@ -121,15 +121,16 @@ struct NarrowFusion {
     const HeadEpilogue* heads = nullptr;
 };
 // Is that kernel possible, and the faster one?
-bool narrow_gemm_takes(const void* x, const void* w, int M, int N, int K, int64_t ldx, int epilogue);
+bool narrow_gemm_takes(const void* x, const void* w, int M, int N, int K, int64_t ldx, int epilogue, bool normed = false);
 int launch_narrow_gemm(void* y, const void* x, const void* w, const void* bias, int M, int N, int K, int64_t ldx, int epilogue,
                        int* status, cudaStream_t stream, const NarrowFusion* fuse = nullptr, float act_limit = 0.f);
 // Expert GEMMs (launch_grouped_gemm) of about that many rows per expert, whichever experts the rows choose.
 bool narrow_grouped_takes(const void* x, const void* w, int64_t total_rows, int max_rows, int num_groups, int n_out, int K, int epilogue);
 int launch_narrow_grouped(void* y, const void* x, const void* w, const int32_t* counts, const int32_t* offsets, int num_groups, int N,
                           int K, int epilogue, cudaStream_t stream, float act_limit);
-// The kernel (B200_GEMM_*) of launch_linear (groups 0) or launch_grouped_gemm with aligned operands and nothing fused.
-int gemm_kernel_of(int64_t rows, int N, int K, int epilogue, int groups, int max_rows);
+// The kernel (B200_GEMM_*) of launch_linear (groups 0) or launch_grouped_gemm with aligned operands and nothing fused but,
+// where asked for, the norm of the rows of x in a decode step.
+int gemm_kernel_of(int64_t rows, int N, int K, int epilogue, int groups, int max_rows, bool normed);
 // The K split launch_linear picks for a slab of this shape (the fusions need it above 1).
 int skinny_gemm_split(int M, int N, int K, int epilogue);
 

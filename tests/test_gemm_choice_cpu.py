@@ -7,8 +7,8 @@ PLAIN, SWIGLU = 0, 1
 
 def experts(lib, tokens, experts, per_token, hidden, inter):
     """The kernels of an expert layer's two projections."""
-    return (lib.b200_gemm_kernel(tokens * per_token, 2 * inter, hidden, SWIGLU, experts, tokens),
-            lib.b200_gemm_kernel(tokens * per_token, hidden, inter, PLAIN, experts, tokens))
+    return (lib.b200_gemm_kernel(tokens * per_token, 2 * inter, hidden, SWIGLU, experts, tokens, 0),
+            lib.b200_gemm_kernel(tokens * per_token, hidden, inter, PLAIN, experts, tokens, 0))
 
 
 @pytest.mark.parametrize("shape,hidden,inter,narrow,not_narrow", [
@@ -28,6 +28,16 @@ def test_experts_whose_tokens_may_all_choose_alike(pkg, shape, hidden, inter, na
         assert NARROW not in experts(lib, tokens, *shape, hidden, inter), tokens
 
 
+@pytest.mark.parametrize("hidden,narrow,not_narrow", [(768, (1, 8, 9, 16), (17,)), (1024, (1, 8, 9, 16), (17,)),
+                                                      (1280, (1, 2), (3, 8, 9, 16)), (2048, (1, 2), (4, 8, 9, 16)), (2304, (), (1, 2, 16))])
+def test_projections_that_carry_the_norm(pkg, hidden, narrow, not_narrow):
+    lib = pkg.load_library()
+    for rows, kernel in [(r, NARROW) for r in narrow] + [(r, STREAM) for r in not_narrow]:
+        for N, epilogue in ((2 * hidden, PLAIN), (4 * hidden, SWIGLU)):
+            assert lib.b200_gemm_kernel(rows, N, hidden, epilogue, 0, 0, 1) == kernel, (rows, N)
+    assert [lib.b200_gemm_kernel(rows, 16384, 1024, SWIGLU, 0, 0, 1) for rows in (4, 5, 8)] == [NARROW, STREAM, STREAM]
+
+
 def test_shapes_that_no_kernel_takes(pkg):
     lib = pkg.load_library()
-    assert [lib.b200_gemm_kernel(*a) for a in [(0, 64, 64, 0, 0, 0), (4, 64, 96, 0, 0, 0), (4, 64, 64, 99, 0, 0), (4, 64, 64, 0, 2, 0)]] == [0] * 4
+    assert [lib.b200_gemm_kernel(*a) for a in [(0, 64, 64, 0, 0, 0, 0), (4, 64, 96, 0, 0, 0, 0), (4, 64, 64, 99, 0, 0, 0), (4, 64, 64, 0, 2, 0, 0)]] == [0] * 4
