@@ -389,9 +389,16 @@ cudaError_t launch(const NarrowParams& p, int tiles, cudaStream_t stream) {
 
 }  // namespace
 
-// Two tiles of tokens double a warp's operands and products, and a long K is walked a buffer at a time behind the wait,
-// where the TMA ring of gemm_skinny.cu keeps more bytes in flight (us, this against that, 16 rows: 6144 x 1024 5.0 and 8.7,
-// 2048 x 6144 8.8 and 14.4, 12288 x 2048 18.6 and 16.1; 4 rows of 28672 x 4096 43 and 45, but 57 and 44 with the norm).
+// Plain projections, us, this kernel against the weight-streaming one of gemm_skinny.cu:
+//   * Up to 8 rows it is the faster one, but CTAs with little to load cost more than they bring: 151936 x 64 26 and 17 (2048 x 64
+//     2.0 and 3.8), and with K a little above 1024 half of the second register buffer stays empty: 32768 x 1088 21 and 17,
+//     32768 x 1536 23 and 22, 16384 x 1088 11.8 and 12.9; 32768 x 2048 with 4 rows 27 and 27.  In a chain of programmatic launches
+//     they load beside the kernels before: as the head of a decode step 32768 x 1536 is 10 us ahead, 32768 x 1280 3 to 7 behind.
+//   * A long K is walked a buffer at a time behind the wait, where the TMA ring over there keeps more bytes in flight: 2048 x 6144
+//     with 4 rows 8.9 and 14.4, 28672 x 4096 43 and 45; 12288 x 2048 with 16 rows 18.6 and 16.1.
+//   * Two tiles of tokens double a warp's operands and products; with more than 1024 columns and more CTAs than SMs it is ahead
+//     up to 6144 rows of W only (16 rows: 6144 x 1536 9.6 and 10.4, 8192 x 1536 12.0 and 11.2, with SwiGLU 12.1 and 10.4), with more
+//     than 2048 columns only without a gate (4096 x 3072 10.6 and 11.1; 3584 x 3584 with SwiGLU 11.1 and 10.8).
 // With the norm (and the chain of a decode step around it: the residual, the heads), every CTA computes it, which grows with K
 // and with the CTAs: a step of 12 layers against the split-K kernel with folded norms (us)
 //   hidden 768   1 request 254, 371   8: 279, 401   16: 312, 409     hidden 1024, gate and up of 16 MB   1: 330, 412   8: 356, 438   16: 428, 444
@@ -401,7 +408,15 @@ bool narrow_gemm_takes(const void* x, const void* w, int M, int N, int K, int64_
     const int64_t bytes = static_cast<int64_t>(N) * K * 2;
     if (normed && (K > (M <= 2 ? 2048 : 1024) || (M > 4 && bytes > (18ll << 20)))) return false;
     const int n_out = epilogue_is_gated(epilogue) ? N / 2 : N;
-    const bool faster = (M <= 8 && K <= 2048) || (M <= kNarrowRows && bytes <= (26ll << 20));
+    const bool light = bytes <= (26ll << 20);
+    bool faster;
+    if (N > 8192 && K < 512)
+        faster = false;
+    else if (M <= 8)
+        faster = K <= 1024 || light || (K <= 2048 && (N <= 16384 || (M <= 4 && K > 31 * 64) || (K >= 1536 && pdl_launches_enabled())));
+    else
+        faster = M <= kNarrowRows && light &&
+                 (K <= 1024 || div_ceil(N, 16) <= sm_count() || (K <= 2048 ? N <= 6144 : N <= 4096 && !epilogue_is_gated(epilogue)));
     return M >= 1 && faster && n_out % 8 == 0 && K % 32 == 0 && ldx % 8 == 0 &&
            ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
 }

@@ -38,6 +38,21 @@ def test_projections_that_carry_the_norm(pkg, hidden, narrow, not_narrow):
     assert [lib.b200_gemm_kernel(rows, 16384, 1024, SWIGLU, 0, 0, 1) for rows in (4, 5, 8)] == [NARROW, STREAM, STREAM]
 
 
+@pytest.mark.parametrize("N,K,epilogue,narrow,not_narrow", [
+    (4096, 1024, PLAIN, (1, 8, 9, 16), (17,)), (151936, 1024, PLAIN, (1, 8), (9,)), (12288, 1024, SWIGLU, (1, 8, 16), (17,)),
+    (2048, 64, PLAIN, (1, 8, 16), ()), (151936, 64, PLAIN, (), (1, 8, 16)), (151936, 256, PLAIN, (), (1, 8)), (151936, 512, PLAIN, (1, 8), ()),
+    (16384, 1088, SWIGLU, (1, 8), (9,)), (32768, 1088, PLAIN, (), (1, 8)), (32768, 1536, PLAIN, (), (1, 8)), (32768, 2048, PLAIN, (1, 4), (6, 8)),
+    (6144, 1536, SWIGLU, (9, 16), ()), (8192, 1536, PLAIN, (8,), (9, 16)), (8192, 1536, SWIGLU, (8,), (9, 16)), (12288, 1088, SWIGLU, (8,), (9,)),
+    (2048, 6144, PLAIN, (1, 16), ()), (4096, 3072, PLAIN, (8, 9, 16), ()), (3584, 3584, SWIGLU, (8,), (9, 16)), (4096, 4096, PLAIN, (), (1, 8, 16)),
+])
+def test_projections_of_a_handful_of_rows(pkg, N, K, epilogue, narrow, not_narrow):
+    lib = pkg.load_library()
+    for rows in narrow:
+        assert lib.b200_gemm_kernel(rows, N, K, epilogue, 0, 0, 0) == NARROW, rows
+    for rows in not_narrow:
+        assert lib.b200_gemm_kernel(rows, N, K, epilogue, 0, 0, 0) == STREAM, rows
+
+
 def test_shapes_that_no_kernel_takes(pkg):
     lib = pkg.load_library()
     assert [lib.b200_gemm_kernel(*a) for a in [(0, 64, 64, 0, 0, 0, 0), (4, 64, 96, 0, 0, 0, 0), (4, 64, 64, 99, 0, 0, 0), (4, 64, 64, 0, 2, 0, 0)]] == [0] * 4
