@@ -425,13 +425,13 @@ bool narrow_gemm_takes(const void* x, const void* w, int M, int N, int K, int64_
 // What this kernel gains by starting at once (two launches of a layer together 20 us) goes into CTAs of groups without rows,
 // 0.65 ns each, and into turns after a CTA's first 8 rows, 2.2 ns more than the 256 columns that the other kernel takes at once.
 // Layers (us, this kernel against the other one; rows spread at random, and all tokens with the same experts):
-//   64 experts of 2 x 1024 x 2048, 4 per token   32 tokens 152, 173 and 53, 56;   64: 170, 186 and 65, 61;   128: 185, 190 and 87, 70
+//   64 experts of 2 x 1024 x 2048, 4 per token   48 tokens 162, 182 and 58, 59;   64: 170, 186 and 65, 61;   128: 185, 190 and 87, 70
 //   128 of 2 x 768 x 2048, 8 per token            8 tokens 129, 148 and 68, 67;   32: 225, 238 and 82, 70;   128: 281, 276 and 136, 84
 //   32 of 2 x 1024 x 2048, 2 per token           64 tokens 96, 97 and 42, 53;    128: 104, 99 and 58, 61
 bool narrow_grouped_takes(const void* x, const void* w, int64_t total_rows, int max_rows, int num_groups, int n_out, int K, int epilogue) {
     const int64_t tiles = epilogue_is_gated(epilogue) ? div_ceil(n_out, 8) : div_ceil(n_out, 16);
     const int64_t turns = max_rows > 8 ? tiles * total_rows * (max_rows - 8) / (8ll * max_rows) : 0;
-    return 0.65 * tiles * num_groups + 2.2 * turns <= 10800. && total_rows <= 8ll * num_groups && num_groups <= 65535 && K <= 64 * 32 &&
+    return 0.65 * tiles * num_groups + 2.2 * turns <= 11000. && total_rows <= 8ll * num_groups && num_groups <= 65535 && K <= 64 * 32 &&
            K % 32 == 0 && n_out % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
 }
 

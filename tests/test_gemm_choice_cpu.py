@@ -12,7 +12,7 @@ def experts(lib, tokens, experts, per_token, hidden, inter):
 
 
 @pytest.mark.parametrize("shape,hidden,inter,narrow,not_narrow", [
-    ((64, 4), 2048, 1024, (1, 8, 16, 32), (64, 96, 128)),
+    ((64, 4), 2048, 1024, (1, 8, 16, 32, 48), (64, 96, 128)),
     ((128, 8), 2048, 768, (1, 8), (24, 32, 64, 128)),
     ((32, 2), 2048, 1024, (8, 32, 64), (128,)),
     ((16, 4), 1024, 2048, (1, 8, 16, 32), (33, 64)),
