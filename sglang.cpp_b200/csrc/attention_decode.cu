@@ -637,7 +637,9 @@ __device__ __forceinline__ int3 request_stages(const DecodeParams& p, int b) {
 }
 
 // SPLIT: a CTA's warps share the partials of one head instead (few requests with many partials: one request of 700 keys has
-// 22, whose rows one warp fetched 8 at a time: 4.6 us against 7.3).
+// 22, whose rows one warp fetched 8 at a time: 4.6 us against 7.3).  Where a request turns out to have no more than that, the
+// split only costs (a decode step of Qwen3-0.6B with 2 requests of 100 keys: 726 us with it, 676 without): its heads go back to a
+// warp each, and the CTAs left over end ahead of the wait (692; one of 40 keys 666, of 2000 keys 792 against 912 without).
 template <bool WINDOW, bool SPLIT>
 __global__ void __launch_bounds__(kMergeWarps * 32)
 attention_decode_merge_kernel(const DecodeParams p, int attn_grid) {
@@ -647,8 +649,7 @@ attention_decode_merge_kernel(const DecodeParams p, int attn_grid) {
     constexpr int kHeads = SPLIT ? 1 : kMergeWarps;   // per CTA
     const int ctas_per_req = (p.q_heads + kHeads - 1) / kHeads;
     const int b = static_cast<int>(blockIdx.x) / ctas_per_req;
-    const int head = (static_cast<int>(blockIdx.x) % ctas_per_req) * kHeads + (SPLIT ? 0 : warp);
-    const int row0 = SPLIT ? warp : 0, row_step = SPLIT ? kMergeWarps : 1;   // of 32 partials, this warp's
+    int head = (static_cast<int>(blockIdx.x) % ctas_per_req) * kHeads + (SPLIT ? 0 : warp);
     pdl_launch_dependents();
     // seq_lens were complete before the attention kernel started: the split runs ahead of the wait
     if (warp == 0) {
@@ -665,8 +666,15 @@ attention_decode_merge_kernel(const DecodeParams p, int attn_grid) {
     const int KG = kConsumerWarps / p.kv_heads;
     const int c0 = first / per;
     const int nparts = st > 0 ? ((first + st - 1) / per - c0 + 1) * KG : 0;
+    constexpr int kAhead = 8;                       // rows that a warp fetches at once
+    const bool shared = SPLIT && nparts > kAhead;   // (fewer: a warp per head after all, and every fourth CTA)
+    if (SPLIT && !shared) {
+        if (head % kMergeWarps > 0) return;
+        head += warp;
+    }
     pdl_wait_prior();
     if (nparts <= 1 || head >= p.q_heads) return;   // a single partial was written as bf16 by the kernel above
+    const int row0 = shared ? warp : 0, row_step = shared ? kMergeWarps : 1;   // of 32 partials, this warp's
     const int Hq = p.q_heads;
     const int64_t part0 = static_cast<int64_t>(b + c0) * KG;
     const float* ml = p.ws_ml + (part0 * Hq + head) * 2;
@@ -679,9 +687,9 @@ attention_decode_merge_kernel(const DecodeParams p, int attn_grid) {
         // this chunk's (max, sum) pairs, one per lane, and its rows: all loads are independent
         float2 mine = make_float2(-INFINITY, 0.f);
         if (lane < n) mine = __ldcg(reinterpret_cast<const float2*>(ml + (base + lane) * ml_stride));
-        float4 rows[8];
+        float4 rows[kAhead];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < kAhead; ++j) {
             const int r = row0 + j * row_step;
             rows[j] = r < n ? __ldcg(reinterpret_cast<const float4*>(po + (base + r) * o_stride))
                             : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -696,7 +704,7 @@ attention_decode_merge_kernel(const DecodeParams p, int attn_grid) {
         Lsum = Lsum * rescale + warp_sum(mine.y * w_mine);
         M = Mc;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < kAhead; ++j) {
             const int r = row0 + j * row_step;
             if (r < n) {   // n is the same on every lane
                 const float w = __shfl_sync(0xffffffffu, w_mine, r);
@@ -706,7 +714,7 @@ attention_decode_merge_kernel(const DecodeParams p, int attn_grid) {
                 acc.w += rows[j].w * w;
             }
         }
-        for (int j = 8; !SPLIT && j < n; ++j) {
+        for (int j = kAhead; !SPLIT && j < n; ++j) {
             const float w = __shfl_sync(0xffffffffu, w_mine, j);
             const float4 r = __ldcg(reinterpret_cast<const float4*>(po + (base + j) * o_stride));
             acc.x += r.x * w;
@@ -715,7 +723,7 @@ attention_decode_merge_kernel(const DecodeParams p, int attn_grid) {
             acc.w += r.w * w;
         }
     }
-    if (SPLIT) {
+    if (shared) {
         s_acc[warp][lane] = acc;
         __syncthreads();
         if (warp > 0) return;
@@ -960,7 +968,9 @@ int launch_attention_decode(void* out, const void* q, int64_t q_st, int64_t q_sh
     B200_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     B200_CHECK_CUDA(launch_kernel(kernel, dim3(grid), dim3(kThreads), smem, stream,
                                   dim3(1, 1, 1), tmap_k, tmap_v, p));
-    const bool split = batch * q_heads <= 4 * sm_count();   // CTAs that run at once
+    // Few CTAs (those of requests with few partials only end: 28 requests of 100 keys, 448 of them, 9.0 us against 8.4), and
+    // requests that may get more partials than a warp fetches at once.
+    const bool split = batch * q_heads <= 2 * sm_count() && sm_count() * kg > 7 * batch;
     const int merge_ctas = split ? batch * q_heads : batch * ((q_heads + kMergeWarps - 1) / kMergeWarps);
     auto merge = window ? (split ? attention_decode_merge_kernel<true, true> : attention_decode_merge_kernel<true, false>)
                         : (split ? attention_decode_merge_kernel<false, true> : attention_decode_merge_kernel<false, false>);

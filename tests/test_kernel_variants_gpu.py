@@ -38,7 +38,7 @@ def test_decode_of_two_token_tiles(pkg, monkeypatch, kind, nreq):
 
 
 @pytest.mark.parametrize("seq_lens,page_size,hq,hkv", [([700], 16, 16, 8), ([33], 16, 16, 8), ([5000, 2], 16, 16, 8), ([3000], 1, 8, 1),
-                                                       ([900] * 5, 64, 32, 4)])
+                                                       ([900] * 5, 64, 32, 4), ([256, 257], 16, 16, 8), ([257], 16, 16, 8), ([256, 1, 300], 16, 6, 2), ([64] * 14, 16, 14, 2)])
 def test_decode_of_few_requests_with_many_partials(L, seq_lens, page_size, hq, hkv):
     got, want, _ = decode_attention_case(L, seq_lens, page_size, hq, hkv, seed=len(seq_lens))
     assert_close_bf16(got, want, 2e-2, 2e-2, "decode attention")
