@@ -944,13 +944,18 @@ static float skinny_gemm_us(int M, int N, int K, int epilogue) {
     return static_cast<float>(N) * K * 2e-6f / 5.7f + 5.f + (epilogue_is_gated(epilogue) ? 4.2f : 1.9f) * div_ceil(M, kRoundCols);
 }
 
-// Do tiles take this many rows?  (They are stored 16 bytes at a time.)
+// Do tiles take this many rows?  From 65 on where they are a tenth faster (they are stored 16 bytes at a time), from 257 on
+// always; B200_GEMM_TILE_MIN_M sets one line instead.  The estimate is too high for few rows of a small W (us, tiles and slabs:
+// 65 rows of 3072 x 640 9.9 and 8.2, of 2048 x 1024 9.4 and 8.5, 129 of 1024 x 1024 9.4 and 8.7; but 65 of 12288 x 1024 11.8 and
+// 14.9, 129 of 2048 x 1024 9.6 and 10.6).
 static bool linear_on_tiles(const void* y, int M, int N, int K, int epilogue, bool fused) {
-    const int tile_min = env_int("B200_GEMM_TILE_MIN_M", 257);
-    const bool whole_vectors = (epilogue_is_gated(epilogue) ? N / 2 : N) % 8 == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0;
-    const bool tiles_faster = tile_min == 257 && !fused && M > kRoundCols && whole_vectors &&
-                              tile_gemm_us(M, N, K, epilogue) < 0.9f * skinny_gemm_us(M, N, K, epilogue);
-    return M >= tile_min || tiles_faster;
+    const int tile_min = env_int("B200_GEMM_TILE_MIN_M", 0);
+    if (tile_min > 0 || M > 256) return M >= tile_min;
+    const bool gated = epilogue_is_gated(epilogue);
+    if (fused || M <= kRoundCols || (gated ? N / 2 : N) % 8 != 0 || (reinterpret_cast<uintptr_t>(y) & 15) != 0) return false;
+    const bool small = M <= 128 ? static_cast<int64_t>(N) * K < 6000000 : M <= 192 && K > 640 && N < 2048;
+    if (!gated && K <= 1024 && small) return false;
+    return tile_gemm_us(M, N, K, epilogue) < 0.9f * skinny_gemm_us(M, N, K, epilogue);
 }
 
 int gemm_kernel_of(int64_t rows, int N, int K, int epilogue, int groups, int max_rows, bool normed) {

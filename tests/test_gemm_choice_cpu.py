@@ -53,6 +53,18 @@ def test_projections_of_a_handful_of_rows(pkg, N, K, epilogue, narrow, not_narro
         assert lib.b200_gemm_kernel(rows, N, K, epilogue, 0, 0, 0) == STREAM, rows
 
 
+@pytest.mark.parametrize("M,N,K,epilogue,kernel", [
+    (64, 6144, 1024, SWIGLU, STREAM), (65, 6144, 1024, SWIGLU, PAIR), (65, 3072, 640, PLAIN, STREAM), (128, 2048, 1024, PLAIN, STREAM),
+    (65, 12288, 1024, PLAIN, PAIR), (129, 2048, 1024, PLAIN, PAIR), (129, 1024, 1024, PLAIN, STREAM), (256, 1024, 1024, PLAIN, PAIR),
+    (256, 4096, 1024, PLAIN, PAIR), (256, 1024, 2048, PLAIN, STREAM), (257, 1024, 2048, PLAIN, PAIR), (600, 6144, 4096, PLAIN, TILE),
+])
+def test_batches_between_decoding_and_prompts(pkg, monkeypatch, M, N, K, epilogue, kernel):
+    lib = pkg.load_library()
+    assert lib.b200_gemm_kernel(M, N, K, epilogue, 0, 0, 0) == kernel
+    monkeypatch.setenv("B200_GEMM_TILE_MIN_M", "257")   # one line, and nothing below it
+    assert lib.b200_gemm_kernel(M, N, K, epilogue, 0, 0, 0) == (STREAM if M < 257 else kernel)
+
+
 def test_shapes_that_no_kernel_takes(pkg):
     lib = pkg.load_library()
     assert [lib.b200_gemm_kernel(*a) for a in [(0, 64, 64, 0, 0, 0, 0), (4, 64, 96, 0, 0, 0, 0), (4, 64, 64, 99, 0, 0, 0), (4, 64, 64, 0, 2, 0, 0)]] == [0] * 4
