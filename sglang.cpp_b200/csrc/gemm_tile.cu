@@ -456,18 +456,13 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
                     if (it >= early) tma_load_2d_pair(dst + kABytes, &tmap_w, kb * kBK, w_row, bar);
                 }
             }
-            // Neither CTA may end while something is under way to its memory: the last commits' arrivals at the "empty"
-            // barriers (nothing orders them before the accumulator's, which the epilogue waits for); or, where a wait ran
-            // out, the copies themselves, of both CTAs (the first one sees them all, and the second one waits for it below).
-            for (int i = it > STAGES ? it - STAGES : 0; i < it; ++i) {
-                const uint32_t par = static_cast<uint32_t>(i / STAGES) & 1u;
-                if (!failed && !mbar_wait_bounded(smem_u32(&empty_bar[i % STAGES]), par, p.status, 125)) failed = true;
-                if (failed && (rank > 0 || !mbar_wait_bounded(smem_u32(&full_bar[i % STAGES]), par, p.status, 126))) break;
-            }
         }
     } else if (warp == 1) {
         if (rank == 0 && elect_one()) {
             const uint32_t idesc = idesc_bf16(kPairM, TN);
+            // Neither CTA may end while something is under way to its memory.  So stages that are not filled again are not
+            // handed back: nothing would order those arrivals before the accumulator's, which the epilogue waits for.
+            const int fills = first < total_tiles ? ((total_tiles - 1 - first) / step + 1) * p.kb_total : 0;
             int it = 0, tcount = 0;
             bool failed = false;
             for (int t = first; t < total_tiles && !failed; t += step, ++tcount) {
@@ -495,11 +490,14 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
                     for (int k = 0; k < kBK / 16; ++k)
                         tc_mma_bf16_pair(d, kmajor_sw128_desc(a0 + k * 32), kmajor_sw128_desc(b0 + k * 32), idesc,
                                          (kb > 0 || k > 0) ? 1u : 0u);
-                    tc_commit_pair(smem_u32(&empty_bar[s]));
+                    if (it + STAGES < fills) tc_commit_pair(smem_u32(&empty_bar[s]));
                 }
                 if (failed) break;
                 tc_commit_pair(smem_u32(&acc_full_bar[acc]));
             }
+            // Where a wait ran out: the copies of both CTAs that may still be on their way.
+            for (int i = it; failed && i < fills && i < it + STAGES; ++i)
+                if (!mbar_wait_bounded(smem_u32(&full_bar[i % STAGES]), static_cast<uint32_t>(i / STAGES) & 1u, p.status, 125)) break;
         }
     } else {
         pdl_wait_prior();   // (y may still be read)
