@@ -545,7 +545,9 @@ TileKernel pair_kernel_for(int epilogue) {
 // measured on B200 (M 64 to 8192, K 1024 to 14336).  Pairs fetch a third less per product, which is what bounds full waves
 // (8192 x 4096 x 1024: 57 us against 62; 3000 x 28672 x 4096: 479 against 523); blocks of 128 tokens waste less of a short
 // batch (300 x 28672 x 4096: 92 against 96); narrow tiles put more SMs to work where there are few (600 x 1024 x 3072: 18 us
-// with 64 features, 19 with 128, 26 with 256), or leave fewer of them idle in the last wave.
+// with 64 features, 19 with 128, 26 with 256), or leave fewer of them idle in the last wave.  With a short K a pair's longer start
+// counts (8000 x 4096 x 512: 41.9 us against 39.8), and of 128 features a single CTA multiplies and loads half a tile (300 x 128 x
+// 512: 7.5 against 6.8).
 struct TilePick {
     int tn;
     float us;
@@ -560,11 +562,12 @@ TilePick pick_tile(int M, int n_out, bool gated, int kb) {
         return static_cast<float>(div_ceil(div_ceil(M, tm) * div_ceil(n_out * per, tn), slots)) * kb * each + once;
     };
     const bool one_wave = div_ceil(M, kTM) * div_ceil(n_out * per, kTN) <= sms;
-    TilePick best = {0, cost(kTM, kTN, sms, one_wave ? 0.42f : 0.44f, 2.5f)};
+    TilePick best = {0, cost(kTM, kTN, sms, (one_wave ? 0.42f : 0.44f) * (n_out * per <= kTN / 2 ? 0.8f : 1.f), 2.5f)};
+    const float margin = kb < 12 ? 1.05f : 1.f;
     const struct { int tn; float each; } pairs[] = {{256, 0.40f}, {192, 0.32f}, {128, 0.25f}, {64, 0.22f}};
     for (const auto& t : pairs) {
         const float c = cost(kPairM, t.tn, sms / 2, t.each, 4.0f);
-        if (c < best.us) best = {t.tn, c};
+        if (c * margin < best.us) best = {t.tn, c};
     }
     return best;
 }
@@ -599,12 +602,15 @@ int tile_gemm_features(int M, int N, int K, int epilogue) {
     return pick_tile(M, gated ? N / 2 : N, gated, K / kBK).tn;
 }
 
-// Blocks of 128 tokens on one CTA each, or of 256 on a pair: what a group's rows come to in either, where groups differ by a
-// seventh (64 groups of 189 rows, 2048 x 2048 and 1024 x 2048: a layer of 430 us against 456).
+// Blocks of 256 tokens on a pair of CTAs where a group's rows, give or take a seventh, fill one of them and more than one of the
+// 128 of a single CTA (151 to 222 rows on average; 64 groups of 189 rows, 2048 x 2048 and 1024 x 2048: a layer of 430 us against
+// 456).  Beyond, it depends on how blocks fall to waves (16 groups of 256, 300, 400, 560 rows: pairs 1.07, 0.93, 1.07 and 0.985 times
+// as fast), until the blocks are many (640 rows on, 8, 16 and 32 groups: 0.994 to 1.09; but 0.92 and 0.985 for 8 groups of 1100,
+// some of which need a fifth block).
 bool grouped_on_pairs(int64_t total_rows, int num_groups) {
     const float rows = static_cast<float>(total_rows) / num_groups;
-    auto blocks = [&](float per) { return ceilf(rows * 0.85f / per) + ceilf(rows * 1.15f / per); };
-    return 0.80f * blocks(kPairM) < 0.44f * blocks(kTM);
+    if (rows >= 640.f) return rows < 1024.f || rows >= 1152.f;
+    return rows * 0.85f > kTM && rows * 1.15f <= kPairM;
 }
 
 int launch_tile_gemm(void* y, const void* x, const void* w, const void* bias, int M, int N, int K,

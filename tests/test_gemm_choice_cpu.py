@@ -65,6 +65,17 @@ def test_batches_between_decoding_and_prompts(pkg, monkeypatch, M, N, K, epilogu
     assert lib.b200_gemm_kernel(M, N, K, epilogue, 0, 0, 0) == (STREAM if M < 257 else kernel)
 
 
+@pytest.mark.parametrize("M,N,K,kernel", [(300, 128, 512, TILE), (8000, 128, 640, TILE), (8000, 4096, 512, TILE), (8000, 4096, 640, TILE), (3000, 520, 640, TILE),
+                                          (300, 1024, 640, PAIR), (1000, 1024, 768, PAIR), (8192, 4096, 1024, PAIR), (257, 64, 4096, PAIR)])
+def test_tiles_of_a_short_k(pkg, M, N, K, kernel):
+    assert pkg.load_library().b200_gemm_kernel(M, N, K, PLAIN, 0, 0, 0) == kernel
+
+
+@pytest.mark.parametrize("rows,kernel", [(127, STREAM), (130, TILE), (150, TILE), (151, PAIR), (222, PAIR), (223, TILE), (300, TILE), (560, TILE), (630, TILE), (680, PAIR), (1000, PAIR), (1100, TILE), (1200, PAIR)])
+def test_expert_tiles(pkg, rows, kernel):
+    assert pkg.load_library().b200_gemm_kernel(rows * 16, 2048, 2048, SWIGLU, 16, rows * 16, 0) == kernel
+
+
 def test_shapes_that_no_kernel_takes(pkg):
     lib = pkg.load_library()
     assert [lib.b200_gemm_kernel(*a) for a in [(0, 64, 64, 0, 0, 0, 0), (4, 64, 96, 0, 0, 0, 0), (4, 64, 64, 99, 0, 0, 0), (4, 64, 64, 0, 2, 0, 0)]] == [0] * 4
