@@ -1451,10 +1451,12 @@ int launch_chunked(const Recurrence& a, cudaStream_t stream) {
     const int parts = div_ceil(a.heads / a.kv_heads, kPrepareHeads);
     B200_CHECK_CUDA(launch_kernel(prepare, dim3(div_ceil(a.max_extend, kChunk), a.kv_heads * parts, a.batch), dim3(kPrepareThreads),
                                   sizeof(PrepareSmem), stream, dim3(1, 1, 1), a, parts));
-    // the narrowest slices whose CTAs still run at once
+    // The narrowest slices whose CTAs still run at once, for prompts of three chunks and more: every slice loads the chunk's keys
+    // and queries and solves it for itself, which one or two chunks do not make up for (a Saluzen prompt of 60 tokens 791 us with 64
+    // columns, 798 with 16; of 100 tokens 842 and 843, of 200 994 and 982).
     const int units = a.heads * a.batch;
     int slice = kSlice;
-    while (RULE != kMemory && slice > 16 && static_cast<int64_t>(units) * (a.padded_value_dim / slice) * 2 <= sm_count()) slice /= 2;
+    while (RULE != kMemory && a.max_extend > 2 * kChunk && slice > 16 && static_cast<int64_t>(units) * (a.padded_value_dim / slice) * 2 <= sm_count()) slice /= 2;
     if (slice == 64) return launch_walk<RULE, 64>(a, stream);
     if constexpr (RULE != kMemory) return slice == 32 ? launch_walk<RULE, 32>(a, stream) : launch_walk<RULE, 16>(a, stream);
     return B200_OK;

@@ -139,9 +139,10 @@ def test_head_pass_of_many_tokens(L, tokens, hq, hkv, qk_norm):
 @pytest.mark.parametrize("rule", [SSD, DELTA])
 @pytest.mark.parametrize("heads", [4, 12, 20])
 @pytest.mark.parametrize("dv", [64, 128])
-def test_recurrence_in_slices_of_every_width(call, rule, heads, dv):  # noqa: F811
-    """Two requests, one of whole chunks; 4 to 20 heads are dealt in 16, 32 and 64 value columns per CTA."""
-    r = Recurrence(rule, [192, 65], heads, heads // 2, 128, dv, 4, BF16, 1)
+@pytest.mark.parametrize("lens", [[192, 65], [128, 65], [129, 3]])
+def test_recurrence_in_slices_of_every_width(call, rule, heads, dv, lens):  # noqa: F811
+    """Two requests, whole chunks and parts; 4 to 20 heads are dealt in 16, 32 and 64 value columns per CTA, up to two chunks in 64."""
+    r = Recurrence(rule, lens, heads, heads // 2, 128, dv, 4, BF16, 1)
     states = r.states(3)
     got = r.run(call, states, [0, 0], [2, 0])
     outs, last = r.want()
