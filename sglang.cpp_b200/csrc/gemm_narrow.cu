@@ -281,7 +281,11 @@ narrow_gemm_kernel(const NarrowParams p) {
             }
         }
         if (!live) return;
-        const float r0 = v0 * cs - v1 * sn, r1 = v1 * cs + v0 * sn;
+        float r0 = v0, r1 = v1;   // (values as they are: 0 times what is not finite would reach the other half)
+        if (head_kind < 2) {
+            r0 = v0 * cs - v1 * sn;
+            r1 = v1 * cs + v0 * sn;
+        }
         __nv_bfloat16* dst = nullptr;
         if (head_kind == 0)
             dst = p.y + m * p.y_pitch + head * 128;

@@ -1,10 +1,12 @@
 """Kernels that a rule on sizes picks, at the sizes where each can go wrong, against the oracle.
 
 Tolerances are those of the operators' own tests: the variants differ from one another in the order of fp32 sums only."""
+import numpy as np
 import pytest
 import torch
 
 from oracle import token_loop_oracle as O
+from tests import test_engine_gpu as engine_tests
 from tests.parity_cases import assert_close_bf16, decode_attention_case, prefill_attention_case, randn_bf16
 from tests.test_engine_gpu import test_decode_with_norms_folded_into_the_gemms as folded_decode
 from tests.test_moe_gpu import test_moe_forward_matches_oracle as moe_forward
@@ -35,6 +37,27 @@ def test_linear_of_few_rows(L, pkg, M, N, K):
 @pytest.mark.parametrize("kind,nreq", [("qwen3", 12), ("llama", 9), ("qwen2", 16)])
 def test_decode_of_two_token_tiles(pkg, monkeypatch, kind, nreq):
     folded_decode(pkg, monkeypatch, kind, nreq, "1")
+
+
+@pytest.mark.parametrize("nreq", [1, 9])
+def test_values_that_are_not_finite_stay_where_they_are(pkg, nreq):
+    """Values are not rotated: an infinite one must not reach the feature that a rotation would pair it with."""
+    cfg = engine_tests.small_cfg("qwen2")
+    pr = engine_tests.Pair(pkg, cfg, 16, max_running_req=max(nreq, 8))
+    reqs = [pr.hb.add_request(np.arange(1, 6 + i, dtype=np.int32), 4) for i in range(nreq)]
+    pr.hb.prefill(reqs).synchronize()
+    at = (cfg.num_qo_heads + cfg.num_kv_heads + 2) * 128
+    bias = pr.w["layers"][0]["qkv_bias"].clone()
+    bias[at + 3], bias[at + 70] = float("inf"), float("-inf")
+    pr.engine.load("qkv_bias", 0, bias)
+    pr.hb.allocate(reqs)
+    slots = [int(pr.hb.slots_of(r)[r.device_len - 1]) for r in reqs]
+    pr.hb.decode(reqs).synchronize()
+    pool = pr.engine.device_view("kv_cache").view(torch.bfloat16).view(2, cfg.num_layers, -1, cfg.num_kv_heads, 128).cpu()
+    for slot in slots:
+        v = pool[1, 0, slot].float()
+        assert v[2, 3] == float("inf") and v[2, 70] == float("-inf") and int(torch.isfinite(v).logical_not().sum()) == 2
+    pr.engine.close()
 
 
 @pytest.mark.parametrize("seq_lens,page_size,hq,hkv", [([700], 16, 16, 8), ([33], 16, 16, 8), ([5000, 2], 16, 16, 8), ([3000], 1, 8, 1),
