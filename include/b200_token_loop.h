@@ -115,6 +115,9 @@ B200_API int b200_qknorm_rope_store(void* qkv, const void* q_weight, const void*
                                     int kv_heads, int head_dim, int max_pos, int64_t num_slots,
                                     float eps, int write_k_back, b200_stream_t stream);
 
+/* Does that pass give each warp a token (1) or the next rows of any token (0)?  With aligned tables; nothing is launched. */
+B200_API int b200_head_pass_by_tokens(int tokens, int q_heads, int kv_heads, int head_dim, int norms);
+
 /* ---- activation (include/sglang/layers/activation.h:8-11) ----------------- */
 
 /* silu_and_mul / gelu_and_mul (src/layers/activation.cu:15-75):

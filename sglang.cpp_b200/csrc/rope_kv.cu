@@ -226,7 +226,7 @@ qknorm_rope_store_kernel(__nv_bfloat16* qkv, const __nv_bfloat16* __restrict__ q
     }
 }
 
-// The same for many tokens with heads of 128: a warp per token, four rows (heads) at a time and sixteen in flight.  A token's
+// The same for many tokens with heads of 128 (head_pass_by_tokens): a warp per token, four rows (heads) at a time and sixteen in flight.  A token's
 // rotation is read once, and no row number has to be divided (8192 tokens of 32 rows, 134 MB: 26.8 us against 43.8 with rows
 // dealt to warps one after the other).
 constexpr int kTokenWarps = 4;
@@ -327,6 +327,14 @@ qknorm_rope_store_tokens_kernel(__nv_bfloat16* qkv, const __nv_bfloat16* __restr
 
 }  // namespace
 
+// A warp per token takes its rows 16 at a time, one turn after the other, so that few tokens of many heads leave it behind rows
+// dealt to warps (us, with head norms: 228 tokens of 128 / 8 heads 16.1 and 7.3, 274 of 40 / 40 12.1 and 7.4, 592 of 64 / 8 9.8 and
+// 8.3, 740 of 32 / 8 7.5 and 7.3, of 128 / 8 19.6 and 18.2; 900 of 32 / 8 7.5 and 8.2, of 128 / 8 19.5 and 20.5, of 64 / 8 11.5 and
+// 12.9; without: 274 of 40 / 40 7.8 and 5.7, 450 of 64 / 8 5.8 and 5.6; 500 5.9 and 6.1, of 128 / 8 9.2 and 9.9).
+bool head_pass_by_tokens(int tokens, int q_heads, int kv_heads, int head_dim, bool norms) {
+    return static_cast<int64_t>(tokens) * (q_heads + 2 * kv_heads) >= 32768 && head_dim == 128 && tokens >= (norms ? 900 : 500);
+}
+
 int launch_qknorm_rope_store(void* qkv, const void* q_weight, const void* k_weight,
                              const float* cos_table, const float* sin_table,
                              const int32_t* positions, const int32_t* out_loc, void* k_cache,
@@ -336,7 +344,7 @@ int launch_qknorm_rope_store(void* qkv, const void* q_weight, const void* k_weig
     const int64_t rows = static_cast<int64_t>(tokens) * (q_heads + 2 * kv_heads);
     if (rows == 0) return B200_OK;
     const bool aligned = ((reinterpret_cast<uintptr_t>(cos_table) | reinterpret_cast<uintptr_t>(sin_table)) & 15) == 0;
-    if (rows >= 32768 && head_dim == 128 && aligned) {
+    if (aligned && head_pass_by_tokens(tokens, q_heads, kv_heads, head_dim, q_weight != nullptr)) {
         B200_CHECK_CUDA(launch_kernel(qknorm_rope_store_tokens_kernel, dim3(div_ceil(tokens, kTokenWarps)), dim3(kTokenWarps * 32), 0,
                                       stream, dim3(1, 1, 1), static_cast<__nv_bfloat16*>(qkv),
                                       static_cast<const __nv_bfloat16*>(q_weight), static_cast<const __nv_bfloat16*>(k_weight),
@@ -424,6 +432,10 @@ int b200_store_kv(void* k_cache, void* v_cache, const void* k, const void* v,
         static_cast<int>(elems / 8), k_stride_token, v_stride_token, num_slots, status);
     B200_CHECK_LAUNCH();
     return B200_OK;
+}
+
+int b200_head_pass_by_tokens(int tokens, int q_heads, int kv_heads, int head_dim, int norms) {
+    return b200::head_pass_by_tokens(tokens, q_heads, kv_heads, head_dim, norms != 0) ? 1 : 0;
 }
 
 int b200_qknorm_rope_store(void* qkv, const void* q_weight, const void* k_weight,

@@ -79,3 +79,14 @@ def test_expert_tiles(pkg, rows, kernel):
 def test_shapes_that_no_kernel_takes(pkg):
     lib = pkg.load_library()
     assert [lib.b200_gemm_kernel(*a) for a in [(0, 64, 64, 0, 0, 0, 0), (4, 64, 96, 0, 0, 0, 0), (4, 64, 64, 99, 0, 0, 0), (4, 64, 64, 0, 2, 0, 0)]] == [0] * 4
+
+
+@pytest.mark.parametrize("q_heads,kv_heads,norms,by_tokens,by_rows", [
+    (128, 8, 1, (900, 3000), (228, 342, 650, 740)), (40, 40, 1, (900,), (274, 411)), (64, 8, 1, (900, 1100), (410, 592)), (32, 8, 1, (900, 1024), (683, 740)),
+    (16, 8, 1, (1024, 8192), (1023,)), (64, 8, 0, (500, 1500), (410, 450)), (40, 40, 0, (500,), (274,)), (128, 8, 0, (500,), (228, 342)), (32, 8, 0, (683,), (682,)),
+])
+def test_head_pass_of_few_tokens_with_many_heads(pkg, q_heads, kv_heads, norms, by_tokens, by_rows):
+    """A warp per token only where that was the faster way to deal the rows."""
+    lib = pkg.load_library()
+    assert [lib.b200_head_pass_by_tokens(t, q_heads, kv_heads, 128, norms) for t in by_tokens + by_rows] == [1] * len(by_tokens) + [0] * len(by_rows)
+    assert lib.b200_head_pass_by_tokens(8192, q_heads, kv_heads, 64, norms) == 0

@@ -133,7 +133,8 @@ def test_norms_of_many_rows(L, rows, hidden):
     assert_close_bf16(norm.forward(x.cuda()), O.rmsnorm(x, norm.weight.cpu(), 1e-6), 1e-6, RTOL, "norm")
 
 
-@pytest.mark.parametrize("tokens,hq,hkv,qk_norm", [(4700, 5, 1, True), (1025, 16, 8, False), (2341, 6, 4, True)])
+@pytest.mark.parametrize("tokens,hq,hkv,qk_norm", [(4700, 5, 1, True), (1025, 16, 8, False), (2341, 6, 4, True), (900, 64, 8, True),
+                                                     (500, 40, 40, False)])
 def test_head_pass_of_many_tokens(L, tokens, hq, hkv, qk_norm):
     """Rows per token that are not a multiple of the four a warp takes at a time, keys beginning inside such a group: the same
     bits as in pieces that are few enough rows for the other kernel (which has its own test against the oracle)."""
@@ -146,7 +147,7 @@ def test_head_pass_of_many_tokens(L, tokens, hq, hkv, qk_norm):
         qn, kn = L.RMSNorm(128, 1e-6), L.RMSNorm(128, 1e-6)
         qn.weight, kn.weight = randn_bf16(gen, 128).cuda(), randn_bf16(gen, 128).cuda()
     results = []
-    for piece in (tokens, 500):
+    for piece in (tokens, 499 if tokens * (hq + 2 * hkv) < 65536 else 300):
         cache = L.MHAKVCache(hkv, 1, 128, tokens // 16 + 2, 16)
         loc = torch.randperm(cache.total_slots, generator=torch.Generator().manual_seed(3))[:tokens].to(torch.int32).cuda()
         x = qkv.cuda()
