@@ -15,7 +15,7 @@
 // rare occasions the row's O is rescaled in TMEM by the threads that own the row.  Nothing else touches
 // O until the end, so the softmax threads carry no accumulator and no P tile goes through shared memory.
 //
-// Roles: warp 0 producer (K/V tiles through a 2-stage TMA ring, as in attention_prefill_tc.cu), warp 1
+// Roles: warp 0 producer (K and V tiles in turn through one TMA ring of five slots), warp 1
 // one thread issues every MMA, warps 4-7 softmax of tile 0, warps 8-11 softmax of tile 1 (thread = TMEM lane).
 // A row's scores fit its thread's registers: S is read once and the row's maximum needs no exchange.  (Two threads per row,
 // 16 warps and two stages of K and V, before: 4 x 2048 tokens behind 2048 cached, 16 / 8 heads, 327 us against 321 with

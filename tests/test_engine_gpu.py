@@ -187,7 +187,8 @@ def test_decode_with_norms_folded_into_the_gemms(pkg, monkeypatch, kind, nreq, f
     """Decode steps of dense, unsharded models have no add + norm kernels: o_proj and down_proj add the
     residual and accumulate each row's sum of squares in their split-K epilogue, qkv_proj and
     gate_up_proj multiply un-normalised rows by weights with the norm weight folded in and scale by
-    1 / rms afterwards.  The same requests with that (the default) and without (B200_FOLD_NORM=0, read
+    1 / rms afterwards; a handful of requests of a narrow model runs on the narrow kernel instead, which adds the residual
+    and computes the norms itself (test_kernel_variants_gpu.py has the split-K form at so few).  The same requests with that (the default) and without (B200_FOLD_NORM=0, read
     when the engine is created): each against the oracle at the usual bars, and against one another
     (the folded form rounds the normalised activation at a different point: about one bf16 step of a logit).
     fold_heads: the qkv projection's epilogue also applies the QK-norm and the rotation to whole heads and

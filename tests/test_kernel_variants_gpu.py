@@ -16,13 +16,16 @@ from tests.test_saluzen_ops_gpu import BF16
 
 pytestmark = pytest.mark.gpu
 RTOL = 2 ** -7
+NARROW, STREAM, TILE, PAIR = 1, 2, 3, 4   # what b200_gemm_kernel calls the kernels
 BIG = (2e-3, 1e-3)   # absolute: sqrt(K / 1024) of the first, plus the second (as in test_linear_gpu.py)
 
 
 @pytest.mark.parametrize("M", [1, 7, 8, 9, 16])
-@pytest.mark.parametrize("N,K", [(8, 64), (24, 64), (1000, 192), (520, 2048), (1024, 3072), (4096, 1024), (128, 5632)])
+@pytest.mark.parametrize("N,K", [(8, 64), (24, 64), (1000, 192), (520, 2048), (1024, 3072), (4096, 1024), (128, 5632), (3072, 2048), (2400, 1088)])
 def test_linear_of_few_rows(L, pkg, M, N, K):
-    """One and two tiles of tokens, features behind the last whole tile of 16, K within a register buffer and beyond two."""
+    """One and two tiles of tokens, features behind the last whole tile of 16, K within a register buffer and beyond two; two
+    buffers with as many CTAs as SMs and with more."""
+    assert pkg.load_library().b200_gemm_kernel(M, N, K, pkg.EPILOGUE_NONE, 0, 0, 0) == NARROW
     gen = torch.Generator().manual_seed(M + N + K)
     buf, w, b = randn_bf16(gen, M, K + 64), randn_bf16(gen, N, K, std=0.05), randn_bf16(gen, N)
     atol = BIG[0] * (K / 1024) ** 0.5 + BIG[1]
@@ -37,6 +40,36 @@ def test_linear_of_few_rows(L, pkg, M, N, K):
 @pytest.mark.parametrize("kind,nreq", [("qwen3", 12), ("llama", 9), ("qwen2", 16)])
 def test_decode_of_two_token_tiles(pkg, monkeypatch, kind, nreq):
     folded_decode(pkg, monkeypatch, kind, nreq, "1")
+
+
+def on_narrow(pkg, cfg, nreq):
+    """Whether a decode step's projections that carry the norm run on the narrow kernel."""
+    qkv = (cfg.num_qo_heads + 2 * cfg.num_kv_heads) * cfg.head_dim
+    return pkg.load_library().b200_gemm_kernel(nreq, qkv, cfg.hidden_size, pkg.EPILOGUE_NONE, 0, 0, 1) == NARROW
+
+
+@pytest.mark.parametrize("fold_heads", ["1", "0"])
+@pytest.mark.parametrize("kind,nreq", [("qwen3", 20), ("llama", 24), ("qwen2", 17), ("llama", 33)])
+def test_decode_on_split_projections_with_folded_norms(pkg, monkeypatch, kind, nreq, fold_heads):
+    """More requests than the narrow kernel takes: the split-K kernel's accumulator of 32 tokens and the one of 64."""
+    assert not on_narrow(pkg, engine_tests.small_cfg(kind), nreq)
+    folded_decode(pkg, monkeypatch, kind, nreq, fold_heads)
+
+
+@pytest.mark.parametrize("fold_heads", ["1", "0"])
+@pytest.mark.parametrize("hidden,nreq,narrow", [(2304, 1, False), (2304, 5, False), (2304, 16, False), (2048, 1, True), (1984, 2, True), (2048, 9, False)])
+@pytest.mark.parametrize("qwen", [True, False])
+def test_decode_of_a_wide_layer(pkg, monkeypatch, qwen, hidden, nreq, narrow, fold_heads):
+    """A handful of requests of a model too wide for the narrow kernel's norm (split-K, accumulator of 32 tokens), and of the
+    widest that it takes (two register buffers).  The bars are for logits below 2, where a bf16 step is at most 2^-7: weights are
+    scaled by 1 / sqrt(hidden), and the output head is its own (against the table of the embedding, one layer further on, a
+    token's own logit is about 5, and one step 2^-5)."""
+    cfg = O.ModelConfig(1, hidden, 4, 2, 128, 512, 1024, 1e-6, 1e6, 512, False, qwen, qwen)
+    assert on_narrow(pkg, cfg, nreq) == narrow
+    init = O.init_weights
+    monkeypatch.setattr(engine_tests, "small_cfg", lambda kind: cfg)
+    monkeypatch.setattr(engine_tests.O, "init_weights", lambda c, seed, std: init(c, seed=seed, std=std * (256 / hidden) ** 0.5))
+    folded_decode(pkg, monkeypatch, "wide", nreq, fold_heads)
 
 
 @pytest.mark.parametrize("nreq", [1, 9])
@@ -57,6 +90,32 @@ def test_values_that_are_not_finite_stay_where_they_are(pkg, nreq):
     for slot in slots:
         v = pool[1, 0, slot].float()
         assert v[2, 3] == float("inf") and v[2, 70] == float("-inf") and int(torch.isfinite(v).logical_not().sum()) == 2
+    pr.engine.close()
+
+
+@pytest.mark.parametrize("nreq", [1, 8, 9, 16])
+def test_experts_layer_of_two_register_buffers(pkg, nreq):
+    """Decode steps of a Qwen3-MoE layer of hidden 2048: qkv with its head operations on the narrow kernel, without a norm.
+    Every token takes all experts (of two almost equal ones either could be chosen otherwise); weights as above."""
+    cfg = O.ModelConfig(1, 2048, 4, 2, 128, 512, 1024, 1e-6, 1e6, 512, False, True, True, "silu", 8, 8, 128, True)
+    rng = np.random.default_rng(nreq)
+    with pytest.MonkeyPatch.context() as mp:
+        init = O.init_weights
+        mp.setattr(engine_tests.O, "init_weights", lambda c, seed, std: init(c, seed=seed, std=std * (256 / 2048) ** 0.5))
+        pr = engine_tests.Pair(pkg, cfg, 16, num_pages=nreq * 4 + 8, max_running_req=max(nreq, 8))
+    reqs = [pr.hb.add_request(rng.integers(0, cfg.vocab_size, size=int(n)).astype(np.int32), 6) for n in rng.integers(3, 40, size=nreq)]
+    pr.host_tokens = {r.table_idx: list(r.input_ids[:r.device_len]) + [0] * 16 for r in reqs}
+    for step in range(3):
+        pr.hb.allocate(reqs)
+        ob, pt = pr.oracle_batch(reqs, step == 0)
+        want = pr.oracle.forward(ob, pr.kv, pt)
+        (pr.hb.decode if step else pr.hb.prefill)(reqs).synchronize()
+        engine_tests.check_logits(pr.engine.logits(nreq), want, f"step {step}")
+        tok = want.argmax(-1).tolist()
+        for r, t in zip(reqs, tok):
+            pr.host_tokens[r.table_idx][r.cached_len] = t
+        pr.engine.write_token_pool([r.table_idx for r in reqs], [r.cached_len for r in reqs], tok)
+    assert pr.engine_status_clean()
     pr.engine.close()
 
 
@@ -100,20 +159,59 @@ def test_pairs_of_ctas_one_after_another(L, monkeypatch, tile, K):
     assert L.read_device_status() == (0, 0)
 
 
-@pytest.mark.parametrize("M,N,K,gated", [(65, 6144, 1024, True), (100, 4096, 1024, False), (181, 6144, 1024, True), (256, 1024, 2048, False)])
+@pytest.mark.parametrize("M,N,K,gated", [(65, 6144, 1024, True), (100, 12288, 1024, False), (181, 6144, 1024, True), (256, 4096, 1024, False)])
 def test_batches_that_either_kernel_takes(L, pkg, monkeypatch, M, N, K, gated):
+    """On tiles by the rule, and on slabs when the environment says so: each against the oracle, and against one another."""
+    lib = pkg.load_library()
     gen = torch.Generator().manual_seed(M)
-    x, w = randn_bf16(gen, M, K).cuda(), randn_bf16(gen, N, K, std=0.05).cuda()
+    x, w = randn_bf16(gen, M, K), randn_bf16(gen, N, K, std=0.05)
+    xs, ws = x.cuda(), w.cuda()
     epilogue = pkg.EPILOGUE_SWIGLU if gated else pkg.EPILOGUE_NONE
-    y = L.linear(x, w, epilogue=epilogue)
+    want = O.silu_and_mul(O.linear(x, w)) if gated else O.linear(x, w)
+    atol, rtol = (2 * sum(BIG), 3 * RTOL) if gated else (sum(BIG), RTOL)   # (K is 1024)
+    assert lib.b200_gemm_kernel(M, N, K, epilogue, 0, 0, 0) in (TILE, PAIR)
+    y = L.linear(xs, ws, epilogue=epilogue)
+    assert_close_bf16(y, want, atol, rtol, "tiles")
     monkeypatch.setenv("B200_GEMM_TILE_MIN_M", "1000000")
-    assert_close_bf16(y, L.linear(x, w, epilogue=epilogue), 4e-3, 3 * RTOL, "tiles against slabs")
+    assert lib.b200_gemm_kernel(M, N, K, epilogue, 0, 0, 0) == STREAM
+    slabs = L.linear(xs, ws, epilogue=epilogue)
+    assert_close_bf16(slabs, want, atol, rtol, "slabs")
+    assert_close_bf16(y, slabs, 4e-3, 3 * RTOL, "tiles against slabs")
 
 
-@pytest.mark.parametrize("T,E,k", [(380, 4, 2), (450, 3, 1), (1030, 8, 1)])
-def test_experts_of_one_pair_tile(L, T, E, k):
-    """Between 128 and 256 rows per expert on average: pairs of CTAs."""
-    moe_forward(L, T, E, k, 128, 192, True, "silu")
+def expert_kernel(pkg, T, E, k, H, I):
+    return pkg.load_library().b200_gemm_kernel(T * k, 2 * I, H, pkg.EPILOGUE_SWIGLU, E, T, 0)
+
+
+@pytest.mark.parametrize("T,E,k,H,I,kernel", [(380, 4, 2, 128, 192, PAIR), (570, 3, 1, 1088, 1024, PAIR), (1520, 32, 4, 1024, 1024, PAIR),
+                                              (2048, 6, 2, 640, 384, PAIR), (450, 3, 1, 128, 192, TILE), (1030, 8, 1, 128, 192, TILE)])
+def test_experts_of_one_pair_tile(L, pkg, T, E, k, H, I, kernel):
+    """151 to 222 rows per expert on average, or 640 and more, run on pairs of CTAs: K of two blocks and of more than the ring's
+    six stages, tiles for two turns of every pair and more, one and several blocks of tokens per expert; other averages on
+    single CTAs."""
+    assert expert_kernel(pkg, T, E, k, H, I) == kernel
+    moe_forward(L, T, E, k, H, I, True, "silu")
+
+
+def test_experts_on_pair_tiles_that_tokens_do_not_choose_alike(L, pkg):
+    """Experts with no row, a few, less than a block of 256, and several blocks, beside one another."""
+    T, E, k, H, I = 1500, 24, 3, 576, 320
+    assert expert_kernel(pkg, T, E, k, H, I) == PAIR
+    gen = torch.Generator().manual_seed(24)
+    liking = torch.linspace(-3, 3, E)[torch.randperm(E, generator=gen)]
+    liking[::5] = -1e9
+    gumbel = -torch.log(-torch.log(torch.rand(T, E, generator=gen).clamp(1e-6, 1 - 1e-6)))
+    rank = (liking + gumbel).argsort(-1).argsort(-1)
+    logits = ((rank.float() - E / 2) / 4).to(torch.bfloat16)      # (distinct in a row: no ties)
+    rows = torch.bincount(rank.topk(k, -1).indices.flatten(), minlength=E)
+    assert (rows == 0).any() and (rows > 512).any() and ((rows > 0) & (rows < 128)).any() and ((rows > 128) & (rows < 256)).any()
+    hidden, gu, dn = randn_bf16(gen, T, H), randn_bf16(gen, E, 2 * I, H, std=H ** -0.5), randn_bf16(gen, E, H, I, std=I ** -0.5)
+    moe = L.MoELayer(E, k, H, I, True, "silu")
+    moe.gate_up_proj.copy_(gu.cuda())
+    moe.down_proj.copy_(dn.cuda())
+    want = O.moe_forward(hidden, logits, gu, dn, k, True, "silu", O.store_bf16)
+    assert_close_bf16(moe.forward(hidden.cuda(), logits.cuda()), want, 2e-2, 4 * 2 ** -7, "skewed")
+    assert L.read_device_status() == (0, 0)
 
 
 @pytest.mark.parametrize("T,E,k,H,I,act", [(32, 16, 4, 2048, 1024, "silu"), (1, 64, 4, 1088, 64, "silu"), (9, 3, 1, 64, 192, "gelu"),
