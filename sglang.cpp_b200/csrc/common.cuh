@@ -229,6 +229,13 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, uint32_t parity,
     return true;
 }
 
+// The same where the barrier is mostly ready: the first test stands before the loop.  (Where one elected lane waits, a ready
+// barrier takes 47 cycles this way and 170 as the first round of the loop.)
+__device__ __forceinline__ bool mbar_wait_mostly_ready(uint32_t bar, uint32_t parity, int* status, int site) {
+    if (mbar_try_wait(bar, parity)) return true;
+    return mbar_wait_bounded(bar, parity, status, site);
+}
+
 // ---- TMA (tiled tensor copies, never multicast) -----------------------------
 
 __device__ __forceinline__ void tma_prefetch_desc(const void* tmap) {
@@ -255,7 +262,16 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const void* tmap, int 
         : "memory");
 }
 
-// The same copy with an L2 eviction policy (from l2_policy_evict_first) for data read once.
+__device__ __forceinline__ void tma_load_5d(uint32_t dst, const void* tmap, int c0, int c1, int c2, int c3, int c4,
+                                            uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%2, %3, %4, %5, %6}], [%7];" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(tmap)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(bar)
+        : "memory");
+}
+
+// The 3-D copy with an L2 eviction policy (from l2_policy_evict_first) for data read once.
 __device__ __forceinline__ void tma_load_3d_hint(uint32_t dst, const void* tmap, int c0, int c1, int c2,
                                                  uint32_t bar, uint64_t policy) {
     asm volatile(

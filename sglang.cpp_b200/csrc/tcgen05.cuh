@@ -174,6 +174,18 @@ __device__ __forceinline__ uint64_t mnmajor_sw128_desc(uint32_t smem_addr) {
     d |= static_cast<uint64_t>(2) << 61;
     return d;
 }
+// A tile of keys in groups of 8, each both 64-element halves of the head dimension (8 rows of 128 bytes under the 128-byte
+// swizzle): groups 2048 bytes apart.  `half` = 0 for K (rows along the product's inner dimension; the second half is
+// addressed by itself), 1024 for V as an MN-major operand.
+__device__ __forceinline__ uint64_t grouped_keys_desc(uint32_t smem_addr, uint32_t half) {
+    uint64_t d = 0;
+    d |= static_cast<uint64_t>((smem_addr >> 4) & 0x3FFFu);
+    d |= static_cast<uint64_t>(half != 0 ? half >> 4 : 1) << 16;
+    d |= static_cast<uint64_t>(2048 >> 4) << 32;
+    d |= static_cast<uint64_t>(1) << 46;
+    d |= static_cast<uint64_t>(2) << 61;
+    return d;
+}
 __device__ __forceinline__ uint32_t idesc_bf16_128xn(int n, bool b_mn_major) {
     return (1u << 4) | (1u << 7) | (1u << 10) | (b_mn_major ? (1u << 16) : 0u) |
            (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(128 >> 4) << 24);

@@ -113,3 +113,35 @@ def test_prefill_equals_decode_on_last_row(L):
     assert_close_bf16(got_p, want, ATOL, RTOL, "last prefill row")
     # the two kernels round the probabilities at different points: a few bf16 steps apart at most
     assert_close_bf16(got_p, got_d, 8e-3, 2e-2, "last prefill row against the decode step")
+
+
+@pytest.mark.parametrize("page_size", [1, 2, 4, 8, 16, 64, 128, 256])
+@pytest.mark.parametrize("offset,seq_lens,extend_lens", [
+    (0, [129, 640, 17, 383], [129, 500, 17, 65]),   # several blocks per request, ragged, behind prefixes
+    (8, [300, 641], [300, 641]),                    # pages that start in the middle of a page's range, at a group of 8 slots
+    (3, [300, 641], [300, 641]),                    # ... inside such a group: copied half row by half row
+])
+def test_prefill_copies_pages_of_any_size_and_place(L, page_size, offset, seq_lens, extend_lens):
+    """The copies of K and V tiles: whole rows of a page, of a tile of neighbouring pages, and half rows of up to 8 keys."""
+    import math
+
+    from tests.parity_cases import PagedSetup, randn_bf16
+    from oracle import token_loop_oracle as O
+
+    hq, hkv, d = 16, 8, 128
+    ps = PagedSetup(seq_lens, page_size, hkv, d, seed=offset + page_size)
+    pad = -(-offset // page_size) * page_size
+    kc, vc = (torch.cat([t.new_full((offset, hkv, d), float("nan")), t, t.new_full((pad - offset, hkv, d), float("nan"))])
+              for t in (ps.k_cache, ps.v_cache))
+    table = ps.page_table + offset
+    cache = L.MHAKVCache(hkv, 1, d, len(kc) // page_size, page_size, device="cuda")
+    cache.kv_buffer_[0, 0].copy_(kc.cuda())
+    cache.kv_buffer_[1, 0].copy_(vc.cuda())
+    qo = np.concatenate([[0], np.cumsum(extend_lens)]).astype(np.int32)
+    q = randn_bf16(torch.Generator().manual_seed(3), int(qo[-1]), hq, d)
+    attn = L.PagedAttention(cache, hq, hkv, d, max_batch=len(seq_lens))
+    got = attn.prefill(q.cuda(), 0, *(torch.from_numpy(a).cuda() for a in (table, ps.table_idx, ps.seq_lens, qo)), max(extend_lens))
+    torch.cuda.synchronize()
+    want = O.paged_attention(q, kc, vc, table, ps.table_idx, ps.seq_lens, qo, 1.0 / math.sqrt(d), O.store_fp32)
+    assert_close_bf16(got, want.reshape(len(q), hq * d), ATOL, RTOL, "prefill attention")
+    assert L.read_device_status() == (0, 0)
