@@ -1,9 +1,9 @@
 // Mixture-of-experts layer: router top-k, token permute, grouped expert GEMMs, weighted combine.
 //
 // Stands where MoELayer::forward does (src/moe/moe.cc:36-96).  The reference walks
-// top_k x num_experts host-synchronised iterations; here one step is six launches with no host
-// involvement: route (softmax + top-k per token, expert histogram) -> scan -> scatter (rows
-// grouped by expert) -> grouped gate_up GEMM with the gated activation in its epilogue ->
+// top_k x num_experts host-synchronised iterations; here one step is five or six launches with no host
+// involvement: route (softmax + top-k per token) and place (histogram, first rows, a row per choice; one kernel for few
+// tokens) -> scatter (rows grouped by expert) -> grouped gate_up GEMM with the gated activation in its epilogue ->
 // grouped down GEMM -> combine in the reference's accumulation order (k ascending, bf16 after
 // every multiply and add, as index_add_ on bf16 tensors does).
 #include "common.cuh"
@@ -14,17 +14,11 @@ namespace {
 
 constexpr int kMaxExpertsPerLane = 8;  // num_experts <= 256
 constexpr int kMaxTopK = 16;
+constexpr int kRouteInOneCta = 64;     // tokens whose choices and rows one CTA finds (two per warp)
 
-// One warp per token.
-__global__ void __launch_bounds__(128)
-moe_route_kernel(const __nv_bfloat16* __restrict__ logits, int tokens, int E, int top_k, int renorm,
-                 int32_t* __restrict__ ids, float* __restrict__ weights, int32_t* __restrict__ counts) {
-    pdl_launch_dependents();
-    pdl_wait_prior();
-    const int lane = threadIdx.x & 31;
-    const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (t >= tokens) return;
-    const __nv_bfloat16* row = logits + static_cast<int64_t>(t) * E;
+// Softmax and top-k of one token's router logits by a warp; `put(k, expert, weight)` runs on lane 0.
+template <typename Put>
+__device__ __forceinline__ void route_token(const __nv_bfloat16* __restrict__ row, int E, int top_k, int renorm, int lane, Put put) {
     float v[kMaxExpertsPerLane];
     float mx = -INFINITY;
 #pragma unroll
@@ -64,6 +58,7 @@ moe_route_kernel(const __nv_bfloat16* __restrict__ logits, int tokens, int E, in
                 bi = oi;
             }
         }
+        if (bi >= E) bi = k;   // NaN logits: a token's experts are valid and differ all the same
         if ((bi & 31) == lane) v[bi >> 5] = -1.f;
         wsel[k] = best * inv;
         isel[k] = bi;
@@ -73,61 +68,118 @@ moe_route_kernel(const __nv_bfloat16* __restrict__ logits, int tokens, int E, in
         for (int k = 0; k < top_k; ++k) {
             float w = wsel[k];
             if (renorm) w = w / (wsum + 1e-8f);
-            ids[t * top_k + k] = isel[k];
-            weights[t * top_k + k] = round_bf16(w);  // the reference casts the weights to bf16
-            atomicAdd(&counts[isel[k]], 1);
+            put(k, isel[k], round_bf16(w));  // the reference casts the weights to bf16
         }
     }
 }
 
-// Row ranges of the experts [e_begin, e_begin + e_count) this call computes (all of them unless
-// the experts are partitioned over ranks); every other expert gets offset -1 = "not here".
-__global__ void __launch_bounds__(256)
-moe_scan_kernel(const int32_t* __restrict__ counts, int32_t* __restrict__ offsets,
-                int32_t* __restrict__ cursor, int E, int e_begin, int e_count) {
-    pdl_launch_dependents();
-    pdl_wait_prior();
-    __shared__ int s[256];
-    const int e = threadIdx.x;
-    const bool local = e >= e_begin && e < e_begin + e_count;
-    s[e] = (e < E && local) ? counts[e] : 0;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int run = 0;
-        for (int i = 0; i < E; ++i) {
-            const int c = s[i];
-            s[i] = run;
-            run += c;
-        }
-        offsets[E] = run;
-    }
-    __syncthreads();
-    if (e < E) {
-        offsets[e] = local ? s[e] : -1;
-        cursor[e] = 0;
-    }
-}
-
-// One CTA per (token, k) pair: claim a row in the expert's range and copy the token there.
+// One warp per token.  COUNT: the expert histogram too (`counts` zero before).
+template <bool COUNT>
 __global__ void __launch_bounds__(128)
-moe_scatter_kernel(const uint4* __restrict__ hidden, uint4* __restrict__ xp,
-                   const int32_t* __restrict__ ids, const int32_t* __restrict__ offsets,
-                   int32_t* __restrict__ cursor, int32_t* __restrict__ pos, int top_k, int vec_per_row) {
+moe_route_kernel(const __nv_bfloat16* __restrict__ logits, int tokens, int E, int top_k, int renorm,
+                 int32_t* __restrict__ ids, float* __restrict__ weights, int32_t* __restrict__ counts) {
     pdl_launch_dependents();
     pdl_wait_prior();
-    __shared__ int s_row;
-    const int pair = blockIdx.x;
-    if (threadIdx.x == 0) {
-        const int e = ids[pair];
-        const int base = offsets[e];
-        s_row = base < 0 ? -1 : base + atomicAdd(&cursor[e], 1);
-        pos[pair] = s_row;
+    const int lane = threadIdx.x & 31;
+    const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (t >= tokens) return;
+    route_token(logits + static_cast<int64_t>(t) * E, E, top_k, renorm, lane, [&](int k, int e, float w) {
+        ids[t * top_k + k] = e;
+        weights[t * top_k + k] = w;
+        if (COUNT) atomicAdd(&counts[e], 1);
+    });
+}
+
+// Rows of the experts, by one CTA: histogram of the choices in shared memory, the first row of every expert
+// [e_begin, e_begin + e_count) that this call computes (all of them unless the experts are partitioned over ranks; every other
+// one gets offset -1 = "not here"), and a row for every choice (-1: another rank's).  ROUTE: the choices themselves too, a
+// warp per token.
+struct PlaceArgs {
+    const __nv_bfloat16* logits;   // ROUTE
+    float* weights;                // ROUTE
+    int32_t* ids;                  // written by ROUTE
+    int32_t *counts, *offsets, *rows;
+    int tokens, experts, top, renorm, e_begin, e_count;
+};
+template <bool ROUTE>
+__global__ void __launch_bounds__(1024)
+moe_place_kernel(const PlaceArgs a) {
+    __shared__ int s_count[256], s_first[256];
+    pdl_launch_dependents();
+    pdl_wait_prior();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int pairs = a.tokens * a.top;
+    if (threadIdx.x < 256) s_count[threadIdx.x] = 0;
+    __syncthreads();
+    auto local = [&](int e) { return e >= a.e_begin && e < a.e_begin + a.e_count; };
+    // a choice's place among its expert's, in `rows` until the first rows are known (each written and read by one thread)
+    if (ROUTE) {
+        for (int t = warp; t < a.tokens; t += blockDim.x >> 5)
+            route_token(a.logits + static_cast<int64_t>(t) * a.experts, a.experts, a.top, a.renorm, lane, [&](int k, int e, float w) {
+                a.ids[t * a.top + k] = e;
+                a.weights[t * a.top + k] = w;
+                a.rows[t * a.top + k] = atomicAdd(&s_count[e], 1);
+            });
+    } else {
+        for (int i = threadIdx.x; i < pairs; i += blockDim.x) a.rows[i] = atomicAdd(&s_count[a.ids[i]], 1);
     }
     __syncthreads();
-    if (s_row < 0) return;  // another rank's expert
-    const uint4* src = hidden + static_cast<int64_t>(pair / top_k) * vec_per_row;
-    uint4* dst = xp + static_cast<int64_t>(s_row) * vec_per_row;
-    for (int v = threadIdx.x; v < vec_per_row; v += blockDim.x) dst[v] = src[v];
+    if (warp == 0) {   // eight neighbouring experts per lane
+        int c[8], sum = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            c[i] = local(lane * 8 + i) ? s_count[lane * 8 + i] : 0;
+            sum += c[i];
+        }
+        int incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int up = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += up;
+        }
+        int run = incl - sum;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            s_first[lane * 8 + i] = local(lane * 8 + i) ? run : -1;
+            run += c[i];
+        }
+        if (lane == 31) a.offsets[a.experts] = incl;
+    }
+    __syncthreads();
+    if (threadIdx.x < a.experts) {
+        a.counts[threadIdx.x] = s_count[threadIdx.x];
+        a.offsets[threadIdx.x] = s_first[threadIdx.x];
+    }
+    if (ROUTE) {
+        for (int t = warp; t < a.tokens; t += blockDim.x >> 5)
+            if (lane == 0)
+                for (int i = t * a.top; i < (t + 1) * a.top; ++i) {
+                    const int first = s_first[a.ids[i]];
+                    a.rows[i] = first < 0 ? -1 : first + a.rows[i];
+                }
+    } else {
+        for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
+            const int first = s_first[a.ids[i]];
+            a.rows[i] = first < 0 ? -1 : first + a.rows[i];
+        }
+    }
+}
+
+// One CTA per token: its activations to the rows of its choices.
+__global__ void __launch_bounds__(128)
+moe_scatter_kernel(const uint4* __restrict__ hidden, uint4* __restrict__ xp, const int32_t* __restrict__ rows, int top_k,
+                   int vec_per_row) {
+    __shared__ int s_row[kMaxTopK];
+    pdl_launch_dependents();
+    pdl_wait_prior();
+    const int64_t t = blockIdx.x;
+    if (threadIdx.x < top_k) s_row[threadIdx.x] = rows[t * top_k + threadIdx.x];
+    __syncthreads();
+    for (int v = threadIdx.x; v < vec_per_row; v += blockDim.x) {
+        const uint4 x = hidden[t * vec_per_row + v];
+        for (int k = 0; k < top_k; ++k)
+            if (s_row[k] >= 0) xp[static_cast<int64_t>(s_row[k]) * vec_per_row + v] = x;   // (else another rank's expert)
+    }
 }
 
 // out[t] = fold over k of bf16(acc + bf16(y[pos[t,k]] * w[t,k])), acc starting at 0.
@@ -448,7 +500,7 @@ score_place_kernel(uint4* __restrict__ xp, const uint4* __restrict__ x, int32_t*
 }
 
 struct MoeWorkspace {
-    int32_t *ids, *counts, *offsets, *cursor, *pos;
+    int32_t *ids, *counts, *offsets, *pos;
     float* weights;
     __nv_bfloat16 *xp, *hact, *y2;
 };
@@ -468,7 +520,6 @@ int64_t carve(MoeWorkspace* w, uint8_t* base, int tokens, int E, int top_k, int 
     w->pos = reinterpret_cast<int32_t*>(take(pairs * 4));
     w->counts = reinterpret_cast<int32_t*>(take((E + 1) * 4));
     w->offsets = reinterpret_cast<int32_t*>(take((E + 1) * 4));
-    w->cursor = reinterpret_cast<int32_t*>(take((E + 1) * 4));
     w->xp = reinterpret_cast<__nv_bfloat16*>(take(pairs * H * 2));
     w->hact = reinterpret_cast<__nv_bfloat16*>(take(pairs * I * 2));
     w->y2 = reinterpret_cast<__nv_bfloat16*>(take(pairs * H * 2));
@@ -531,7 +582,7 @@ int launch_moe_route(int32_t* ids, float* weights, int32_t* counts, const void* 
     B200_CHECK_CUDA(cudaMemsetAsync(counts, 0, (E + 1) * sizeof(int32_t), stream));
     const bool pdl = pdl_launches_enabled();
     set_pdl_launches(false);  // follows a memset
-    cudaError_t ce = launch_kernel(moe_route_kernel, dim3(div_ceil(tokens, 4)), dim3(128), 0, stream, dim3(1, 1, 1),
+    cudaError_t ce = launch_kernel(moe_route_kernel<true>, dim3(div_ceil(tokens, 4)), dim3(128), 0, stream, dim3(1, 1, 1),
                                    static_cast<const __nv_bfloat16*>(logits), tokens, E, top_k, renorm, ids,
                                    weights, counts);
     set_pdl_launches(pdl);
@@ -547,21 +598,41 @@ int launch_moe_forward(void* out, const void* hidden, const void* router_logits,
     MoeWorkspace w;
     carve(&w, static_cast<uint8_t*>(workspace), tokens, E, top_k, H, I);
     const int pairs = tokens * top_k;
-    int err = launch_moe_route(w.ids, w.weights, w.counts, router_logits, tokens, E, top_k, renorm, stream);
-    if (err != B200_OK) return err;
-    B200_CHECK_CUDA(launch_kernel(moe_scan_kernel, dim3(1), dim3(256), 0, stream, dim3(1, 1, 1),
-                                  static_cast<const int32_t*>(w.counts), w.offsets, w.cursor, E, expert_begin,
-                                  num_local_experts));
-    B200_CHECK_CUDA(launch_kernel(moe_scatter_kernel, dim3(pairs), dim3(128), 0, stream, dim3(1, 1, 1),
-                                  static_cast<const uint4*>(hidden), reinterpret_cast<uint4*>(w.xp),
-                                  static_cast<const int32_t*>(w.ids), static_cast<const int32_t*>(w.offsets),
-                                  w.cursor, w.pos, top_k, H / 8));
+    PlaceArgs place;
+    place.logits = static_cast<const __nv_bfloat16*>(router_logits);
+    place.weights = w.weights;
+    place.ids = w.ids;
+    place.counts = w.counts;
+    place.offsets = w.offsets;
+    place.rows = w.pos;
+    place.tokens = tokens;
+    place.experts = E;
+    place.top = top_k;
+    place.renorm = renorm;
+    place.e_begin = expert_begin;
+    place.e_count = num_local_experts;
+    if (tokens <= kRouteInOneCta) {
+        B200_CHECK_CUDA(launch_kernel(moe_place_kernel<true>, dim3(1), dim3(1024), 0, stream, dim3(1, 1, 1), place));
+    } else {
+        B200_CHECK_CUDA(launch_kernel(moe_route_kernel<false>, dim3(div_ceil(tokens, 4)), dim3(128), 0, stream, dim3(1, 1, 1),
+                                      place.logits, tokens, E, top_k, renorm, w.ids, w.weights, nullptr));
+        B200_CHECK_CUDA(launch_kernel(moe_place_kernel<false>, dim3(1), dim3(1024), 0, stream, dim3(1, 1, 1), place));
+    }
+    // (few tokens: not as a dependent of the placing kernel.  The experts' kernel that runs here keeps x in L1, and CTAs of it
+    // that start under kernels with large rings find the SM divided for those: 103 + 48 us against 93 + 42)
+    const bool pdl = pdl_launches_enabled();
+    if (tokens <= kRouteInOneCta) set_pdl_launches(false);
+    const cudaError_t ce = launch_kernel(moe_scatter_kernel, dim3(tokens), dim3(128), 0, stream, dim3(1, 1, 1),
+                                         static_cast<const uint4*>(hidden), reinterpret_cast<uint4*>(w.xp),
+                                         static_cast<const int32_t*>(w.pos), top_k, H / 8);
+    set_pdl_launches(pdl);
+    B200_CHECK_CUDA(ce);
     const int epi = activation == 1 ? B200_EPILOGUE_GEGLU_ERF : B200_EPILOGUE_SWIGLU;
     // A token picks distinct experts, so no expert gets more rows than there are tokens.
     // gate_up / down hold the local experts only, so group g is expert expert_begin + g.
     const int32_t* counts = w.counts + expert_begin;
     const int32_t* offsets = w.offsets + expert_begin;
-    err = launch_grouped_gemm(w.hact, w.xp, gate_up, counts, offsets, num_local_experts, tokens, pairs, 2 * I, H,
+    int err = launch_grouped_gemm(w.hact, w.xp, gate_up, counts, offsets, num_local_experts, tokens, pairs, 2 * I, H,
                               epi, status, stream);
     if (err != B200_OK) return err;
     err = launch_grouped_gemm(w.y2, w.hact, down, counts, offsets, num_local_experts, tokens, pairs, H, I,

@@ -100,3 +100,19 @@ def test_moe_rejects_bad_arguments(L, pkg):
         moe.forward(torch.zeros(3, 32, dtype=bf16, device="cuda"), torch.zeros(3, 4, dtype=bf16, device="cuda"))
     with pytest.raises(pkg.B200Error):
         moe.forward(torch.zeros(3, 64, dtype=bf16, device="cuda"), torch.zeros(2, 4, dtype=bf16, device="cuda"))
+
+
+@pytest.mark.parametrize("T", [1, 33, 64, 65, 129])   # both sides of the tokens that one CTA routes and places
+@pytest.mark.parametrize("E,k,begin,local", [(256, 16, 40, 160), (256, 16, 0, 256), (8, 3, 0, 8), (33, 1, 32, 1)])
+def test_moe_routes_and_places_rows(L, T, E, k, begin, local):
+    gen = torch.Generator().manual_seed(T + E)
+    hidden = randn_bf16(gen, T, 64)
+    logits = torch.randn(T, E, generator=gen).argsort(1).to(bf16) / 32   # distinct in every row
+    gu, dn = randn_bf16(gen, local, 128, 64, std=1 / 8), randn_bf16(gen, local, 64, 64, std=1 / 8)
+    moe = L.MoELayer(E, k, 64, 64, True, "silu", expert_begin=begin, num_local_experts=local)
+    moe.gate_up_proj.copy_(gu.cuda())
+    moe.down_proj.copy_(dn.cuda())
+    got = moe.forward(hidden.cuda(), logits.cuda())
+    want = O.moe_forward(hidden, logits, gu, dn, k, True, "silu", O.store_bf16, expert_begin=begin)
+    assert_close_bf16(got, want, 2e-2, 4 * 2 ** -7, f"moe forward {T}x{E} top{k}")
+    assert L.read_device_status() == (0, 0)
