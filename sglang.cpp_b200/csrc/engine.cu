@@ -572,9 +572,11 @@ int enqueue_forward(b200_engine* e, int phase, int B, int Bp, int T, int max_ext
                                e->status, s, &into_residual));
     }
 
+    // The add and norm behind an expert layer ride in the kernel that adds up its outputs (no all-reduce in between).
+    const bool moe_norms = m.num_experts > 0 && !tp && hidden <= kMoeNormHidden;
     for (int l = 0; l < (chain || fold ? 0 : m.num_layers); ++l) {
         LayerWeights& L = e->layers[l];
-        B200_TRY(add_norm(L.input_norm));
+        if (!moe_norms || l == 0) B200_TRY(add_norm(L.input_norm));
         HeadEpilogue he;
         fill_heads(he, l);
         if (heads_few) {
@@ -610,11 +612,13 @@ int enqueue_forward(b200_engine* e, int phase, int B, int Bp, int T, int max_ext
         B200_TRY(add_norm(L.post_norm));
         if (m.num_experts > 0) {
             // MoEMLP::forward (src/models/utils.cc:82-91): router logits, then the expert layer.
+            const MoeNorm norm{e->residual, l + 1 < m.num_layers ? e->layers[l + 1].input_norm : e->final_norm, m.rms_norm_eps,
+                               round_first ? 1 : 0};
             B200_TRY(linear(e->router_logits, e->x, L.router, nullptr, m.num_experts, hidden, B200_EPILOGUE_NONE));
             B200_TRY(launch_moe_forward(proj_out(), e->x, e->router_logits, L.experts_gate_up, L.experts_down, T,
                                         m.num_experts, m.num_experts_per_tok, hidden, e->moe_inter,
                                         m.norm_topk_prob, m.hidden_act == 1 ? 1 : 0, e->expert_begin,
-                                        e->experts_local, e->moe_ws, e->status, s));
+                                        e->experts_local, e->moe_ws, e->status, s, moe_norms ? &norm : nullptr));
             continue;
         }
         B200_TRY(linear(e->h, e->x, L.gate_up, nullptr, 2 * e->inter, hidden, epi));
@@ -622,7 +626,7 @@ int enqueue_forward(b200_engine* e, int phase, int B, int Bp, int T, int max_ext
     }
     if (fold)
         B200_TRY(launch_rmsnorm(e->x, e->residual, e->final_norm, T, hidden, m.rms_norm_eps, s));
-    else
+    else if (!moe_norms)
         B200_TRY(add_norm(e->final_norm));
     B200_TRY(enqueue_output(e, phase, B, Bp, sampling, step_index));
     e->launches_last_step = static_cast<int>(kernel_launch_count() - launches_before);

@@ -282,10 +282,19 @@ int launch_move_rows(void* out, const void* in, const int32_t* rows, int count, 
                      cudaStream_t stream);
 
 int64_t moe_workspace_bytes(int tokens, int E, int top_k, int H, int I);
+// What follows an expert layer whose experts are all on this device: residual <- residual + sum, out <- norm(residual) * weight
+// instead of the sum.  hidden <= kMoeNormHidden.
+struct MoeNorm {
+    void* residual;
+    const void* weight;
+    float eps;
+    int round_first;   // the sum is rounded before it is squared
+};
+constexpr int kMoeNormHidden = 8192;
 int launch_moe_forward(void* out, const void* hidden, const void* router_logits, const void* gate_up,
                        const void* down, int tokens, int E, int top_k, int H, int I, int renorm,
                        int activation, int expert_begin, int num_local_experts, void* workspace,
-                       int* status, cudaStream_t stream);
+                       int* status, cudaStream_t stream, const MoeNorm* norm = nullptr);
 
 // Decode-step layer chain (decode_chain.cu): o_proj -> add + norm -> gate_up -> act -> down ->
 // add + norm -> the next layer's qkv -> QK-norm -> RoPE -> KV store, as one persistent kernel.

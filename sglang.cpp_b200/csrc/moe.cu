@@ -182,30 +182,105 @@ moe_scatter_kernel(const uint4* __restrict__ hidden, uint4* __restrict__ xp, con
     }
 }
 
-// out[t] = fold over k of bf16(acc + bf16(y[pos[t,k]] * w[t,k])), acc starting at 0.
+// Eight elements of a token's output: fold over its choices of bf16(acc + bf16(y[row] * w)), acc starting at 0.  Rows are
+// fetched four at a time.
+__device__ __forceinline__ void combine8(float (&acc)[8], const uint4* __restrict__ y, const int32_t* __restrict__ rows,
+                                         const float* __restrict__ weights, int top_k, int vec_per_row, int v) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+    for (int k0 = 0; k0 < top_k; k0 += 4) {
+        int row[4];
+        float w[4];
+        uint4 a[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            row[k] = k0 + k < top_k ? rows[k0 + k] : -1;
+            w[k] = k0 + k < top_k ? weights[k0 + k] : 0.f;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (row[k] >= 0) a[k] = y[static_cast<int64_t>(row[k]) * vec_per_row + v];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            if (row[k] < 0) continue;  // another rank's expert: its term arrives through the all-reduce
+            const uint32_t aw[4] = {a[k].x, a[k].y, a[k].z, a[k].w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                acc[2 * j] = round_bf16(acc[2 * j] + round_bf16(bf16_lo(aw[j]) * w[k]));
+                acc[2 * j + 1] = round_bf16(acc[2 * j + 1] + round_bf16(bf16_hi(aw[j]) * w[k]));
+            }
+        }
+    }
+}
+
 __global__ void __launch_bounds__(128)
 moe_combine_kernel(uint4* __restrict__ out, const uint4* __restrict__ y, const int32_t* __restrict__ pos,
                    const float* __restrict__ weights, int top_k, int vec_per_row) {
     pdl_launch_dependents();
     pdl_wait_prior();
-    const int t = blockIdx.x;
+    const int64_t t = blockIdx.x;
     for (int v = threadIdx.x; v < vec_per_row; v += blockDim.x) {
-        float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        for (int k = 0; k < top_k; ++k) {
-            const float w = weights[t * top_k + k];
-            const int row = pos[t * top_k + k];
-            if (row < 0) continue;  // another rank's expert: its term arrives through the all-reduce
-            const uint4 a = y[static_cast<int64_t>(row) * vec_per_row + v];
-            const uint32_t aw[4] = {a.x, a.y, a.z, a.w};
+        float acc[8];
+        combine8(acc, y, pos + t * top_k, weights + t * top_k, top_k, vec_per_row, v);
+        out[t * vec_per_row + v] = make_uint4(pack_bf16(acc[0], acc[1]), pack_bf16(acc[2], acc[3]), pack_bf16(acc[4], acc[5]),
+                                              pack_bf16(acc[6], acc[7]));
+    }
+}
+
+// The same with what follows in an engine whose experts are all here: residual <- residual + sum, out <- norm(residual) * w,
+// with the roundings of the two kernels that it stands for (the sum's last one is combine8's).  One CTA per token, VECS
+// vectors per thread.
+template <int VECS>
+__global__ void __launch_bounds__(256)
+moe_combine_norm_kernel(uint4* __restrict__ out, uint4* __restrict__ residual, const uint4* __restrict__ y,
+                        const int32_t* __restrict__ pos, const float* __restrict__ weights, int top_k, int vec_per_row,
+                        const uint4* __restrict__ norm_w, float eps, int round_first) {
+    __shared__ float red[8];
+    pdl_launch_dependents();
+    const int64_t t = blockIdx.x;
+    uint4 nw[VECS];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                acc[2 * j] = round_bf16(acc[2 * j] + round_bf16(bf16_lo(aw[j]) * w));
-                acc[2 * j + 1] = round_bf16(acc[2 * j + 1] + round_bf16(bf16_hi(aw[j]) * w));
-            }
+    for (int i = 0; i < VECS; ++i) {
+        const int v = threadIdx.x + i * blockDim.x;
+        nw[i] = v < vec_per_row ? __ldg(norm_w + v) : make_uint4(0, 0, 0, 0);
+    }
+    pdl_wait_prior();
+    float x[VECS][8], ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < VECS; ++i) {
+        const int v = threadIdx.x + i * blockDim.x;
+        if (v >= vec_per_row) continue;
+        const uint4 r = residual[t * vec_per_row + v];
+        combine8(x[i], y, pos + t * top_k, weights + t * top_k, top_k, vec_per_row, v);
+        const uint32_t rw[4] = {r.x, r.y, r.z, r.w};
+        uint32_t sum[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            x[i][2 * j] += bf16_lo(rw[j]);
+            x[i][2 * j + 1] += bf16_hi(rw[j]);
+            sum[j] = pack_bf16(x[i][2 * j], x[i][2 * j + 1]);
+            if (round_first) x[i][2 * j] = bf16_lo(sum[j]), x[i][2 * j + 1] = bf16_hi(sum[j]);
         }
-        out[static_cast<int64_t>(t) * vec_per_row + v] =
-            make_uint4(pack_bf16(acc[0], acc[1]), pack_bf16(acc[2], acc[3]), pack_bf16(acc[4], acc[5]),
-                       pack_bf16(acc[6], acc[7]));
+        residual[t * vec_per_row + v] = make_uint4(sum[0], sum[1], sum[2], sum[3]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ss += x[i][j] * x[i][j];
+    }
+    ss = warp_sum(ss);
+    const int lane = threadIdx.x & 31;
+    if (lane == 0) red[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    ss = warp_sum(lane < static_cast<int>(blockDim.x >> 5) ? red[lane] : 0.f);
+    const float scale = rsqrtf(ss / static_cast<float>(vec_per_row * 8) + eps);
+#pragma unroll
+    for (int i = 0; i < VECS; ++i) {
+        const int v = threadIdx.x + i * blockDim.x;
+        if (v >= vec_per_row) continue;
+        const uint32_t ww[4] = {nw[i].x, nw[i].y, nw[i].z, nw[i].w};
+        uint32_t packed[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            packed[j] = pack_bf16(x[i][2 * j] * scale * bf16_lo(ww[j]), x[i][2 * j + 1] * scale * bf16_hi(ww[j]));
+        out[t * vec_per_row + v] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
     }
 }
 
@@ -593,7 +668,7 @@ int launch_moe_route(int32_t* ids, float* weights, int32_t* counts, const void* 
 int launch_moe_forward(void* out, const void* hidden, const void* router_logits, const void* gate_up,
                        const void* down, int tokens, int E, int top_k, int H, int I, int renorm,
                        int activation, int expert_begin, int num_local_experts, void* workspace,
-                       int* status, cudaStream_t stream) {
+                       int* status, cudaStream_t stream, const MoeNorm* norm) {
     if (tokens == 0) return B200_OK;
     MoeWorkspace w;
     carve(&w, static_cast<uint8_t*>(workspace), tokens, E, top_k, H, I);
@@ -638,6 +713,15 @@ int launch_moe_forward(void* out, const void* hidden, const void* router_logits,
     err = launch_grouped_gemm(w.y2, w.hact, down, counts, offsets, num_local_experts, tokens, pairs, H, I,
                               B200_EPILOGUE_NONE, status, stream);
     if (err != B200_OK) return err;
+    if (norm != nullptr) {
+        const int vecs = H / 8, threads = vecs <= 256 ? (vecs + 31) / 32 * 32 : 256;
+        auto kernel = vecs <= 256 ? moe_combine_norm_kernel<1> : vecs <= 512 ? moe_combine_norm_kernel<2> : moe_combine_norm_kernel<4>;
+        B200_CHECK_CUDA(launch_kernel(kernel, dim3(tokens), dim3(threads), 0, stream, dim3(1, 1, 1), static_cast<uint4*>(out),
+                                      static_cast<uint4*>(norm->residual), reinterpret_cast<const uint4*>(w.y2),
+                                      static_cast<const int32_t*>(w.pos), static_cast<const float*>(w.weights), top_k, vecs,
+                                      static_cast<const uint4*>(norm->weight), norm->eps, norm->round_first));
+        return B200_OK;
+    }
     B200_CHECK_CUDA(launch_kernel(moe_combine_kernel, dim3(tokens), dim3(128), 0, stream, dim3(1, 1, 1),
                                   static_cast<uint4*>(out), reinterpret_cast<const uint4*>(w.y2),
                                   static_cast<const int32_t*>(w.pos), static_cast<const float*>(w.weights),
@@ -752,7 +836,7 @@ int b200_moe_forward_local(void* out, const void* hidden_states, const void* rou
     return b200::launch_moe_forward(out, hidden_states, router_logits, gate_up_proj, down_proj, tokens,
                                     num_experts, top_k, hidden_size, intermediate_size, renormalize, activation,
                                     expert_begin, num_local_experts, workspace, status,
-                                    static_cast<cudaStream_t>(stream));
+                                    static_cast<cudaStream_t>(stream), nullptr);
 }
 
 int b200_moe_forward(void* out, const void* hidden_states, const void* router_logits, const void* gate_up_proj,

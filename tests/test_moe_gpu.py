@@ -116,3 +116,32 @@ def test_moe_routes_and_places_rows(L, T, E, k, begin, local):
     want = O.moe_forward(hidden, logits, gu, dn, k, True, "silu", O.store_bf16, expert_begin=begin)
     assert_close_bf16(got, want, 2e-2, 4 * 2 ** -7, f"moe forward {T}x{E} top{k}")
     assert L.read_device_status() == (0, 0)
+
+
+@pytest.mark.parametrize("H,k,qk_norm", [(64, 1, True), (2304, 5, False), (4224, 6, True)])   # one, two and four vectors per thread
+def test_expert_sum_with_the_norm_behind_it(L, pkg, H, k, qk_norm):
+    """In an engine the kernel that adds up the experts' outputs adds the residual and normalises too: logits of a prompt and of
+    a decode step against the oracle.  Two pipelines that sum in different orders may round every stored tensor one way or the
+    other: the residual after each of four blocks and the logits, five independent steps (2^-8 relative) add up to sqrt(5) on
+    average; at most four at the largest logit.  (Add and norm as kernels of their own give the same bits as this.)"""
+    import numpy as np
+
+    from tests.test_engine_gpu import Pair
+
+    cfg = O.ModelConfig(2, H, 2, 1, 128, 128, 512, 1e-6, 1e4, 512, False, qk_norm, qk_norm, "silu", 8, k, 64, True)
+    pr = Pair(pkg, cfg, 16)
+    prompt = np.random.default_rng(H).integers(0, 512, size=70).astype(np.int32)
+    reqs = [pr.hb.add_request(prompt, 4)]
+    pr.host_tokens = {reqs[0].table_idx: list(prompt) + [0] * 8}
+    for prefill in (True, False):
+        pr.hb.allocate(reqs)
+        ob, pt = pr.oracle_batch(reqs, prefill)
+        want = pr.oracle.forward(ob, pr.kv, pt)
+        (pr.hb.prefill if prefill else pr.hb.decode)(reqs).synchronize()
+        got = pr.engine.logits(1)
+        diff, rms = (got.float() - want.float()).abs(), float(want.float().pow(2).mean().sqrt())
+        assert float(diff.max()) <= 4 * 2 ** -8 * float(want.float().abs().max()) and float(diff.mean()) <= rms * 2 ** -8 * 5 ** 0.5
+        token = int(want.argmax())
+        pr.host_tokens[reqs[0].table_idx][reqs[0].cached_len] = token
+        pr.engine.write_token_pool([reqs[0].table_idx], [reqs[0].cached_len], [token])
+    pr.engine.close()
