@@ -127,6 +127,12 @@ __global__ void publish_step_kernel(int32_t* __restrict__ tokens_out, uint8_t* _
     }
 }
 
+__global__ void publish_tokens_kernel(int32_t* __restrict__ tokens_out, int32_t* __restrict__ status_out,
+                                      const int32_t* __restrict__ next_tokens, const int* __restrict__ status, int B) {
+    for (int i = threadIdx.x; i < B; i += blockDim.x) tokens_out[i] = next_tokens[i];
+    if (threadIdx.x < 2) status_out[threadIdx.x] = status[threadIdx.x];
+}
+
 __global__ void fill_int32_kernel(int32_t* p, int32_t v, int64_t n) {
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i < n) p[i] = v;
@@ -868,7 +874,7 @@ static int create_engine(const b200_model_config* model, const b200_stack_config
     E_TRY(dev_alloc(e, reinterpret_cast<void**>(&e->row_ids_dev), e->max_batch * 4, true));
 
     e->meta_ints = 9 * e->max_batch + 16;
-    if (cudaMallocHost(&e->meta_host, e->meta_ints * sizeof(int32_t)) != cudaSuccess) {
+    if (cudaMallocHost(&e->meta_host, (e->meta_ints + 2) * sizeof(int32_t)) != cudaSuccess) {
         set_last_error("engine_create: pinned staging allocation failed");
         return fail(B200_ERR_CUDA);
     }
@@ -1115,9 +1121,25 @@ static int run_step(b200_engine* e, const b200_step* st, int32_t* next_tokens_ho
     } else {
         B200_TRY(enqueue_forward(e, st->phase, B, Bg, T, max_ext, sampling, st->step_index));
     }
-    if (next_tokens_host && B > 0)
-        B200_CHECK_CUDA(cudaMemcpyAsync(next_tokens_host, e->next_tokens, B * sizeof(int32_t),
-                                        cudaMemcpyDeviceToHost, s));
+    // Tokens and what the step's kernels report, written to the host by one kernel where the caller's buffer is pinned (two
+    // copies on the engine's stream take 12 us, and a copy for b200_engine_synchronize alone as long).
+    e->status_copied = slot == nullptr;
+    if (!slot) {
+        const bool tokens = next_tokens_host && B > 0;
+        cudaPointerAttributes at = {};
+        const bool pinned = !tokens || (cudaPointerGetAttributes(&at, next_tokens_host) == cudaSuccess &&
+                                        at.type == cudaMemoryTypeHost && at.devicePointer != nullptr);
+        if (!pinned) {
+            cudaGetLastError();
+            B200_CHECK_CUDA(cudaMemcpyAsync(next_tokens_host, e->next_tokens, B * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+        }
+        void* status_host = nullptr;
+        B200_CHECK_CUDA(cudaHostGetDevicePointer(&status_host, e->meta_host + e->meta_ints, 0));
+        B200_CHECK_CUDA(launch_kernel(publish_tokens_kernel, dim3(1), dim3(128), 0, s, dim3(1, 1, 1),
+                                      static_cast<int32_t*>(at.devicePointer), static_cast<int32_t*>(status_host),
+                                      static_cast<const int32_t*>(e->next_tokens), static_cast<const int*>(e->status),
+                                      pinned && tokens ? B : 0));   // (not one of the model's: not counted with them)
+    }
     if (slot) {
         B200_CHECK_CUDA(launch_kernel(publish_step_kernel, dim3(1), dim3(256), 0, s, dim3(1, 1, 1), slot->tokens,
                                       slot->finished, static_cast<const uint8_t*>(slot->ignore_eos), slot->status,
@@ -1191,8 +1213,10 @@ int b200_engine_wait(b200_engine* e, int64_t ticket, const int32_t** tokens, con
 int b200_engine_synchronize(b200_engine* e) {
     B200_CHECK_ARG(e, "engine_synchronize: NULL engine");
     B200_CHECK_CUDA(cudaStreamSynchronize(e->stream));
-    int host[2] = {0, 0};
-    B200_CHECK_CUDA(cudaMemcpy(host, e->status, sizeof(host), cudaMemcpyDeviceToHost));
+    int host[2] = {e->meta_host[e->meta_ints], e->meta_host[e->meta_ints + 1]};
+    if (!e->status_copied)   // (something other than a step has run since)
+        B200_CHECK_CUDA(cudaMemcpy(host, e->status, sizeof(host), cudaMemcpyDeviceToHost));
+    e->status_copied = false;
     if (host[0] != 0) {
         cudaMemset(e->status, 0, sizeof(host));
         set_last_error("a bounded wait inside a kernel ran out (site %d)", host[0]);
@@ -1224,6 +1248,7 @@ int b200_engine_token_logits(b200_engine* e, const int32_t* tokens, int count, f
     const int row_bytes = hidden_row_bytes(e), vocab = e->m.vocab_size, ld = logits_ld(e);
     const size_t z = logits_f32(e) ? 4 : 2;
     std::vector<uint16_t> narrow;
+    e->status_copied = false;
     for (int i0 = 0; i0 < count; i0 += e->max_batch) {
         const int n = count - i0 < e->max_batch ? count - i0 : e->max_batch;
         B200_CHECK_CUDA(cudaStreamSynchronize(e->stream));

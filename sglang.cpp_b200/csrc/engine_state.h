@@ -68,7 +68,8 @@ struct b200_engine {
     void* moe_ws = nullptr;
 
     // per-step metadata: pinned staging + device mirror
-    int32_t* meta_host = nullptr;
+    int32_t* meta_host = nullptr;   // (and behind it the status words that came along with the last step)
+    bool status_copied = false;     // ... nothing but that step has run since they were read last
     int32_t* meta_dev = nullptr;
     int meta_ints = 0;
     int32_t *scatter_host = nullptr, *scatter_dev = nullptr;

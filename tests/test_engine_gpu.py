@@ -665,3 +665,41 @@ def test_engine_runs_a_checkpoint_read_from_safetensors_shards(pkg, tmp_path, ki
     check_logits(pr.engine.logits(2), want, f"{kind} checkpoint decode")
     assert pr.engine_status_clean()
     pr.engine.close()
+
+
+@pytest.mark.parametrize("nreq", [1, 5])
+def test_tokens_into_pinned_and_pageable_memory_and_reports_of_steps(pkg, nreq):
+    """The step's last kernel writes tokens into a pinned buffer; another buffer gets a copy.  What a step's kernels report comes
+    with it, whichever kind of step ran last, and is told once."""
+    import ctypes
+
+    from sglang_cpp_b200._lib import StepStruct, call
+
+    cfg = small_cfg("qwen3")
+    pr = Pair(pkg, cfg, 16)
+    rng = np.random.default_rng(nreq)
+    reqs = [pr.hb.add_request(rng.integers(0, cfg.vocab_size, size=9 + i).astype(np.int32), 8) for i in range(nreq)]
+    pr.hb.allocate(reqs)
+    out = pr.hb.prefill(reqs)
+    out.synchronize()
+    e, rows = pr.engine, np.array([r.table_idx for r in reqs], np.int32)
+    zeros, lens, none = np.zeros(nreq, np.int32), np.array([9 + i for i in range(nreq)], np.int32), np.full(nreq, -1, np.int32)
+    pageable = np.full(nreq, -7, np.int32)
+    step = StepStruct(0, nreq, nreq, rows.ctypes.data, zeros.ctypes.data, lens.ctypes.data, none.ctypes.data, None, None, None, None, 0)
+    call("b200_engine_step", e._h, ctypes.byref(step), pageable.ctypes.data)   # the same prompts again
+    e.synchronize()
+    assert np.array_equal(pageable, out.next_tokens_cpu.numpy())
+    assert np.array_equal(e.forward_batch_async(0, rows, zeros, lens, none).wait()[0], pageable)
+    good = e.read_table("token_pool")[rows[0], :1].tolist()
+    e.write_token_pool(rows[:1], [0], [cfg.vocab_size + 3])   # a token that is no token
+    e.forward_batch(0, rows, zeros, lens, none)
+    with pytest.raises(pkg.B200Error, match=str(cfg.vocab_size + 3)):
+        e.synchronize()
+    e.synchronize()
+    e.forward_batch(0, rows, zeros, lens, none)               # reported by the step before the last one
+    e.forward_batch_async(0, rows, zeros, lens, none)
+    with pytest.raises(pkg.B200Error, match=str(cfg.vocab_size + 3)):
+        e.synchronize()
+    e.write_token_pool(rows[:1], [0], good)
+    e.forward_batch(0, rows, zeros, lens, none).synchronize()
+    e.close()
