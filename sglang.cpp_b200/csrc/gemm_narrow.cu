@@ -6,8 +6,8 @@
 //   * 16 rows of W per CTA and the whole of K, dealt to its warps: no exchange between CTAs.  A lane loads 16
 //     contiguous bytes of a row; which of the k of a 32-wide step these are does not matter, because x is loaded
 //     the same way, so the bytes are the operands of two m16n8k16 products as they are (weights as the left one,
-//     8 tokens as the right one).  No shared memory, no barrier before the sums meet.
-//   * the weights that fit in registers are requested before griddepcontrol.wait.  CTAs are small (8 warps, a few
+//     8 tokens as the right one).  No exchange through shared memory, no barrier before the sums meet.
+//   * the weights that fit in registers (or, in a chain of such calls, in shared memory) are requested before griddepcontrol.wait.  CTAs are small (8 warps, a few
 //     KB of shared memory), so those of the next kernels of the chain become resident beside the running one.
 //   * behind the wait: x (from L2), the products, one exchange through shared memory, the epilogue.
 // tcgen05 has no place here: its operands would have to pass through shared memory, and 128 x 64 tiles of W leave
@@ -63,6 +63,9 @@ __device__ __forceinline__ uint4 load_weights(const uint4* p) {
     asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
     return v;
 }
+__device__ __forceinline__ void stage_weights(uint4* to, const uint4* from) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(to)), "l"(from) : "memory");
+}
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void store_in_cluster(const float* mine, uint32_t rank, float v) {
@@ -105,9 +108,11 @@ __device__ __forceinline__ void store_plain(const NarrowParams& p, bool gated, i
 }
 
 // BUFS register buffers of kSteps steps: with one, a warp's whole share of K is requested ahead of the wait.
-template <int KIND, bool NORM, int NT, int WARPS, int BUFS>
+// STAGED: the share goes to shared memory instead (every lane reads back what it has copied itself).
+template <int KIND, bool NORM, int NT, int WARPS, int BUFS, bool STAGED>
 __global__ void __launch_bounds__(WARPS * 32)
 narrow_gemm_kernel(const NarrowParams p) {
+    extern __shared__ uint4 s_weights[];   // STAGED: [warp][step][row group][lane]
     __shared__ float s_part[WARPS][NT * 8 * kTokenPitch];
     __shared__ float s_ssq[WARPS][NT * 8];
     __shared__ float s_head[kHeadRanks][NT * 8];
@@ -131,7 +136,9 @@ narrow_gemm_kernel(const NarrowParams p) {
     const uint4* wb = reinterpret_cast<const uint4*>(p.w + row_b * p.K) + t;
     const int first = warp * p.steps / WARPS, last = (warp + 1) * p.steps / WARPS;
     const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-    uint4 a[BUFS][kSteps], b[BUFS][kSteps];
+    constexpr int kShare = BUFS * kSteps;   // steps of a warp that are requested ahead of the wait
+    uint4* staged = s_weights + warp * kShare * 64 + lane;
+    uint4 a[STAGED ? 1 : BUFS][kSteps], b[STAGED ? 1 : BUFS][kSteps];
     auto fetch = [&](int buf, int at) {
 #pragma unroll
         for (int u = 0; u < kSteps; ++u) {
@@ -140,8 +147,18 @@ narrow_gemm_kernel(const NarrowParams p) {
             b[buf][u] = there ? load_weights(wb + (at + u) * 4) : zero;
         }
     };
+    if constexpr (STAGED) {
 #pragma unroll
-    for (int i = 0; i < BUFS; ++i) fetch(i, first + i * kSteps);
+        for (int u = 0; u < kShare; ++u)
+            if (first + u < last) {
+                stage_weights(staged + u * 64, wa + (first + u) * 4);
+                stage_weights(staged + u * 64 + 32, wb + (first + u) * 4);
+            }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    } else {
+#pragma unroll
+        for (int i = 0; i < BUFS; ++i) fetch(i, first + i * kSteps);
+    }
     // what the epilogue needs and no kernel of the chain writes: one thread per token and pair of features
     const int m = static_cast<int>(threadIdx.x) >> 3, f = static_cast<int>(threadIdx.x) & 7;
     const bool finishes = threadIdx.x < NT * 64;
@@ -187,6 +204,24 @@ narrow_gemm_kernel(const NarrowParams p) {
     const uint4* xr[NT];
 #pragma unroll
     for (int n = 0; n < NT; ++n) xr[n] = reinterpret_cast<const uint4*>(p.x + (n * 8 + g) * p.ldx) + t;
+    // products of one step's weights with the tokens' x, normalised input included
+    auto step = [&](const uint4& wa4, const uint4& wb4, const uint4 (&x)[NT], const uint4& nw) {
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+            uint32_t v[4] = {x[n].x, x[n].y, x[n].z, x[n].w};
+            if (NORM) {
+                const uint32_t w4[4] = {nw.x, nw.y, nw.z, nw.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float lo = bf16_lo(v[e]), hi = bf16_hi(v[e]);
+                    ss[n] = fmaf(lo, lo, fmaf(hi, hi, ss[n]));
+                    v[e] = pack_bf16(lo * bf16_lo(w4[e]), hi * bf16_hi(w4[e]));
+                }
+            }
+            mma_bf16_16816(acc[n], {wa4.x, wb4.x, wa4.y, wb4.y}, v[0], v[1]);
+            mma_bf16_16816(acc[n], {wa4.z, wb4.z, wa4.w, wb4.w}, v[2], v[3]);
+        }
+    };
     auto multiply = [&](int buf, int at) {
         uint4 x[kSteps][NT], nw[kSteps];
 #pragma unroll
@@ -196,25 +231,21 @@ narrow_gemm_kernel(const NarrowParams p) {
             if (NORM) nw[u] = at + u < last ? *(reinterpret_cast<const uint4*>(p.norm_w) + (at + u) * 4 + t) : zero;
         }
 #pragma unroll
-        for (int u = 0; u < kSteps; ++u) {
-#pragma unroll
-            for (int n = 0; n < NT; ++n) {
-                uint32_t v[4] = {x[u][n].x, x[u][n].y, x[u][n].z, x[u][n].w};
-                if (NORM) {
-                    const uint32_t w4[4] = {nw[u].x, nw[u].y, nw[u].z, nw[u].w};
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        const float lo = bf16_lo(v[e]), hi = bf16_hi(v[e]);
-                        ss[n] = fmaf(lo, lo, fmaf(hi, hi, ss[n]));
-                        v[e] = pack_bf16(lo * bf16_lo(w4[e]), hi * bf16_hi(w4[e]));
-                    }
-                }
-                mma_bf16_16816(acc[n], {a[buf][u].x, b[buf][u].x, a[buf][u].y, b[buf][u].y}, v[0], v[1]);
-                mma_bf16_16816(acc[n], {a[buf][u].z, b[buf][u].z, a[buf][u].w, b[buf][u].w}, v[2], v[3]);
-            }
-        }
+        for (int u = 0; u < kSteps; ++u) step(a[buf][u], b[buf][u], x[u], nw[u]);
     };
-    if (BUFS == 1) {
+    if constexpr (STAGED) {
+        uint4 x[kShare][NT], nw[kShare];
+#pragma unroll
+        for (int u = 0; u < kShare; ++u) {
+#pragma unroll
+            for (int n = 0; n < NT; ++n) x[u][n] = first + u < last && n * 8 + g < p.M ? xr[n][(first + u) * 4] : zero;
+            if (NORM) nw[u] = first + u < last ? *(reinterpret_cast<const uint4*>(p.norm_w) + (first + u) * 4 + t) : zero;
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+        for (int u = 0; u < kShare; ++u)
+            if (first + u < last) step(staged[u * 64], staged[u * 64 + 32], x[u], nw[u]);
+    } else if (BUFS == 1) {
         multiply(0, first);
     } else {
         for (int at = first; at < last; at += BUFS * kSteps) {
@@ -375,15 +406,32 @@ narrow_grouped_kernel(const NarrowParams p, const int32_t* __restrict__ counts, 
 template <int KIND, bool NORM, int NT>
 cudaError_t launch(const NarrowParams& p, int tiles, cudaStream_t stream) {
     const dim3 cluster(KIND == kHeads ? kHeadRanks : 1, 1, 1);
-    auto go = [&](auto kernel, int warps) {
-        return launch_kernel(kernel, dim3(tiles), dim3(warps * 32), 0, stream, cluster, p);
+    auto go = [&](auto kernel, int warps, size_t smem) {
+        if (smem > 0) {
+            const cudaError_t err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+            if (err != cudaSuccess) return err;
+        }
+        return launch_kernel(kernel, dim3(tiles), dim3(warps * 32), smem, stream, cluster, p);
     };
+    // In a decode step whose projections are all this kernel's (dense models: norms and residual ride in them) the weights are
+    // staged in shared memory.  In registers they keep the next kernels' CTAs out: 64 CTAs of 1024 x 3072 with 16 warps and 128
+    // registers each wait for empty SMs until gate and up (384 CTAs) end, and then take 4 us to request their weights.  Steps of
+    // Qwen3-0.6B, 1 request of 700 keys / 2 of 300 / 5 of 200 to 3000 / 12 of 500: 598 / 627 / 872 / 976 us against 674 / 696 /
+    // 987 / 1050.  Elsewhere L1 is worth more to the kernels around than shared memory to this one (Qwen3-MoE, 1 request: 660 us
+    // against 649; Saluzen, 2 requests: 426 against 407).
+    constexpr bool kStage = NORM || KIND == kResidual;
+    auto share_bytes = [](int warps, int bufs) { return kStage ? static_cast<size_t>(warps) * bufs * kSteps * 1024 : 0; };
     // Few tiles: more warps each.  A share of K that one buffer holds needs fewer registers.
     if (tiles <= sm_count() && p.steps > 8 * kSteps) {
-        if (p.steps <= 16 * kSteps) return go(narrow_gemm_kernel<KIND, NORM, NT, 16, 1>, 16);
-        if constexpr (KIND != kHeads && !NORM) return go(narrow_gemm_kernel<KIND, NORM, NT, 16, 2>, 16);
+        if (p.steps <= 16 * kSteps) return go(narrow_gemm_kernel<KIND, NORM, NT, 16, 1, kStage>, 16, share_bytes(16, 1));
+        if constexpr (KIND != kHeads && !NORM) {
+            if (p.steps <= 32 * kSteps) return go(narrow_gemm_kernel<KIND, NORM, NT, 16, 2, kStage>, 16, share_bytes(16, 2));
+            return go(narrow_gemm_kernel<KIND, NORM, NT, 16, 2, false>, 16, 0);
+        }
     }
-    return p.steps <= 8 * kSteps ? go(narrow_gemm_kernel<KIND, NORM, NT, 8, 1>, 8) : go(narrow_gemm_kernel<KIND, NORM, NT, 8, 2>, 8);
+    if (p.steps <= 8 * kSteps) return go(narrow_gemm_kernel<KIND, NORM, NT, 8, 1, kStage>, 8, share_bytes(8, 1));
+    if (p.steps <= 16 * kSteps) return go(narrow_gemm_kernel<KIND, NORM, NT, 8, 2, kStage>, 8, share_bytes(8, 2));
+    return go(narrow_gemm_kernel<KIND, NORM, NT, 8, 2, false>, 8, 0);   // (K beyond what is requested ahead)
 }
 
 template <int KIND, bool NORM>

@@ -72,6 +72,16 @@ def test_decode_of_a_wide_layer(pkg, monkeypatch, qwen, hidden, nreq, narrow, fo
     folded_decode(pkg, monkeypatch, "wide", nreq, fold_heads)
 
 
+@pytest.mark.parametrize("nreq", [1, 8, 9, 16])
+@pytest.mark.parametrize("inter", [576, 2048, 2112, 4032, 4096, 4160])   # steps of 32 that do not fall evenly to the warps; one and
+def test_decode_with_staged_weights(pkg, monkeypatch, inter, nreq):      # two buffers; the most that is requested ahead, and more
+    """The down projection of a decode step, K = `inter`, keeps its weights in shared memory."""
+    cfg = O.ModelConfig(1, 256, 4, 2, 128, inter, 1024, 1e-6, 1e6, 512, True, True, True)
+    assert on_narrow(pkg, cfg, nreq)
+    monkeypatch.setattr(engine_tests, "small_cfg", lambda kind: cfg)
+    folded_decode(pkg, monkeypatch, "long", nreq, "1")
+
+
 @pytest.mark.parametrize("nreq", [1, 9])
 def test_values_that_are_not_finite_stay_where_they_are(pkg, nreq):
     """Values are not rotated: an infinite one must not reach the feature that a rotation would pair it with."""
