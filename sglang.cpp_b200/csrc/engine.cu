@@ -396,7 +396,10 @@ int enqueue_forward(b200_engine* e, int phase, int B, int Bp, int T, int max_ext
     // two exchange rounds (128 tokens) the separate kernel is the faster of the two, and on a sharded
     // engine (few heads per rank) it is no gain: Llama-3-8B at batch 128 ran 7.21 against 7.44 ms with it
     // on one GPU, 5.52 against 5.51 on two, 3.33 against 3.31 on eight.
-    const bool heads_in_qkv = e->use_fold_heads && d == 128 && T <= 128 && !tp &&
+    // Up to 16 rows of a W that the ring kernel takes: that one, and the head pass behind it (Llama-3-8B, 4 requests: 3077 us per step
+    // against 3285).
+    const bool qkv_on_ring = e->use_fold && !fold && ring_gemm_takes(nullptr, nullptr, T, e->qkv_dim, hidden, hidden, B200_EPILOGUE_NONE, false);
+    const bool heads_in_qkv = e->use_fold_heads && d == 128 && T <= 128 && !tp && !qkv_on_ring &&
                               skinny_gemm_split(T, e->qkv_dim, hidden, B200_EPILOGUE_NONE) > 1;
 
     const bool heads_few = e->use_fold && e->use_fold_heads && d == 128 && !tp &&

@@ -1,0 +1,386 @@
+// y = x W^T for a handful of rows and a W that takes longer to read than a kernel takes to start: one CTA per SM streams its
+// share of W through a ring in shared memory.
+//
+// What bounds it is the memory, and what keeps a kernel from the memory's rate here is that nothing is requested while a CTA
+// finishes, while the next one starts, and while the kernel before ends.  So
+//   * a CTA walks over tiles of 16 rows of W; one thread does nothing but request them, 16 KB at a time (512 of K: one copy, or two
+//     where gate and up rows lie apart) and x of the same columns, as far ahead as the ring goes, from one tile to the next
+//     without a break (x by the multiplying warps themselves, two stages ahead: trips to L2 beside a memory in full use take 1500
+//     cycles, 97 us more for an expert layer);
+//   * the weights do not depend on the kernel before, so the ring fills with them ahead of griddepcontrol.wait;
+//   * the ring holds 96 KB of weights (64 KB, so that two CTAs share an SM: 3350 us per step of Llama-3-8B with 4 requests against
+//     3077; 128 KB 3134).
+// A warp multiplies 64 of a stage's 512 columns: 16 bytes of a row are operands of two mma.sync products as they are (as in
+// gemm_narrow.cu), the sums of the eight warps meet once per tile.
+//
+// Experts (GROUPED): the same over the tiles of all groups that have rows, 8 rows at a time.
+#include "common.cuh"
+#include "kernels.h"
+#include "narrow.cuh"
+#include "tensormap.cuh"
+
+namespace b200 {
+namespace {
+
+constexpr int kChunk = 512;                        // columns per stage, 64 per warp
+constexpr uint32_t kWBytes = 16 * kChunk * 2, kXBytes = 8 * kChunk * 2;   // of a stage, x per block of 8 tokens
+constexpr int kStages = 6;
+constexpr int kWideStages = 4;                     // GROUPED, where some group has more than 8 rows
+constexpr uint32_t ring_bytes(int blocks) { return kStages * (kWBytes + blocks * kXBytes); }
+static_assert(kWideStages * (kWBytes + 2 * kXBytes) <= ring_bytes(1), "");
+constexpr int kWarps = 8;                          // that multiply; one more requests
+constexpr int kMaxRingGroups = 1024;
+
+struct RingPass {   // of a group's rows over its weights
+    int group, x_row, count;
+};
+
+struct RingShared {
+    alignas(8) uint64_t full[kStages];
+    alignas(8) uint64_t empty[kStages];
+    float part[2][kWarps][8 * kTokenPitch];
+    int passes, wide;
+};
+
+struct RingParams : NarrowOut {
+    const __nv_bfloat16* bias;
+    int M, n_rows, up_row_offset, tiles, chunks, K;
+    int x_box;        // rows of x per copy
+    int* status;
+    const int32_t *counts, *offsets;   // GROUPED
+    int groups;
+};
+
+// A CTA's share: tiles of every pass.  BLOCKS of 8 tokens (GROUPED: at most that many of a group in one pass over its weights).
+template <bool GROUPED, int BLOCKS, int STAGES>
+__device__ __forceinline__ void ring_walk(const CUtensorMap& tmap_w, const CUtensorMap& tmap_x, const RingParams& p, uint32_t ring,
+                                          const RingPass* s_pass, RingShared& s, int warp, int lane) {
+    constexpr uint32_t kStageBytes = kWBytes + BLOCKS * kXBytes;
+    const bool gated = p.up_row_offset > 0;
+    // this CTA's tiles: neighbours, so that experts change rarely
+    const int64_t items = static_cast<int64_t>(GROUPED ? s.passes : 1) * p.tiles;
+    const int first = static_cast<int>(items * blockIdx.x / gridDim.x), last = static_cast<int>(items * (blockIdx.x + 1) / gridDim.x);
+    bool failed = false;
+
+    // a place in the walk: stepped, not found by division
+    struct Place {
+        int pass, tile, w_row, x_row, count;
+    };
+    auto open = [&](Place& at) {
+        const RingPass r = GROUPED ? s_pass[at.pass] : RingPass{0, 0, p.M};
+        at.w_row = r.group * p.n_rows + at.tile * (gated ? 8 : 16);
+        at.x_row = r.x_row;
+        at.count = r.count;
+    };
+    auto start = [&]() {
+        Place at = {GROUPED ? first / p.tiles : 0, GROUPED ? first % p.tiles : first, 0, 0, 0};
+        if (first < last) open(at);
+        return at;
+    };
+    auto next = [&](Place& at, int item) {   // `item`: the one to come
+        ++at.tile;
+        at.w_row += gated ? 8 : 16;
+        if (GROUPED && at.tile == p.tiles) {
+            at.tile = 0;
+            ++at.pass;
+            if (item < last) open(at);
+        }
+    };
+
+    if (warp == kWarps) {
+        // ================= requests =================
+        if (lane == 0) {
+            auto request_w = [&](const Place& at, int c, uint32_t slot) {
+                const uint32_t bar = smem_u32(&s.full[slot]), dst = ring + slot * kStageBytes;
+                mbar_arrive_expect_tx(bar, kWBytes + (GROUPED && BLOCKS > 1 && at.count > 8 ? 2 : 1) * p.x_box * (kChunk * 2));
+                tma_load_3d(dst, &tmap_w, 0, at.w_row, c * (kChunk / 64), bar);
+                if (gated) tma_load_3d(dst + kWBytes / 2, &tmap_w, 0, at.w_row + p.up_row_offset, c * (kChunk / 64), bar);
+            };
+            auto request_x = [&](const Place& at, int c, uint32_t slot) {
+                const uint32_t dst = ring + slot * kStageBytes + kWBytes;
+                tma_load_3d(dst, &tmap_x, 0, at.x_row, c * (kChunk / 64), smem_u32(&s.full[slot]));
+                if (GROUPED && BLOCKS > 1 && at.count > 8)
+                    tma_load_3d(dst + kXBytes, &tmap_x, 0, at.x_row + 8, c * (kChunk / 64), smem_u32(&s.full[slot]));
+            };
+            // the first ring-full of weights does not wait for the kernel before this one
+            const int early = GROUPED ? 0 : min(STAGES, (last - first) * p.chunks);
+            Place ahead = start();
+            for (int i = 0, c = 0; i < early; ++i) {
+                request_w(ahead, c, i);
+                if (++c == p.chunks) {
+                    c = 0;
+                    next(ahead, first + (i + 1) / p.chunks);
+                }
+            }
+            if (!GROUPED) pdl_wait_prior();
+            uint32_t slot = 0, phase = 1;   // (the first waits are for stages that nobody has used)
+            int it = 0;
+            Place at = start();
+            for (int item = first; item < last && !failed; next(at, ++item)) {
+                for (int c = 0; c < p.chunks; ++c, ++it) {
+                    if (!mbar_wait_mostly_ready(smem_u32(&s.empty[slot]), phase, p.status, 131)) {
+                        failed = true;
+                        break;
+                    }
+                    if (it >= early) request_w(at, c, slot);
+                    request_x(at, c, slot);
+                    if (++slot == STAGES) {
+                        slot = 0;
+                        phase ^= 1;
+                    }
+                }
+            }
+        }
+        return;
+    }
+
+    // ================= products =================
+    if (!GROUPED) pdl_wait_prior();
+    const int g = lane >> 2, t = lane & 3;
+    // Rows of the operands are rows of W, and tokens, in an order in which neighbouring lanes' 16 bytes lie in different banks.
+    const int local = (g >> 1) | ((g & 1) << 2);
+    const uint32_t row_a = static_cast<uint32_t>(warp) * (gated ? 1024u : 2048u) + local * 128;
+    const uint32_t row_b = row_a + (gated ? kWBytes / 2 : 1024u);
+    const uint32_t at[2] = {static_cast<uint32_t>(t ^ local) << 4, static_cast<uint32_t>((t + 4) ^ local) << 4};
+    // (x has p.x_box rows per block of 64 columns; what a token that is not there reads is used by nobody)
+    const uint32_t x_local = static_cast<uint32_t>(warp) * p.x_box + local;
+    const uint32_t row_x = kWBytes + x_local * 128;
+    const uint32_t at_x[2] = {(static_cast<uint32_t>(t) ^ (x_local & 7)) << 4, (static_cast<uint32_t>(t + 4) ^ (x_local & 7)) << 4};
+    auto lds = [&](uint32_t from) {
+        uint4 v;
+        asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(from) : "memory");
+        return v;
+    };
+    uint32_t slot = 0, phase = 0;
+    int parity = 0;
+    Place here = start();
+    for (int item = first; item < last; next(here, ++item)) {
+        float acc[BLOCKS][4] = {};
+        for (int c = 0; c < p.chunks; ++c) {
+            if (!failed && !mbar_wait_mostly_ready(smem_u32(&s.full[slot]), phase, p.status, 132)) failed = true;
+            const uint32_t base = ring + slot * kStageBytes;
+            // (columns behind K are zeros in both operands)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const uint4 a = lds(base + row_a + at[h]), b = lds(base + row_b + at[h]);
+#pragma unroll
+                for (int i = 0; i < BLOCKS; ++i) {
+                    if (GROUPED && i > 0 && here.count <= i * 8) break;
+                    const uint4 v = lds(base + row_x + i * (GROUPED ? kXBytes : 1024u) + at_x[h]);
+                    mma_bf16_16816(acc[i], {a.x, b.x, a.y, b.y}, v.x, v.y);
+                    mma_bf16_16816(acc[i], {a.z, b.z, a.w, b.w}, v.z, v.w);
+                }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&s.empty[slot]));
+            if (++slot == STAGES) {
+                slot = 0;
+                phase ^= 1;
+            }
+        }
+        const int m = static_cast<int>(threadIdx.x) >> 3, f = static_cast<int>(threadIdx.x) & 7;
+        const int n0 = here.tile * (gated ? 8 : 16) + f;
+#pragma unroll
+        for (int i = 0; i < BLOCKS; ++i) {
+            if (GROUPED && i > 0 && here.count <= i * 8) break;
+            // a thread's two tokens are t and t + 4
+            float* part = &s.part[parity][warp][t * kTokenPitch + local];
+            part[0] = acc[i][0];
+            part[4 * kTokenPitch] = acc[i][1];
+            part[8] = acc[i][2];
+            part[4 * kTokenPitch + 8] = acc[i][3];
+            // (two buffers: whoever writes one of them again has passed the barrier in between)
+            asm volatile("bar.sync 1, %0;" ::"n"(kWarps * 32) : "memory");
+            if (threadIdx.x < 64 && i * 8 + m < here.count && n0 < p.n_out) {
+                float v0 = 0.f, v1 = 0.f;
+#pragma unroll
+                for (int w = 0; w < kWarps; ++w) {
+                    v0 += s.part[parity][w][m * kTokenPitch + f];
+                    v1 += s.part[parity][w][m * kTokenPitch + 8 + f];
+                }
+                if (!gated && p.bias != nullptr) {
+                    v0 += __bfloat162float(p.bias[n0]);
+                    if (n0 + 8 < p.n_out) v1 += __bfloat162float(p.bias[n0 + 8]);
+                }
+                store_plain(p, gated, static_cast<int64_t>(here.x_row) + i * 8 + m, n0, n0 + 8, v0, v1);
+            }
+            parity ^= 1;
+        }
+    }
+}
+
+template <bool GROUPED, int BLOCKS>
+__global__ void __launch_bounds__((kWarps + 1) * 32)
+ring_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const RingParams p) {
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ RingShared s;
+    const int warp = static_cast<int>(threadIdx.x) >> 5, lane = static_cast<int>(threadIdx.x) & 31;
+    const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    RingPass* passes = reinterpret_cast<RingPass*>(smem_raw + (ring - smem_u32(smem_raw)) + ring_bytes(BLOCKS));
+
+    pdl_launch_dependents();
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < kStages; ++i) {
+            mbar_init(smem_u32(&s.full[i]), 1);
+            mbar_init(smem_u32(&s.empty[i]), kWarps);
+        }
+        fence_mbar_init();
+        tma_prefetch_desc(&tmap_w);
+        tma_prefetch_desc(&tmap_x);
+    }
+    if (GROUPED) {
+        pdl_wait_prior();   // (the group table comes from the kernel before this one)
+        if (warp == 0) {
+            int most = 0;
+            for (int g = lane; g < p.groups; g += 32) most = max(most, p.counts[g]);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
+            const int width = most > 8 ? 16 : 8;
+            int total = 0;
+            for (int base = 0; base < p.groups; base += 32) {
+                const int g = base + lane;
+                const int rows = g < p.groups ? max(p.counts[g], 0) : 0, n = (rows + width - 1) / width;
+                int incl = n;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int up = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += up;
+                }
+                const int row0 = n > 0 ? p.offsets[g] : 0;
+                for (int i = 0; i < n; ++i) passes[total + incl - n + i] = {g, row0 + i * width, min(rows - i * width, width)};
+                total += __shfl_sync(0xffffffffu, incl, 31);
+            }
+            if (lane == 0) {
+                s.passes = total;
+                s.wide = most > 8;
+            }
+        }
+    }
+    __syncthreads();
+    if (GROUPED && s.wide)
+        ring_walk<true, 2, kWideStages>(tmap_w, tmap_x, p, ring, passes, s, warp, lane);
+    else
+        ring_walk<GROUPED, BLOCKS, kStages>(tmap_w, tmap_x, p, ring, passes, s, warp, lane);
+}
+
+// [rows, K] bf16 as 64-column blocks of rows: boxes of `box_rows` rows x 512 columns under the 128-byte swizzle.
+int make_ring_tmap(CUtensorMap* out, const void* w, int64_t rows, int K, int64_t ld, int box_rows) {
+    struct Entry {
+        const void* w = nullptr;
+        int64_t rows, ld;
+        int K, box_rows;
+        CUtensorMap map;
+    };
+    constexpr int kEntries = 1024;
+    thread_local Entry cache[kEntries];   // (encoding a tensor map costs about a microsecond)
+    Entry& e = cache[(reinterpret_cast<uintptr_t>(w) * 0x9E3779B97F4A7C15ull >> 20) % kEntries];
+    if (e.w != w || e.rows != rows || e.ld != ld || e.K != K || e.box_rows != box_rows) {
+        EncodeTiledFn fn = encode_tiled_fn();
+        if (!fn) {
+            set_last_error("cuTensorMapEncodeTiled is not available from this driver");
+            return B200_ERR_CUDA;
+        }
+        const cuuint64_t dims[3] = {64, static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(K / 64)};
+        const cuuint64_t strides[2] = {static_cast<cuuint64_t>(ld) * 2, 128};
+        const cuuint32_t box[3] = {64, static_cast<cuuint32_t>(box_rows), kChunk / 64};
+        const cuuint32_t es[3] = {1, 1, 1};
+        e.w = nullptr;
+        const CUresult r = fn(&e.map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(w), dims, strides, box, es,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+        if (r != CUDA_SUCCESS) {
+            set_last_error("cuTensorMapEncodeTiled (weight blocks) failed with CUresult %d", static_cast<int>(r));
+            return B200_ERR_CUDA;
+        }
+        e.w = w;
+        e.rows = rows;
+        e.ld = ld;
+        e.K = K;
+        e.box_rows = box_rows;
+    }
+    *out = e.map;
+    return B200_OK;
+}
+
+int launch_ring(RingParams p, const void* x, int64_t x_rows, int64_t ldx, const void* w, int64_t w_rows, bool grouped, cudaStream_t stream) {
+    const bool gated = p.up_row_offset > 0;
+    const int blocks = grouped || p.M <= 8 ? 1 : 2;
+    CUtensorMap tmap_w, tmap_x;
+    p.x_box = grouped ? 8 : p.M;   // (rows that a copy has to fill with zeros cost it: 151936 x 1024 with 1 row 66 us, with 4 rows 52)
+    int err = make_ring_tmap(&tmap_w, w, w_rows, p.K, p.K, gated ? 8 : 16);
+    if (err == B200_OK) err = make_ring_tmap(&tmap_x, x, x_rows, p.K, ldx, p.x_box);
+    if (err != B200_OK) return err;
+    p.tiles = gated ? div_ceil(p.n_out, 8) : div_ceil(p.n_rows, 16);
+    p.chunks = div_ceil(p.K, kChunk);
+    auto kernel = grouped ? ring_gemm_kernel<true, 1> : blocks == 1 ? ring_gemm_kernel<false, 1> : ring_gemm_kernel<false, 2>;
+    const size_t smem = ring_bytes(blocks) + 1024 +
+                        (grouped ? (p.groups + x_rows / 8 + 1) * sizeof(RingPass) : 0);
+    const int grid = grouped || p.tiles > sm_count() ? sm_count() : p.tiles;
+    B200_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    B200_CHECK_CUDA(launch_kernel(kernel, dim3(grid), dim3((kWarps + 1) * 32), smem, stream, dim3(1, 1, 1), tmap_w, tmap_x, p));
+    return B200_OK;
+}
+
+bool aligned16(const void* a, const void* b) { return ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b)) & 15) == 0; }
+
+RingParams ring_params(void* y, int N, int K, int epilogue, float act_limit, int* status) {
+    const bool gated = epilogue_is_gated(epilogue);
+    RingParams p = {};
+    p.y = static_cast<__nv_bfloat16*>(y);
+    p.n_out = gated ? N / 2 : N;
+    p.epilogue = epilogue;
+    p.y_pitch = p.n_out;
+    p.act_limit = act_limit;
+    p.n_rows = N;
+    p.up_row_offset = gated ? N / 2 : 0;
+    p.K = K;
+    p.status = status;
+    return p;
+}
+
+}  // namespace
+
+// Rows of W long and many enough to outlast the start of a walk.  us, this kernel against the ones of gemm_skinny.cu and (the first
+// three lines) gemm_narrow.cu, weights not in L2:
+//   1 x 4096 x 1024 6.2, 5.7;  1 x 8192 x 1024 8.3, 6.3;  16 x 6144 x 1024 with SwiGLU 8.0, 6.2;  1 x 151936 x 1024 51, 48
+//   8 x 4096 x 2048 8.3, 8.2;  1 x 6144 x 2048 8.4, 10.2;  1 x 2048 x 6144 8.3, 10.3;  16 rows of it 10.3, 10.3
+//   16 x 4096 x 2048 8.3, 10.0;  16 x 2048 x 2048 6.2, 6.2;  16 x 1024 x 4096 6.9, 7.1;  16 x 6144 x 2048 10.3, 12.3
+//   8 x 4096 x 4096 10.3, 14.4;  8 x 6144 x 4096 12.6, 20.2;  8 x 4096 x 14336 22.8, 29.4;  16 x 4096 x 14336 24.7, 30.0
+//   8 x 28672 x 4096 with SwiGLU 41.1, 46.4;  9 rows of it 43.2, 46.4;  8 x 128256 x 4096 155, 167
+// Steps: Llama-3-8B, 1 request 2906 us against 3542, 4 requests 3025 against 3726, 8 requests 3097 against 3745; Saluzen, 12 requests 455
+// against 529, 16 requests 490 against 562.
+bool ring_gemm_takes(const void* x, const void* w, int M, int N, int K, int64_t ldx, int epilogue, bool narrow) {
+    const int n_out = epilogue_is_gated(epilogue) ? N / 2 : N;
+    return M <= 16 && K >= 2048 && static_cast<int64_t>(N) * K >= (narrow ? 12ll << 20 : 4ll << 20) && n_out % 8 == 0 && K % 64 == 0 && ldx % 8 == 0 &&
+           aligned16(x, w);
+}
+
+int launch_ring_gemm(void* y, const void* x, const void* w, const void* bias, int M, int N, int K, int64_t ldx, int epilogue, int* status,
+                     cudaStream_t stream, float act_limit) {
+    RingParams p = ring_params(y, N, K, epilogue, act_limit, status);
+    p.bias = static_cast<const __nv_bfloat16*>(bias);
+    p.M = M;
+    return launch_ring(p, x, M, ldx, w, N, false, stream);
+}
+
+// Of the calls that narrow_grouped_takes: many groups, and few enough rows that a group with all of them does not take more turns than
+// there.  Layers (us, this kernel against narrow_grouped_kernel; rows spread at random, and all tokens with the same experts):
+//   64 experts of 2 x 1024 x 2048, 4 per token    1 token 36, 43;   8 tokens 77, 86 and 35, 43;   32: 137, 147 and 52, 58;   48: 149, 166 and 70, 70
+//   128 of 2 x 768 x 2048, 8 per token            1 token 45, 60;   8: 115, 129 and 47, 65;   16: 161, 176 and 60, 67
+//   32 of 2 x 1024 x 2048, 2 per token            8: 49, 57 and 27, 31;   32: 83, 88 and 38, 39;   64: 92, 100, but 51, 49
+//   16 of 2 x 2048 x 1024, 4 per token            1 token 33, 31;   32: 77, 67 and 52, 46
+// Steps of 12 such layers (the first kind): 1 request 581 us against 648, 32 requests 2045 against 2264.
+bool ring_grouped_takes(const void* x, const void* w, int max_rows, int num_groups, int n_out, int K) {
+    return num_groups >= 32 && num_groups <= kMaxRingGroups && max_rows <= 48 && n_out % 8 == 0 && K % 64 == 0 && aligned16(x, w);
+}
+
+int launch_ring_grouped(void* y, const void* x, const void* w, const int32_t* counts, const int32_t* offsets, int num_groups,
+                        int64_t total_rows, int N, int K, int epilogue, int* status, cudaStream_t stream, float act_limit) {
+    RingParams p = ring_params(y, N, K, epilogue, act_limit, status);
+    p.counts = counts;
+    p.offsets = offsets;
+    p.groups = num_groups;
+    return launch_ring(p, x, total_rows, K, w, static_cast<int64_t>(num_groups) * N, true, stream);
+}
+
+}  // namespace b200

@@ -828,8 +828,11 @@ int launch_grouped_gemm(void* y, const void* x, const void* w, const int32_t* co
     const int slabs = div_ceil(max_rows_per_group, 256);
     if (num_groups == 0 || slabs == 0 || total_rows == 0) return B200_OK;
     // A handful of rows per group: weights straight into registers.
-    if (narrow_grouped_takes(x, w, total_rows, max_rows_per_group, num_groups, n_out, K, epilogue))
+    if (narrow_grouped_takes(x, w, total_rows, max_rows_per_group, num_groups, n_out, K, epilogue)) {
+        if (ring_grouped_takes(x, w, max_rows_per_group, num_groups, n_out, K))
+            return launch_ring_grouped(y, x, w, counts, offsets, num_groups, total_rows, N, K, epilogue, status, stream, act_limit);
         return launch_narrow_grouped(y, x, w, counts, offsets, num_groups, N, K, epilogue, stream, act_limit);
+    }
     // Many rows per group on average (prefill batches): tensor-bound, take the tile kernel.
     if (grouped_on_tiles(total_rows, num_groups))
         return launch_grouped_tile_gemm(y, x, w, counts, offsets, num_groups, total_rows, N, K, epilogue, status,
@@ -974,9 +977,13 @@ int gemm_kernel_of(int64_t rows, int N, int K, int epilogue, int groups, int max
 int launch_linear(void* y, const void* x, const void* w, const void* bias, int M, int N, int K,
                   int64_t ldx, int epilogue, int* status, cudaStream_t stream, const SkinnyFusion* fuse,
                   float act_limit, bool narrow) {
-    // A handful of rows: weights straight into registers.
-    if (narrow && fuse == nullptr && narrow_gemm_takes(x, w, M, N, K, ldx, epilogue))
-        return launch_narrow_gemm(y, x, w, bias, M, N, K, ldx, epilogue, status, stream, nullptr, act_limit);
+    // A handful of rows: weights straight into registers, or of a large W through a ring.
+    if (narrow && fuse == nullptr) {
+        const bool registers = narrow_gemm_takes(x, w, M, N, K, ldx, epilogue);
+        if (ring_gemm_takes(x, w, M, N, K, ldx, epilogue, registers))
+            return launch_ring_gemm(y, x, w, bias, M, N, K, ldx, epilogue, status, stream, act_limit);
+        if (registers) return launch_narrow_gemm(y, x, w, bias, M, N, K, ldx, epilogue, status, stream, nullptr, act_limit);
+    }
     // Few rows: stream the weights once (swap-AB, split-K).  Many rows: tensor-bound tiles.
     if (linear_on_tiles(y, M, N, K, epilogue, fuse != nullptr)) {
         if (fuse != nullptr) {

@@ -290,3 +290,42 @@ def test_prefill_at_the_edges_of_tiles(L, seq_lens, extend_lens, page_size, hq, 
     got, want = prefill_attention_case(L, seq_lens, extend_lens, page_size, hq, hkv, seed=sum(seq_lens))
     assert_close_bf16(got, want, 2e-2, 2e-2, "prefill attention")
     assert L.read_device_status() == (0, 0)
+
+
+@pytest.mark.parametrize("M", [1, 5, 8, 9, 13, 16])
+@pytest.mark.parametrize("N,K", [(6664, 2112), (3336, 4160), (1000, 14336), (28672, 512)])
+def test_linear_of_few_rows_of_a_large_w(L, pkg, M, N, K):
+    """The ring kernel (the last shape: its neighbours): a last tile of 8 features, K that ends inside a stage of 512, fewer tiles than
+    SMs, one and two blocks of tokens."""
+    lib = pkg.load_library()
+    assert lib.b200_gemm_kernel(M, N, K, pkg.EPILOGUE_NONE, 0, 0, 0) == (STREAM if K > 2048 or M > 8 else NARROW)
+    gen = torch.Generator().manual_seed(M + N + K)
+    buf, w, b = randn_bf16(gen, M, K + 64), randn_bf16(gen, N, K, std=0.05), randn_bf16(gen, N)
+    atol = BIG[0] * (K / 1024) ** 0.5 + BIG[1]
+    x = buf[:, 64:]
+    assert_close_bf16(L.linear(buf.cuda()[:, 64:], w.cuda(), b.cuda()), O.linear(x, w, b), 2 * atol, RTOL, "bias, strided rows")
+    if N % 16 == 0:
+        y = L.linear(x.contiguous().cuda(), w.cuda(), epilogue=pkg.EPILOGUE_SWIGLU)
+        assert_close_bf16(y, O.silu_and_mul(O.linear(x, w)), 2 * atol, 3 * RTOL, "SwiGLU")
+    assert L.read_device_status() == (0, 0)
+
+
+@pytest.mark.parametrize("T", [1, 8, 9, 17, 40])
+@pytest.mark.parametrize("E,k,H,I", [(33, 4, 192, 576), (64, 3, 576, 64), (256, 1, 64, 128)])
+@pytest.mark.parametrize("alike", [False, True])
+def test_many_experts_of_few_rows(L, pkg, T, E, k, H, I, alike):
+    """The ring kernel's experts: rows of an expert below, at and above the 8 and 16 of one pass, K within a stage and beyond."""
+    lib = pkg.load_library()
+    assert lib.b200_gemm_kernel(T * k, 2 * I, H, pkg.EPILOGUE_SWIGLU, E, T, 0) == NARROW
+    gen = torch.Generator().manual_seed(T + E + H)
+    hidden = randn_bf16(gen, T, H)
+    logits = torch.randn(T, E, generator=gen).argsort(1).to(torch.bfloat16) / 32   # distinct in every row
+    if alike:
+        logits[:] = logits[0]
+    moe = L.MoELayer(E, k, H, I, True, "silu")
+    gu, dn = randn_bf16(gen, E, 2 * I, H, std=H ** -0.5), randn_bf16(gen, E, H, I, std=I ** -0.5)
+    moe.gate_up_proj.copy_(gu.cuda())
+    moe.down_proj.copy_(dn.cuda())
+    assert_close_bf16(moe.forward(hidden.cuda(), logits.cuda()), O.moe_forward(hidden, logits, gu, dn, k, True, "silu", O.store_bf16),
+                      2e-2, 4 * 2 ** -7, "experts")
+    assert L.read_device_status() == (0, 0)
