@@ -49,17 +49,25 @@ rmsnorm_kernel(__nv_bfloat16* out, const __nv_bfloat16* x_in,
     }
     pdl_wait_prior();
 
+    // (all loads of the row before the first store of the sum: one trip to L2 for them, not one per vector)
+    uint4 x[kNormVecPerThread], r[kNormVecPerThread];
+#pragma unroll
+    for (int i = 0; i < kNormVecPerThread; ++i) {
+        const int v = threadIdx.x + i * blockDim.x;
+        if (v < nvec) {
+            x[i] = xv[v];
+            if (FUSED_ADD) r[i] = rv[v];
+        }
+    }
     float vals[kNormVecPerThread][8];
     float ss = 0.f;
 #pragma unroll
     for (int i = 0; i < kNormVecPerThread; ++i) {
         const int v = threadIdx.x + i * blockDim.x;
         if (v < nvec) {
-            uint4 a = xv[v];
-            const uint32_t aw[4] = {a.x, a.y, a.z, a.w};
+            const uint32_t aw[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
             if (FUSED_ADD) {
-                uint4 r = rv[v];
-                const uint32_t rw[4] = {r.x, r.y, r.z, r.w};
+                const uint32_t rw[4] = {r[i].x, r[i].y, r[i].z, r[i].w};
                 uint32_t packed[4];
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
