@@ -16,13 +16,13 @@ constexpr int kMaxExpertsPerLane = 8;  // num_experts <= 256
 constexpr int kMaxTopK = 16;
 constexpr int kRouteInOneCta = 64;     // tokens whose choices and rows one CTA finds (two per warp)
 
-// Softmax and top-k of one token's router logits by a warp; `put(k, expert, weight)` runs on lane 0.
-template <typename Put>
+// Softmax and top-k of one token's router logits by a warp, PER experts per lane; `put(k, expert, weight)` runs on lane k.
+template <int PER, typename Put>
 __device__ __forceinline__ void route_token(const __nv_bfloat16* __restrict__ row, int E, int top_k, int renorm, int lane, Put put) {
-    float v[kMaxExpertsPerLane];
+    float v[PER];
     float mx = -INFINITY;
 #pragma unroll
-    for (int i = 0; i < kMaxExpertsPerLane; ++i) {
+    for (int i = 0; i < PER; ++i) {
         const int e = lane + i * 32;
         v[i] = e < E ? __bfloat162float(row[e]) : -INFINITY;
         mx = fmaxf(mx, v[i]);
@@ -30,21 +30,20 @@ __device__ __forceinline__ void route_token(const __nv_bfloat16* __restrict__ ro
     mx = warp_max(mx);
     float sum = 0.f;
 #pragma unroll
-    for (int i = 0; i < kMaxExpertsPerLane; ++i) {
+    for (int i = 0; i < PER; ++i) {
         v[i] = (lane + i * 32) < E ? __expf(v[i] - mx) : -1.f;  // -1 marks "not a candidate"
         if (v[i] > 0.f) sum += v[i];
     }
     sum = warp_sum(sum);
     const float inv = 1.f / sum;
-    float wsel[kMaxTopK];
-    int isel[kMaxTopK];
-    float wsum = 0.f;
+    float mine = 0.f, wsum = 0.f;   // (lane k keeps the k-th choice)
+    int expert = 0;
     for (int k = 0; k < top_k; ++k) {
         // Largest remaining probability; the lower expert index wins ties.
         float best = -1.f;
         int bi = 0x7fffffff;
 #pragma unroll
-        for (int i = 0; i < kMaxExpertsPerLane; ++i)
+        for (int i = 0; i < PER; ++i)
             if (v[i] > best) {
                 best = v[i];
                 bi = lane + i * 32;
@@ -59,18 +58,24 @@ __device__ __forceinline__ void route_token(const __nv_bfloat16* __restrict__ ro
             }
         }
         if (bi >= E) bi = k;   // NaN logits: a token's experts are valid and differ all the same
-        if ((bi & 31) == lane) v[bi >> 5] = -1.f;
-        wsel[k] = best * inv;
-        isel[k] = bi;
-        wsum += wsel[k];
-    }
-    if (lane == 0) {
-        for (int k = 0; k < top_k; ++k) {
-            float w = wsel[k];
-            if (renorm) w = w / (wsum + 1e-8f);
-            put(k, isel[k], round_bf16(w));  // the reference casts the weights to bf16
+#pragma unroll
+        for (int i = 0; i < PER; ++i)
+            if (bi == lane + i * 32) v[i] = -1.f;
+        if (lane == k) {
+            mine = best * inv;
+            expert = bi;
         }
+        wsum += best * inv;
     }
+    if (lane < top_k) put(lane, expert, round_bf16(renorm ? mine / (wsum + 1e-8f) : mine));  // the reference casts the weights to bf16
+}
+
+// The same for any number of experts: up to 64, 128 and kMaxExpertsPerLane * 32 in code of their own.
+template <typename Put>
+__device__ __forceinline__ void route_token(const __nv_bfloat16* __restrict__ row, int E, int top_k, int renorm, int lane, Put put) {
+    if (E <= 64) route_token<2>(row, E, top_k, renorm, lane, put);
+    else if (E <= 128) route_token<4>(row, E, top_k, renorm, lane, put);
+    else route_token<kMaxExpertsPerLane>(row, E, top_k, renorm, lane, put);
 }
 
 // One warp per token.  COUNT: the expert histogram too (`counts` zero before).
@@ -121,7 +126,19 @@ moe_place_kernel(const PlaceArgs a) {
                 a.rows[t * a.top + k] = atomicAdd(&s_count[e], 1);
             });
     } else {
-        for (int i = threadIdx.x; i < pairs; i += blockDim.x) a.rows[i] = atomicAdd(&s_count[a.ids[i]], 1);
+        for (int i0 = threadIdx.x; i0 < pairs; i0 += 4 * blockDim.x) {   // (four trips to L2 at once)
+            int e[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int i = i0 + j * static_cast<int>(blockDim.x);
+                e[j] = i < pairs ? a.ids[i] : 0;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int i = i0 + j * static_cast<int>(blockDim.x);
+                if (i < pairs) a.rows[i] = atomicAdd(&s_count[e[j]], 1);
+            }
+        }
     }
     __syncthreads();
     if (warp == 0) {   // eight neighbouring experts per lane
@@ -152,15 +169,24 @@ moe_place_kernel(const PlaceArgs a) {
     }
     if (ROUTE) {
         for (int t = warp; t < a.tokens; t += blockDim.x >> 5)
-            if (lane == 0)
-                for (int i = t * a.top; i < (t + 1) * a.top; ++i) {
-                    const int first = s_first[a.ids[i]];
-                    a.rows[i] = first < 0 ? -1 : first + a.rows[i];
-                }
+            if (lane < a.top) {
+                const int i = t * a.top + lane, first = s_first[a.ids[i]];
+                a.rows[i] = first < 0 ? -1 : first + a.rows[i];
+            }
     } else {
-        for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
-            const int first = s_first[a.ids[i]];
-            a.rows[i] = first < 0 ? -1 : first + a.rows[i];
+        for (int i0 = threadIdx.x; i0 < pairs; i0 += 4 * blockDim.x) {
+            int e[4], row[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int i = i0 + j * static_cast<int>(blockDim.x);
+                e[j] = i < pairs ? a.ids[i] : 0;
+                row[j] = i < pairs ? a.rows[i] : 0;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int i = i0 + j * static_cast<int>(blockDim.x), first = s_first[e[j]];
+                if (i < pairs) a.rows[i] = first < 0 ? -1 : first + row[j];
+            }
         }
     }
 }
