@@ -32,10 +32,6 @@ namespace {
 
 constexpr int kSteps = 4;        // k-steps of 32 per register buffer
 constexpr int kHeadRanks = 8;    // CTAs that share an attention head
-// From this K on a warp walks much of its share of K behind the wait, and CTAs of the next kernels, let in early, only take
-// bandwidth from it (2048 x 6144 in a decode step of 16 requests: 568 us per step without, 585 with; 1024 x 3072, most of which
-// is requested ahead, the other way round: 723 us per step with, 770 without).
-constexpr int kWalkedK = 4096;
 enum Kind { kPlain, kResidual, kHeads };
 
 struct NarrowParams : NarrowOut {

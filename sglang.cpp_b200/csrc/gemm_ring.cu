@@ -46,6 +46,7 @@ struct RingParams : NarrowOut {
     const __nv_bfloat16* bias;
     int M, n_rows, up_row_offset, tiles, chunks, K;
     int x_box;        // rows of x per copy
+    int early;        // let the next kernel's CTAs in at once
     int* status;
     const int32_t *counts, *offsets;   // GROUPED
     int groups;
@@ -218,7 +219,7 @@ ring_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     const uint32_t ring = (smem_u32(smem_raw) + 1023u) & ~1023u;
     RingPass* passes = reinterpret_cast<RingPass*>(smem_raw + (ring - smem_u32(smem_raw)) + ring_bytes(BLOCKS));
 
-    pdl_launch_dependents();
+    if (p.early) pdl_launch_dependents();
     if (threadIdx.x == 0) {
         for (int i = 0; i < kStages; ++i) {
             mbar_init(smem_u32(&s.full[i]), 1);
@@ -331,6 +332,7 @@ RingParams ring_params(void* y, int N, int K, int epilogue, float act_limit, int
     p.epilogue = epilogue;
     p.y_pitch = p.n_out;
     p.act_limit = act_limit;
+    p.early = 1;
     p.n_rows = N;
     p.up_row_offset = gated ? N / 2 : 0;
     p.K = K;
@@ -347,8 +349,8 @@ RingParams ring_params(void* y, int N, int K, int epilogue, float act_limit, int
 //   16 x 4096 x 2048 8.3, 10.0;  16 x 2048 x 2048 6.2, 6.2;  16 x 1024 x 4096 6.9, 7.1;  16 x 6144 x 2048 10.3, 12.3
 //   8 x 4096 x 4096 10.3, 14.4;  8 x 6144 x 4096 12.6, 20.2;  8 x 4096 x 14336 22.8, 29.4;  16 x 4096 x 14336 24.7, 30.0
 //   8 x 28672 x 4096 with SwiGLU 41.1, 46.4;  9 rows of it 43.2, 46.4;  8 x 128256 x 4096 155, 167
-// Steps: Llama-3-8B, 1 request 2906 us against 3542, 4 requests 3025 against 3726, 8 requests 3097 against 3745; Saluzen, 12 requests 455
-// against 529, 16 requests 490 against 562.
+// Steps: Llama-3-8B, 1 request 2906 us against 3542, 4 requests 3025 against 3726, 8 requests 3097 against 3745; Saluzen, 12 requests 470
+// against 566, 16 requests 498 against 594.
 bool ring_gemm_takes(const void* x, const void* w, int M, int N, int K, int64_t ldx, int epilogue, bool narrow) {
     const int n_out = epilogue_is_gated(epilogue) ? N / 2 : N;
     return M <= 16 && K >= 2048 && static_cast<int64_t>(N) * K >= (narrow ? 12ll << 20 : 4ll << 20) && n_out % 8 == 0 && K % 64 == 0 && ldx % 8 == 0 &&
@@ -356,10 +358,15 @@ bool ring_gemm_takes(const void* x, const void* w, int M, int N, int K, int64_t 
 }
 
 int launch_ring_gemm(void* y, const void* x, const void* w, const void* bias, int M, int N, int K, int64_t ldx, int epilogue, int* status,
-                     cudaStream_t stream, float act_limit) {
+                     cudaStream_t stream, float act_limit, bool narrow) {
     RingParams p = ring_params(y, N, K, epilogue, act_limit, status);
     p.bias = static_cast<const __nv_bfloat16*>(bias);
     p.M = M;
+    // Where the registers' kernel would take the call, the next kernels are let in as that one lets them in.  2048 x 6144 with 16 rows
+    // at the end of a layer, the norm, the latents' projection and their norm let in at once: logits 0.03 to 0.08 from those of
+    // 64 bits in place of 0.0087 (the same with the fences of acquiring loads behind every wait; exact once one kernel of the four
+    // triggers behind its own wait), and no faster: 501 us per step against 498.
+    p.early = !narrow || K < kWalkedK;
     return launch_ring(p, x, M, ldx, w, N, false, stream);
 }
 

@@ -981,7 +981,7 @@ int launch_linear(void* y, const void* x, const void* w, const void* bias, int M
     if (narrow && fuse == nullptr) {
         const bool registers = narrow_gemm_takes(x, w, M, N, K, ldx, epilogue);
         if (ring_gemm_takes(x, w, M, N, K, ldx, epilogue, registers))
-            return launch_ring_gemm(y, x, w, bias, M, N, K, ldx, epilogue, status, stream, act_limit);
+            return launch_ring_gemm(y, x, w, bias, M, N, K, ldx, epilogue, status, stream, act_limit, registers);
         if (registers) return launch_narrow_gemm(y, x, w, bias, M, N, K, ldx, epilogue, status, stream, nullptr, act_limit);
     }
     // Few rows: stream the weights once (swap-AB, split-K).  Many rows: tensor-bound tiles.

@@ -132,7 +132,7 @@ int launch_narrow_grouped(void* y, const void* x, const void* w, const int32_t* 
 // `narrow`: narrow_gemm_takes the call.
 bool ring_gemm_takes(const void* x, const void* w, int M, int N, int K, int64_t ldx, int epilogue, bool narrow);
 int launch_ring_gemm(void* y, const void* x, const void* w, const void* bias, int M, int N, int K, int64_t ldx, int epilogue, int* status,
-                     cudaStream_t stream, float act_limit);
+                     cudaStream_t stream, float act_limit, bool narrow);
 bool ring_grouped_takes(const void* x, const void* w, int max_rows, int num_groups, int n_out, int K);
 int launch_ring_grouped(void* y, const void* x, const void* w, const int32_t* counts, const int32_t* offsets, int num_groups,
                         int64_t total_rows, int N, int K, int epilogue, int* status, cudaStream_t stream, float act_limit);

@@ -6,6 +6,10 @@
 
 namespace b200 {
 
+// From this K on a warp walks much of its share of K behind the wait, and CTAs of the next kernels, let in early, only take
+// bandwidth from it (2048 x 6144 in a decode step of 16 requests: 568 us per step without, 585 with; 1024 x 3072, most of which
+// is requested ahead, the other way round: 723 us per step with, 770 without).
+constexpr int kWalkedK = 4096;
 constexpr int kTokenPitch = 20;  // floats: 16 features of a token, padded so that a warp's stores hit 32 banks
 
 struct NarrowOut {

@@ -339,3 +339,27 @@ def test_generate_command(pkg, tmp_path):
                        timeout=250, env=dict(os.environ))
     assert r.returncode == 0, r.stderr[-2000:]
     assert [[int(t) for t in x.split()] for x in r.stdout.splitlines()] == [greedy("mixed", p, 5) for p in prompts]
+
+
+@pytest.mark.parametrize("requests", [8, 9, 16])
+def test_steps_whose_kernels_start_early_have_the_bits_of_steps_whose_kernels_do_not(pkg, monkeypatch, requests):
+    """Layers wide enough for the GEMMs that walk over a large W, of one and two blocks of 8 rows, behind the latents' chain of
+    small kernels."""
+    cfg = C.config([C.latent(16, 64, 64, 128, 768, 512, 0.0884, ff=6144), C.latent(16, 64, 64, 128, 768, 512, 0.0884, kv_from=0, ff=6144)],
+                   width=2048, vocab=512)
+    if "chained" not in C._models:
+        C._models["chained"] = C.O.random_model(cfg, 5)
+    prompts = [C.prompt(cfg, 70 + i, 40 + i) for i in range(requests)]
+    got = []
+    for early in ("0", "1"):
+        monkeypatch.setenv("B200_PDL", early)
+        e, hb = engine_for(cfg, C._models["chained"], "bfloat16", pages=2 * requests, live=requests, max_extend=2048)
+        e.capture_graphs([requests])
+        live = [hb.open_request(100) for _ in prompts]
+        hb.extend(live, prompts).synchronize()
+        steps = []
+        for step in range(6):
+            hb.extend(live, [[int(p[step])] for p in prompts]).synchronize()
+            steps.append(e.token_logits(range(requests)))
+        got.append(torch.stack(steps))
+    assert torch.equal(got[0], got[1])
