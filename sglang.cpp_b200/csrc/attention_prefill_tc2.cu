@@ -15,9 +15,16 @@
 // rare occasions the row's O is rescaled in TMEM by the threads that own the row.  Nothing else touches
 // O until the end, so the softmax threads carry no accumulator and no P tile goes through shared memory.
 //
-// Roles: warps 0 and 2 fetch K and V tiles (in turn through one TMA ring of five slots), one thread of warp 1 issues the
-// products S, one of warp 3 the products P V, warps 4-7 softmax of tile 0, warps 8-11 softmax of tile 1 (thread = TMEM lane).
+// Roles: warp 0 fetches K tiles, warp 2 V tiles, one thread of warp 1 issues the products S, one of warp 3 the products P V,
+// warps 4-7 softmax of tile 0, warps 8-11 softmax of tile 1 (thread = TMEM lane).
 // A row's scores fit its thread's registers: S is read once and the row's maximum needs no exchange.
+//
+// K and V tiles have a ring of slots each.  A slot's barriers are tested by parity, which tells a phase from the one before it
+// and from no other: whoever tests one has to know that the phase before is over.  With a ring per kind it does.  The producer of
+// a ring waits for the release of the slot's last tile, which it has copied there itself, behind the release of the tile before
+// that one; the issuer waits for a tile behind the slot's last one, which it has multiplied.  (Both kinds in turn through one ring of
+// five slots: V tile j + 5 waits for the release of K tile j + 3, and nothing that its producer has seen tells it that V tile
+// j, in the same slot before, has been multiplied with the second query tile; neither does the issuer of S know that it has arrived.)
 //
 // What bounds it: 2048 cycles of products and 2048 of exponentials (16 per cycle and SM) per K/V tile; 2900 are taken, the
 // rest of a row's softmax (scores, maximum, waits: 900 cycles) being hidden only in part.  Both kinds of products from one
@@ -55,9 +62,9 @@ constexpr int kIssueRegs = 72, kSoftmaxRegs = 216;
 static_assert(128 * (kIssueRegs + 2 * kSoftmaxRegs) <= kThreads * 168, "");
 constexpr uint32_t kAtomBytes = 128 * 128;  // 128 rows x 64 bf16: one swizzle atom column
 constexpr uint32_t kQOff = 0;               // Q: 2 tiles x 2 atoms (d 0-63, d 64-127)
-constexpr uint32_t kKVOff = 4 * kAtomBytes; // ring of K and V tiles in turn, in groups of 8 keys (KvMaps)
+constexpr uint32_t kKVOff = 4 * kAtomBytes; // K tiles, then V tiles, in groups of 8 keys (KvMaps)
 constexpr uint32_t kSlotBytes = 2 * kAtomBytes;
-constexpr int kSlots = 5;
+constexpr int kKSlots = 2, kVSlots = 3, kSlots = kKSlots + kVSlots;   // a ring of tiles each
 constexpr uint32_t kSmemBytes = kKVOff + kSlots * kSlotBytes;
 constexpr uint32_t kColS = 0, kColP = 128, kColO = 256;  // TMEM columns: S (128), P0, P1 (64 each), O0, O1 (128 each)
 constexpr float kLazyLog2 = 8.0f;           // the reference maximum moves when the true one is 2^8 ahead
@@ -112,7 +119,7 @@ template <bool WINDOW>
 __global__ void __launch_bounds__(kThreads, 1)
 attention_prefill_tc2_kernel(const __grid_constant__ KvMaps maps, const PrefillTc2Params p) {
     extern __shared__ uint8_t smem_raw[];
-    __shared__ __align__(8) uint64_t full[kSlots];    // K tile kt is item 2 kt of the ring, V tile kt item 2 kt + 1
+    __shared__ __align__(8) uint64_t full[kSlots];    // slots of K tiles, then of V tiles
     __shared__ __align__(8) uint64_t empty[kSlots];
     __shared__ __align__(8) uint64_t s_full[2];    // per query tile: S of the current K/V tile is in TMEM
     __shared__ __align__(8) uint64_t s_free[2];    // ... and has been read from there (4 warp arrivals)
@@ -184,7 +191,7 @@ attention_prefill_tc2_kernel(const __grid_constant__ KvMaps maps, const PrefillT
             next[i] = copy < n ? pt_row[k0 + copy * p.kpc] : 0;
         }
     };
-    // K (kv = 0) or V tile kt into `slot` of the ring.  A tile whose pages are consecutive slots is fetched with one copy; so
+    // K (kv = 0) or V tile kt into `slot`.  A tile whose pages are consecutive slots is fetched with one copy; so
     // is a page, unless it is smaller than a group or starts inside one.
     auto load_tile = [&](int kv, int kt, uint32_t slot) {
         const int ncopies = copies_of(kt);
@@ -240,9 +247,9 @@ attention_prefill_tc2_kernel(const __grid_constant__ KvMaps maps, const PrefillT
 
     // Rows of V that no copy ever writes (behind the last key, in a slot that had no tile before) must not hold NaN
     // patterns: their probabilities are 0.
-    if (2 * ntiles <= kSlots) {
+    if (ntiles <= kVSlots) {
         const int written = (kv_end - first_key(ntiles - 1) + p.kpc - 1) / p.kpc * p.kpc;
-        uint4* z = reinterpret_cast<uint4*>(smem_gen + kKVOff + (2 * ntiles - 1) * kSlotBytes);
+        uint4* z = reinterpret_cast<uint4*>(smem_gen + kKVOff + (kKSlots + ntiles - 1) * kSlotBytes);
         for (int i = threadIdx.x; i < max(0, kTile - written) * 16; i += kThreads) {
             const int key = written + (i >> 4), at = i & 15;   // 16 bytes of a key's row
             z[(key >> 3) * 128 + (at >> 3) * 64 + (key & 7) * 8 + (at & 7)] = make_uint4(0, 0, 0, 0);
@@ -287,14 +294,14 @@ attention_prefill_tc2_kernel(const __grid_constant__ KvMaps maps, const PrefillT
     if (warp == 0 || warp == 2) {
         // ================= producers: K tiles, V tiles =================
         const int kv = warp >> 1;
-        uint32_t slot = kv == 0 ? 2 : 1, phase = 1;   // (the first waits are for slots that nobody has used)
+        const uint32_t ring = kv == 0 ? 0 : kKSlots, ring_end = kv == 0 ? kKSlots : kSlots;
+        uint32_t slot = kv == 0 ? 1 : kKSlots, phase = 1;   // (the first waits are for slots that nobody has used)
         for (int kt = kv == 0 ? 1 : 0; kt < ntiles; ++kt) {
             if (!mbar_wait_mostly_ready(smem_u32(&empty[slot]), phase, p.status, 321)) break;
             load_tile(kv, kt, slot);
             if (kt + 1 < ntiles) fetch_slots(kt + 1);
-            slot += 2;
-            if (slot >= kSlots) {
-                slot -= kSlots;
+            if (++slot == ring_end) {
+                slot = ring;
                 phase ^= 1;
             }
         }
@@ -328,9 +335,8 @@ attention_prefill_tc2_kernel(const __grid_constant__ KvMaps maps, const PrefillT
                 }
                 if (failed) break;
                 tc_commit(smem_u32(&empty[slot]));   // both tiles have read this K tile
-                slot += 2;
-                if (slot >= kSlots) {
-                    slot -= kSlots;
+                if (++slot == kKSlots) {
+                    slot = 0;
                     phase ^= 1;
                 }
             }
@@ -340,7 +346,7 @@ attention_prefill_tc2_kernel(const __grid_constant__ KvMaps maps, const PrefillT
         if (elect_one()) {
             const uint32_t idesc = idesc_bf16_128x128(true);
             const uint64_t v_desc = grouped_keys_desc(smem_base + kKVOff, 1024);   // second half of the head dimension 1024 bytes on
-            uint32_t slot = 1, phase = 0;
+            uint32_t slot = kKSlots, phase = 0;
             bool failed = false;
             auto wait = [&](uint32_t bar, uint32_t parity, int site) {
                 if (!failed && !mbar_wait_mostly_ready(bar, parity, p.status, site)) failed = true;
@@ -363,9 +369,8 @@ attention_prefill_tc2_kernel(const __grid_constant__ KvMaps maps, const PrefillT
                 }
                 if (failed) break;
                 tc_commit(smem_u32(&empty[slot]));   // both tiles have read this V tile
-                slot += 2;
-                if (slot >= kSlots) {
-                    slot -= kSlots;
+                if (++slot == kSlots) {
+                    slot = kKSlots;
                     phase ^= 1;
                 }
             }
