@@ -405,8 +405,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k,
                         }
                     }
                 }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&empty_bar[slot]));
+                mbar_release_stage(smem_u32(&empty_bar[slot]), lane);
             }
             l0 += __shfl_xor_sync(0xffffffffu, l0, 1);
             l0 += __shfl_xor_sync(0xffffffffu, l0, 2);
@@ -540,8 +539,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k,
                     }
                 }
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&empty_bar[slot]));
+            mbar_release_stage(smem_u32(&empty_bar[slot]), lane);
         }
 
         // The next item's queries are requested now, so their latency hides behind this

@@ -249,8 +249,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tmap_k,
                 }
             }
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&empty_bar[slot]));
+        mbar_release_stage(smem_u32(&empty_bar[slot]), lane);
     }
 
     l0 += __shfl_xor_sync(0xffffffffu, l0, 1);

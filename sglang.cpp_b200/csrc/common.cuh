@@ -185,6 +185,16 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
+// A warp hands a stage back that copies fill and that its lanes have read with ordinary loads.  The arrival alone orders these
+// loads before what other threads do, but not before the next copy, which goes another way to shared memory: without the fence a
+// load that waits in line behind a neighbour CTA's can find the next copy's bytes (experts of a decode step with one request, the
+// following kernels' CTAs beginning to load on the same SM: one step in three had a tile of wrong sums).
+__device__ __forceinline__ void mbar_release_stage(uint32_t bar, int lane) {
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar);
+}
+
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                  : "memory");

@@ -172,8 +172,7 @@ __device__ __forceinline__ void ring_walk(const CUtensorMap& tmap_w, const CUten
                     mma_bf16_16816(acc[i], {a.z, b.z, a.w, b.w}, v.z, v.w);
                 }
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&s.empty[slot]));
+            mbar_release_stage(smem_u32(&s.empty[slot]), lane);
             if (++slot == STAGES) {
                 slot = 0;
                 phase ^= 1;
@@ -362,10 +361,8 @@ int launch_ring_gemm(void* y, const void* x, const void* w, const void* bias, in
     RingParams p = ring_params(y, N, K, epilogue, act_limit, status);
     p.bias = static_cast<const __nv_bfloat16*>(bias);
     p.M = M;
-    // Where the registers' kernel would take the call, the next kernels are let in as that one lets them in.  2048 x 6144 with 16 rows
-    // at the end of a layer, the norm, the latents' projection and their norm let in at once: logits 0.03 to 0.08 from those of
-    // 64 bits in place of 0.0087 (the same with the fences of acquiring loads behind every wait; exact once one kernel of the four
-    // triggers behind its own wait), and no faster: 501 us per step against 498.
+    // Where the registers' kernel would take the call, the next kernels are let in as that one lets them in: 2048 x 6144 with 16 rows
+    // at the end of a layer is no faster with them let in at once, 501 us per step against 498.
     p.early = !narrow || K < kWalkedK;
     return launch_ring(p, x, M, ldx, w, N, false, stream);
 }

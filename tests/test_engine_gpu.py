@@ -703,3 +703,52 @@ def test_tokens_into_pinned_and_pageable_memory_and_reports_of_steps(pkg, nreq):
     e.write_token_pool(rows[:1], [0], good)
     e.forward_batch(0, rows, zeros, lens, none).synchronize()
     e.close()
+
+
+@pytest.mark.parametrize("nreq,cached", [(1, 60), (1, 300), (2, 200), (4, 90)])
+def test_decode_of_wide_experts_repeats_itself(pkg, monkeypatch, nreq, cached):
+    """Experts whose weights stream through a ring while the CTAs of the next kernels begin to load on the same SMs: a stage is not
+    filled again before every warp has its part of it in registers.  The same step many times over, against kernels one by one."""
+    from sglang_cpp_b200.engine import Engine, EngineConfig
+    from sglang_cpp_b200.models import ModelConfig
+
+    cfg = ModelConfig(2, 2048, 16, 4, 128, 1024, 1024, 1e-6, 1e6, 512, False, True, True, "silu", 64, 4, 1024)
+    sizes = {"qkv": (3072, 2048), "o": (2048, 2048), "router": (64, 2048), "experts_gate_up": (64 * 2048, 2048),
+             "experts_down": (64 * 2048, 1024), "lm_head": (1024, 2048), "embed": (1024, 2048)}
+
+    class Owned:
+        def __init__(self, e, name, layer):
+            at, nbytes = e.tensor_info(name, layer)
+            self.__cuda_array_interface__ = {"shape": (nbytes,), "typestr": "|u1", "data": (at, False), "version": 3, "strides": None}
+
+    got = []
+    for early in ("0", "1"):
+        monkeypatch.setenv("B200_PDL", early)
+        e = Engine(cfg, EngineConfig(16, 32 * nreq + 1, nreq, 512, 512))
+
+        def view(name, layer=0):
+            return torch.as_tensor(Owned(e, name, layer), device="cuda").view(torch.bfloat16)
+
+        gen = torch.Generator(device="cuda").manual_seed(7)
+        for layer in range(2):
+            for name in ("qkv", "o", "router", "experts_gate_up", "experts_down"):
+                view(name, layer).normal_(0.0, sizes[name][1] ** -0.5, generator=gen)
+            for name in ("input_norm", "post_norm", "q_norm", "k_norm"):
+                view(name, layer).fill_(1.0)
+        for name in ("embed", "lm_head", "kv_cache"):
+            view(name).normal_(0.0, 1.0, generator=gen)
+        view("final_norm").fill_(0.05)
+        torch.cuda.synchronize()
+        rows, at = np.arange(nreq, dtype=np.int32), np.arange(cached + 1, dtype=np.int32)
+        for r in rows:
+            e.write_page_table(np.full(cached + 1, r, np.int32), at, (r * 512 + at).astype(np.int32))
+        e.write_token_pool(rows, np.full(nreq, cached, np.int32), rows + 5)
+        e.capture_graphs([nreq])
+        steps = []
+        for _ in range(2 if early == "0" else 60):
+            e.forward_batch(1, rows, np.full(nreq, cached, np.int32), np.ones(nreq, np.int32), np.full(nreq, -1, np.int32)).synchronize()
+            steps.append(view("logits")[:nreq * 1024].clone())
+        got.append(steps)
+        e.close()
+    wrong = [i for i, s in enumerate(got[1]) if not torch.equal(s, got[0][0])]
+    assert torch.equal(*got[0]) and torch.isfinite(got[0][0]).all() and wrong == []

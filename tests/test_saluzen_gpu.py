@@ -341,19 +341,20 @@ def test_generate_command(pkg, tmp_path):
     assert [[int(t) for t in x.split()] for x in r.stdout.splitlines()] == [greedy("mixed", p, 5) for p in prompts]
 
 
-@pytest.mark.parametrize("requests", [8, 9, 16])
-def test_steps_whose_kernels_start_early_have_the_bits_of_steps_whose_kernels_do_not(pkg, monkeypatch, requests):
+@pytest.mark.parametrize("requests", [1, 8, 9, 16])
+@pytest.mark.parametrize("ff", [6144, 8192])
+def test_steps_whose_kernels_start_early_have_the_bits_of_steps_whose_kernels_do_not(pkg, monkeypatch, requests, ff):
     """Layers wide enough for the GEMMs that walk over a large W, of one and two blocks of 8 rows, behind the latents' chain of
-    small kernels."""
-    cfg = C.config([C.latent(16, 64, 64, 128, 768, 512, 0.0884, ff=6144), C.latent(16, 64, 64, 128, 768, 512, 0.0884, kv_from=0, ff=6144)],
+    small kernels.  (6144: the last of a layer lets the next kernels in when it ends; 8192: at once.)"""
+    cfg = C.config([C.latent(16, 64, 64, 128, 768, 512, 0.0884, ff=ff), C.latent(16, 64, 64, 128, 768, 512, 0.0884, kv_from=0, ff=ff)],
                    width=2048, vocab=512)
-    if "chained" not in C._models:
-        C._models["chained"] = C.O.random_model(cfg, 5)
+    if f"chained{ff}" not in C._models:
+        C._models[f"chained{ff}"] = C.O.random_model(cfg, 5)
     prompts = [C.prompt(cfg, 70 + i, 40 + i) for i in range(requests)]
     got = []
     for early in ("0", "1"):
         monkeypatch.setenv("B200_PDL", early)
-        e, hb = engine_for(cfg, C._models["chained"], "bfloat16", pages=2 * requests, live=requests, max_extend=2048)
+        e, hb = engine_for(cfg, C._models[f"chained{ff}"], "bfloat16", pages=2 * requests, live=requests, max_extend=2048)
         e.capture_graphs([requests])
         live = [hb.open_request(100) for _ in prompts]
         hb.extend(live, prompts).synchronize()
