@@ -539,6 +539,7 @@ attention_prefill_tc2_kernel(const __grid_constant__ KvMaps maps, const PrefillT
             }
             // Through the query tile's place in shared memory (its last product is done), so that half a warp writes a row.
             const bool ok = __all_sync(0xffffffffu, !failed);
+            __syncwarp();   // (a vote orders no memory)
             const int64_t out_st = WINDOW ? p.w.out_st : static_cast<int64_t>(p.q_heads) * kD;
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
