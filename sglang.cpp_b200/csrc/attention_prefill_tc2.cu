@@ -81,6 +81,7 @@ struct PrefillTc2Params {
     int q_heads, kv_heads, group, batch;
     int blocks;              // of 2 x 128/G query tokens in the longest extension
     int kpc;  // keys of a page in a tile = min(page_size, 128)
+    int whole_pages;       // KvMaps::page is there: pages and a cache of 8 slots and more (the map counts groups of 8)
     int whole_tile_boxes;  // KvMaps::tile is there (kpc < 128 <= num_slots)
     int64_t num_slots;
     float scale_log2;
@@ -93,7 +94,7 @@ struct PrefillTc2Params {
 // more beside the softmax warps, whatever its size).
 struct KvMaps {
     CUtensorMap rows[2];   // half rows of min(page, 8) keys: any slot
-    CUtensorMap page[2];   // whole rows of min(page, 128) keys from a slot that 8 divides
+    CUtensorMap page[2];   // whole rows of min(page, 128) keys from a slot that 8 divides (PrefillTc2Params::whole_pages)
     CUtensorMap tile[2];   // whole rows of 128 keys: tiles whose pages are consecutive slots
 };
 
@@ -142,7 +143,7 @@ attention_prefill_tc2_kernel(const __grid_constant__ KvMaps maps, const PrefillT
     pdl_launch_dependents();
     if (threadIdx.x == 0) {
         for (int kv = 0; kv < 2; ++kv) {
-            if (p.kpc >= 8) tma_prefetch_desc(&maps.page[kv]);
+            if (p.whole_pages) tma_prefetch_desc(&maps.page[kv]);
             if (p.whole_tile_boxes) tma_prefetch_desc(&maps.tile[kv]);
         }
         for (int s = 0; s < kSlots; ++s) {
@@ -195,7 +196,7 @@ attention_prefill_tc2_kernel(const __grid_constant__ KvMaps maps, const PrefillT
     // is a page, unless it is smaller than a group or starts inside one.
     auto load_tile = [&](int kv, int kt, uint32_t slot) {
         const int ncopies = copies_of(kt);
-        bool whole = kv_end - first_key(kt) >= kTile && p.whole_tile_boxes, groups = p.kpc >= 8;
+        bool whole = kv_end - first_key(kt) >= kTile && p.whole_tile_boxes, groups = p.whole_pages;
         int sl[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -583,7 +584,7 @@ int make_kv_tile_tmap(CUtensorMap* out, const void* cache, int64_t num_slots, in
 
 namespace {
 
-// Whole rows of `keys` (a multiple of 8) neighbouring slots, the first of them a multiple of 8: groups of 8 keys, in each
+// Whole rows of `keys` (a multiple of 8) neighbouring slots of 8 or more, the first of them a multiple of 8: groups of 8 keys, in each
 // both halves of the head dimension (coordinates: element of a half, key of a group, half, group, head).
 int make_kv_groups_tmap(CUtensorMap* out, const void* cache, int64_t num_slots, int kv_heads, int keys) {
     EncodeTiledFn fn = encode_tiled_fn();
@@ -592,7 +593,7 @@ int make_kv_groups_tmap(CUtensorMap* out, const void* cache, int64_t num_slots, 
         return B200_ERR_CUDA;
     }
     const cuuint64_t slot = static_cast<cuuint64_t>(kv_heads) * kD * 2;
-    const cuuint64_t dims[5] = {64, 8, 2, static_cast<cuuint64_t>(num_slots / 8 > 0 ? num_slots / 8 : 1), static_cast<cuuint64_t>(kv_heads)};
+    const cuuint64_t dims[5] = {64, 8, 2, static_cast<cuuint64_t>(num_slots / 8), static_cast<cuuint64_t>(kv_heads)};
     const cuuint64_t strides[4] = {slot, 128, slot * 8, kD * 2};
     const cuuint32_t box[5] = {64, 8, 2, static_cast<cuuint32_t>(keys / 8), 1};
     const cuuint32_t es[5] = {1, 1, 1, 1, 1};
@@ -636,11 +637,12 @@ int launch_attention_prefill_tc2(void* out, const void* q, int64_t q_st, int64_t
     if (window) p.w = *window;
     if (p.w.out_st == 0) p.w.out_st = static_cast<int64_t>(q_heads) * kD;
     KvMaps maps = {};
+    p.whole_pages = p.kpc >= 8 && num_slots >= 8 ? 1 : 0;
     p.whole_tile_boxes = p.kpc < kTile && num_slots >= kTile ? 1 : 0;
     for (int kv = 0; kv < 2; ++kv) {
         const void* cache = kv == 0 ? k_cache : v_cache;
         int err = make_kv_tile_tmap(&maps.rows[kv], cache, num_slots, kv_heads, p.kpc < 8 ? p.kpc : 8);
-        if (err == B200_OK && p.kpc >= 8) err = make_kv_groups_tmap(&maps.page[kv], cache, num_slots, kv_heads, p.kpc);
+        if (err == B200_OK && p.whole_pages) err = make_kv_groups_tmap(&maps.page[kv], cache, num_slots, kv_heads, p.kpc);
         if (err == B200_OK && p.whole_tile_boxes) err = make_kv_groups_tmap(&maps.tile[kv], cache, num_slots, kv_heads, kTile);
         if (err != B200_OK) return err;
     }

@@ -145,3 +145,24 @@ def test_prefill_copies_pages_of_any_size_and_place(L, page_size, offset, seq_le
     want = O.paged_attention(q, kc, vc, table, ps.table_idx, ps.seq_lens, qo, 1.0 / math.sqrt(d), O.store_fp32)
     assert_close_bf16(got, want.reshape(len(q), hq * d), ATOL, RTOL, "prefill attention")
     assert L.read_device_status() == (0, 0)
+
+
+@pytest.mark.parametrize("page_size,num_slots", [(8, 1), (8, 4), (8, 7), (16, 4), (16, 7), (16, 12), (256, 7), (256, 12)])
+def test_prefill_from_a_cache_smaller_than_a_page(L, pkg, page_size, num_slots):
+    """Every page is reported, and nothing behind the cache is read: what follows it is not finite."""
+    from sglang_cpp_b200._lib import call
+
+    hq, hkv, d, n = 4, 2, 128, 70
+    gen = torch.Generator(device="cuda").manual_seed(num_slots)
+    k, v = (torch.full((512, hkv, d), float("nan"), device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    for t in (k, v):
+        t[:num_slots].normal_(generator=gen)
+    q = torch.randn(n, hq, d, device="cuda", generator=gen).to(torch.bfloat16)
+    out = torch.full((n, hq * d), 7.0, device="cuda", dtype=torch.bfloat16)
+    table, one, lens, qo = (torch.tensor(x, dtype=torch.int32, device="cuda") for x in (list(range(n)), [0], [n], [0, n]))
+    call("b200_attention_prefill", out.data_ptr(), q.data_ptr(), hq * d, d, k.data_ptr(), v.data_ptr(), num_slots, table.data_ptr(), n,
+         one.data_ptr(), lens.data_ptr(), qo.data_ptr(), 1, n, hq, hkv, d, page_size, d ** -0.5, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert torch.isfinite(out).all()
+    status = L.read_device_status()
+    assert status[0] == 0 and status[1] != 0
