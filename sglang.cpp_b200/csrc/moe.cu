@@ -31,7 +31,10 @@ __device__ __forceinline__ void route_token(const __nv_bfloat16* __restrict__ ro
     float sum = 0.f;
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
-        v[i] = (lane + i * 32) < E ? __expf(v[i] - mx) : -1.f;  // -1 marks "not a candidate"
+        // -1 marks "not a candidate".  What is not a number has no part and comes last, so that a token's experts are valid and differ
+        // (asked of the difference: the compiler takes the exponential for a number)
+        const float below = v[i] - mx;
+        v[i] = (lane + i * 32) < E ? (below <= 0.f ? __expf(below) : 0.f) : -1.f;
         if (v[i] > 0.f) sum += v[i];
     }
     sum = warp_sum(sum);
@@ -57,7 +60,6 @@ __device__ __forceinline__ void route_token(const __nv_bfloat16* __restrict__ ro
                 bi = oi;
             }
         }
-        if (bi >= E) bi = k;   // NaN logits: a token's experts are valid and differ all the same
 #pragma unroll
         for (int i = 0; i < PER; ++i)
             if (bi == lane + i * 32) v[i] = -1.f;

@@ -37,6 +37,38 @@ def test_route_matches_torch_topk(L, T, E, k, renorm):
     assert torch.equal(counts.cpu().long(), torch.bincount(ti.flatten(), minlength=E))
 
 
+@pytest.mark.parametrize("E,k", [(8, 3), (64, 4), (130, 16), (256, 16)])
+def test_route_of_logits_that_are_not_numbers(L, E, k):
+    """Some, all but one, or all of a token's logits NaN, infinities among them: its experts are valid and differ (an expert's rows are
+    counted on that), and those that are numbers come first, in their order."""
+    gen = torch.Generator().manual_seed(E + k)
+    T = 70
+    logits = distinct_router_logits(gen, T, 256)[:, :E].clone()
+    for t in range(T):
+        there = torch.randperm(E, generator=gen)[:[0, 1, 2, k - 1, k, E - 1][t % 6]]
+        keep = logits[t, there].clone()
+        logits[t] = float("nan")
+        logits[t, there] = keep
+    logits[0, 1] = float("inf")
+    logits[6] = -float("inf")
+    for tokens in (T, 9):   # by the kernel for many tokens, and the one that also places their rows
+        ids, w, counts = L.moe_route(logits[:tokens].cuda(), k, True)
+        ids = ids.cpu().long()
+        assert ((ids >= 0) & (ids < E)).all() and all(len(set(row)) == k for row in ids.tolist())
+        assert torch.equal(counts.cpu().long(), torch.bincount(ids.flatten(), minlength=E))
+        for t in range(1, tokens):
+            n = min(int(torch.isfinite(logits[t]).sum()), k)
+            finite = torch.where(torch.isfinite(logits[t]), logits[t].float(), torch.tensor(-1e9))
+            assert torch.equal(ids[t, :n], finite.topk(n).indices), t
+    moe = L.MoELayer(E, k, 64, 64, True, "silu")   # (and through the layer: rows of every expert within what it expects)
+    moe.gate_up_proj.zero_()
+    moe.down_proj.zero_()
+    for tokens in (T, 9):
+        moe.forward(randn_bf16(gen, tokens, 64).cuda(), logits[:tokens].cuda())
+        torch.cuda.synchronize()
+    assert L.read_device_status() == (0, 0)
+
+
 @pytest.mark.parametrize("T,E,k,H,I,renorm,act", [
     (6, 3, 2, 64, 64, True, "silu"),            # the reference test's routing shape
     (64, 16, 4, 256, 128, True, "silu"),
