@@ -1042,6 +1042,7 @@ int b200_engine_capture_graphs(b200_engine* e, const int32_t* batch_sizes, int c
             // Warm-up + capture run on the dummy request only (GraphRunner::capture_graphs does the
             // same): every row is the dummy row, one key each, nothing is written back.
             B200_CHECK_CUDA(cudaStreamSynchronize(e->stream));
+            e->status_copied = false;
             b200_step st = {};
             st.phase = B200_PHASE_DECODE;
             st.num_reqs = 0;
@@ -1085,6 +1086,7 @@ static int run_step(b200_engine* e, const b200_step* st, int32_t* next_tokens_ho
     const int B = st->num_reqs, Bp = st->num_padded_reqs;
     B200_CHECK_ARG(B >= 0 && Bp >= B && Bp <= e->max_batch, "engine_step: batch size out of range");
     if (Bp == 0) return B200_OK;
+    e->status_copied = false;   // (until this step's have been: one that fails half way has run kernels, too)
     B200_CHECK_ARG(st->table_idx && st->cached_lens && st->extend_lens, "engine_step: NULL request arrays");
     const bool sampling = st->temperatures != nullptr;
     if (e->meta_in_flight) {  // the staging block of the previous step must have been consumed
@@ -1126,7 +1128,6 @@ static int run_step(b200_engine* e, const b200_step* st, int32_t* next_tokens_ho
     }
     // Tokens and what the step's kernels report, written to the host by one kernel where the caller's buffer is pinned (two
     // copies on the engine's stream take 12 us, and a copy for b200_engine_synchronize alone as long).
-    e->status_copied = slot == nullptr;
     if (!slot) {
         const bool tokens = next_tokens_host && B > 0;
         cudaPointerAttributes at = {};
@@ -1142,6 +1143,7 @@ static int run_step(b200_engine* e, const b200_step* st, int32_t* next_tokens_ho
                                       static_cast<int32_t*>(at.devicePointer), static_cast<int32_t*>(status_host),
                                       static_cast<const int32_t*>(e->next_tokens), static_cast<const int*>(e->status),
                                       pinned && tokens ? B : 0));   // (not one of the model's: not counted with them)
+        e->status_copied = true;
     }
     if (slot) {
         B200_CHECK_CUDA(launch_kernel(publish_step_kernel, dim3(1), dim3(256), 0, s, dim3(1, 1, 1), slot->tokens,
@@ -1200,8 +1202,9 @@ int b200_engine_wait(b200_engine* e, int64_t ticket, const int32_t** tokens, con
     if (finished) *finished = slot.finished;
     const int timeout_site = slot.status[0], bad_index = slot.status[1];
     if (timeout_site != 0 || bad_index != 0) {
-        // rare: clear the device words for the steps that follow
+        // rare: clear the device words for the steps that follow (and ask them, not what came along with an earlier step)
         cudaStreamSynchronize(e->stream);
+        e->status_copied = false;
         cudaMemset(e->status, 0, 2 * sizeof(int));
         if (timeout_site != 0) {
             set_last_error("a bounded wait inside a kernel ran out (site %d)", timeout_site);

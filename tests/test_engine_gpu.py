@@ -705,6 +705,37 @@ def test_tokens_into_pinned_and_pageable_memory_and_reports_of_steps(pkg, nreq):
     e.close()
 
 
+def test_reports_are_of_what_ran_last(pkg):
+    """What a step brought along is not told in place of the reports of kernels that have run since."""
+    cfg = small_cfg("qwen3")
+    pr = Pair(pkg, cfg, 16)
+    rng = np.random.default_rng(3)
+    req = pr.hb.add_request(rng.integers(0, cfg.vocab_size, size=9).astype(np.int32), 8)
+    pr.hb.allocate([req])
+    pr.hb.prefill([req]).synchronize()
+    e, rows = pr.engine, np.array([req.table_idx], np.int32)
+    zeros, lens, none = np.zeros(1, np.int32), np.array([9], np.int32), np.full(1, -1, np.int32)
+    good, bad = e.read_table("token_pool")[rows[0], :1].tolist(), cfg.vocab_size + 3   # (a token that is no token)
+    # a report that waiting for a step has told is not told again from the copy of a later step
+    e.write_token_pool(rows, [0], [bad])
+    out = e.forward_batch_async(0, rows, zeros, lens, none)
+    e.forward_batch(0, rows, zeros, lens, none)
+    with pytest.raises(pkg.B200Error, match=str(bad)):
+        out.wait()
+    e.synchronize()
+    # the kernels that run before a graph is captured, behind a step with nothing to report
+    e.write_token_pool(rows, [0], good)
+    e.forward_batch(0, rows, zeros, lens, none)
+    dummy = [pr.max_running_req]
+    e.write_token_pool(dummy, [0], [bad])
+    e.capture_graphs([1])
+    with pytest.raises(pkg.B200Error, match=str(bad)):
+        e.synchronize()
+    e.write_token_pool(dummy, [0], [0])
+    e.synchronize()
+    e.close()
+
+
 @pytest.mark.parametrize("nreq,cached", [(1, 60), (1, 300), (2, 200), (4, 90)])
 def test_decode_of_wide_experts_repeats_itself(pkg, monkeypatch, nreq, cached):
     """Experts whose weights stream through a ring while the CTAs of the next kernels begin to load on the same SMs: a stage is not
