@@ -67,7 +67,7 @@ __global__ void select_last_rows_kernel(uint4* __restrict__ dst, const uint4* __
     pdl_launch_dependents();
     pdl_wait_prior();
     const int b = blockIdx.x;
-    const int64_t row = qo[b + 1] - 1;
+    const int64_t row = max(qo[b + 1] - 1, 0);   // (no token at all: some row, which nobody asks for)
     for (int v = threadIdx.x; v < vec_per_row; v += blockDim.x)
         dst[static_cast<int64_t>(b) * vec_per_row + v] = src[row * vec_per_row + v];
 }
