@@ -352,7 +352,7 @@ RingParams ring_params(void* y, int N, int K, int epilogue, float act_limit, int
 // against 566, 16 requests 498 against 594.
 bool ring_gemm_takes(const void* x, const void* w, int M, int N, int K, int64_t ldx, int epilogue, bool narrow) {
     const int n_out = epilogue_is_gated(epilogue) ? N / 2 : N;
-    return M <= 16 && K >= 2048 && static_cast<int64_t>(N) * K >= (narrow ? 12ll << 20 : 4ll << 20) && n_out % 8 == 0 && K % 64 == 0 && ldx % 8 == 0 &&
+    return M >= 1 && M <= 16 && K >= 2048 && static_cast<int64_t>(N) * K >= (narrow ? 12ll << 20 : 4ll << 20) && n_out % 8 == 0 && K % 64 == 0 && ldx % 8 == 0 &&
            aligned16(x, w);
 }
 

@@ -736,6 +736,23 @@ def test_reports_are_of_what_ran_last(pkg):
     e.close()
 
 
+def test_a_step_without_a_token(pkg):
+    """Requests that bring nothing new: nothing is computed, and nothing refuses to (layers wide enough for every GEMM)."""
+    cfg = O.ModelConfig(1, 2048, 8, 8, 128, 2048, 1024, 1e-6, 1e6, 512, True, True, True)
+    pr = Pair(pkg, cfg, 16)
+    rng = np.random.default_rng(4)
+    reqs = [pr.hb.add_request(rng.integers(0, cfg.vocab_size, size=9 + i).astype(np.int32), 8) for i in range(2)]
+    pr.hb.allocate(reqs)
+    first = pr.hb.prefill(reqs)
+    first.synchronize()
+    want = pr.engine.logits(2).clone()
+    rows, zeros, none = np.array([r.table_idx for r in reqs], np.int32), np.zeros(2, np.int32), np.full(2, -1, np.int32)
+    pr.engine.forward_batch(0, rows, np.array([9, 10], np.int32), zeros, none).synchronize()
+    pr.engine.forward_batch(0, rows, zeros, np.array([9, 10], np.int32), none).synchronize()
+    assert torch.equal(pr.engine.logits(2), want)
+    pr.engine.close()
+
+
 @pytest.mark.parametrize("nreq,cached", [(1, 60), (1, 300), (2, 200), (4, 90)])
 def test_decode_of_wide_experts_repeats_itself(pkg, monkeypatch, nreq, cached):
     """Experts whose weights stream through a ring while the CTAs of the next kernels begin to load on the same SMs: a stage is not
