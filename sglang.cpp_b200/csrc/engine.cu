@@ -1130,9 +1130,14 @@ static int run_step(b200_engine* e, const b200_step* st, int32_t* next_tokens_ho
     // copies on the engine's stream take 12 us, and a copy for b200_engine_synchronize alone as long).
     if (!slot) {
         const bool tokens = next_tokens_host && B > 0;
-        cudaPointerAttributes at = {};
-        const bool pinned = !tokens || (cudaPointerGetAttributes(&at, next_tokens_host) == cudaSuccess &&
-                                        at.type == cudaMemoryTypeHost && at.devicePointer != nullptr);
+        // (a copy takes a buffer that lies anywhere, also one of which only the beginning is pinned)
+        cudaPointerAttributes at = {}, end = {};
+        auto mapped = [](cudaPointerAttributes* a, const int32_t* p) {
+            return cudaPointerGetAttributes(a, p) == cudaSuccess && a->type == cudaMemoryTypeHost && a->devicePointer != nullptr;
+        };
+        const bool pinned = !tokens || (reinterpret_cast<uintptr_t>(next_tokens_host) % sizeof(int32_t) == 0 && mapped(&at, next_tokens_host) &&
+                                        mapped(&end, next_tokens_host + B - 1) &&
+                                        static_cast<int32_t*>(end.devicePointer) == static_cast<int32_t*>(at.devicePointer) + B - 1);
         if (!pinned) {
             cudaGetLastError();
             B200_CHECK_CUDA(cudaMemcpyAsync(next_tokens_host, e->next_tokens, B * sizeof(int32_t), cudaMemcpyDeviceToHost, s));
