@@ -1147,8 +1147,7 @@ static int run_step(b200_engine* e, const b200_step* st, int32_t* next_tokens_ho
         B200_CHECK_CUDA(launch_kernel(publish_tokens_kernel, dim3(1), dim3(128), 0, s, dim3(1, 1, 1),
                                       static_cast<int32_t*>(at.devicePointer), static_cast<int32_t*>(status_host),
                                       static_cast<const int32_t*>(e->next_tokens), static_cast<const int*>(e->status),
-                                      pinned && tokens ? B : 0));
-        e->launches_last_step += 1;
+                                      pinned && tokens ? B : 0));   // (not one of the model's: not counted with them)
         e->status_copied = true;
     }
     if (slot) {
