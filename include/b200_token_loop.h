@@ -940,7 +940,8 @@ B200_API b200_stream_t b200_engine_stream(b200_engine* engine);
  * src/engine/engine.cc:36-87): while on, steps run eagerly (no graph replay) with a CUDA event
  * pair around each attention launch.  b200_engine_read_profile synchronises and returns the
  * summed attention time of the last step, how many attention launches that covers, and the
- * number of kernels the last step launched (also valid for graph replays, profiling or not). */
+ * number of kernels the last step launched (also valid for graph replays, profiling or not; b200_engine_step's kernel
+ * that hands tokens and reports to the host, where a copy stood, is not one of them). */
 B200_API int b200_engine_set_profiling(b200_engine* engine, int on);
 B200_API int b200_engine_read_profile(b200_engine* engine, float* attention_ms,
                                       int32_t* attention_launches, int32_t* kernel_launches);
