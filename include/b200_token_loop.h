@@ -378,11 +378,14 @@ B200_API int b200_linear_act(void* y, const void* x, const void* w, int M, int N
 /* The kernel that b200_linear (groups 0) or the expert projections (rows of all `groups` experts together, at most max_rows of
  * them one expert's) run on for a shape with aligned operands; normed: in a decode step, with the norm of its input in the
  * projection; 0: no such shape.  Nothing is launched; needs no device. */
-#define B200_GEMM_NARROW 1   /* weights from memory to registers: a handful of rows (many experts, or a large W of K >= 2048: a ring per SM) */
-#define B200_GEMM_STREAM 2   /* weights through shared memory, split along K: a decode batch (up to 16 rows of K >= 2048: a ring per SM) */
+#define B200_GEMM_NARROW 1   /* weights from memory to registers: a handful of rows; or the ring kernel in its place */
+#define B200_GEMM_STREAM 2   /* weights through shared memory, split along K: a decode batch; or the ring kernel in its place */
 #define B200_GEMM_TILE 3     /* tiles of single CTAs */
 #define B200_GEMM_PAIR 4     /* tiles of pairs of CTAs */
 B200_API int b200_gemm_kernel(int64_t rows, int N, int K, int epilogue, int groups, int max_rows, int normed);
+/* 1 where the ring kernel runs in place of the one that b200_gemm_kernel names (weights through a ring per SM without a break: a
+ * handful of rows of a large W, or of many experts), 0 elsewhere. */
+B200_API int b200_gemm_by_ring(int64_t rows, int N, int K, int epilogue, int groups, int max_rows);
 
 /* The wiring with the norm on what a block returned (layer_norm below: the same with layer norms):
  *   a = sum_k src_weights[t, k] src[src_rows[t, k], :] + src2[t, :]   (src_rows NULL: src[t, :]; weights NULL: 1),

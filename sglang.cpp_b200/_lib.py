@@ -126,6 +126,7 @@ PROTOTYPES: dict[str, tuple] = {
     "b200_linear_f32": (_I, [_P, _P, _P, _I, _I, _I, _I, _P, _P, _I, _P]),
     "b200_head_pass_by_tokens": (_I, [_I, _I, _I, _I, _I]),
     "b200_gemm_kernel": (_I, [c_int64, _I, _I, _I, _I, _I, _I]),
+    "b200_gemm_by_ring": (_I, [c_int64, _I, _I, _I, _I, _I]),
     "b200_linear_act": (_I, [_P, _P, _P, _I, _I, _I, _I, _F, _I, _P]),
     "b200_residual_post_norm": (_I, [_P, _P, _P, _P, _P, _I, _L, _P, _I, _P, _P, _I, _I, _I, _F, _I, _P]),
     "b200_residual_layer_norm": (_I, [_P, _P, _P, _P, _P, _I, _L, _P, _F, _I, _P, _P, _P, _P, _I, _I, _I, _F, _I, _P]),

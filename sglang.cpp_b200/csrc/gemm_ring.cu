@@ -357,13 +357,13 @@ bool ring_gemm_takes(const void* x, const void* w, int M, int N, int K, int64_t 
 }
 
 int launch_ring_gemm(void* y, const void* x, const void* w, const void* bias, int M, int N, int K, int64_t ldx, int epilogue, int* status,
-                     cudaStream_t stream, float act_limit, bool narrow) {
+                     cudaStream_t stream, float act_limit) {
     RingParams p = ring_params(y, N, K, epilogue, act_limit, status);
     p.bias = static_cast<const __nv_bfloat16*>(bias);
     p.M = M;
     // Where the registers' kernel would take the call, the next kernels are let in as that one lets them in: 2048 x 6144 with 16 rows
     // at the end of a layer is no faster with them let in at once, 501 us per step against 498.
-    p.early = !narrow || K < kWalkedK;
+    p.early = K < kWalkedK || !narrow_gemm_takes(x, w, M, N, K, ldx, epilogue);
     return launch_ring(p, x, M, ldx, w, N, false, stream);
 }
 

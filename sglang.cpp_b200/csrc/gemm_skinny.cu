@@ -809,8 +809,16 @@ int launch_skinny_gemm(void* y, const void* x, const void* w, const void* bias, 
     return B200_OK;
 }
 
-static bool grouped_on_tiles(int64_t total_rows, int num_groups) {
-    return total_rows >= static_cast<int64_t>(num_groups) * env_int("B200_GROUPED_TILE_MIN_ROWS", 128) && num_groups <= 256;
+// What b200_gemm_kernel calls by the name of the kernel that it stands in for.
+constexpr int kGemmRing = 5;
+
+// The kernel (B200_GEMM_*, kGemmRing; B200_GEMM_TILE for pairs of CTAs as well) of the expert projections: a handful of rows per group have two,
+// many rows per group on average (prompts) are tensor-bound.
+static int grouped_kernel(const void* x, const void* w, int64_t total_rows, int max_rows, int num_groups, int n_out, int K, int epilogue) {
+    if (narrow_grouped_takes(x, w, total_rows, max_rows, num_groups, n_out, K, epilogue))
+        return ring_grouped_takes(x, w, max_rows, num_groups, n_out, K) ? kGemmRing : B200_GEMM_NARROW;
+    const bool tiles = total_rows >= static_cast<int64_t>(num_groups) * env_int("B200_GROUPED_TILE_MIN_ROWS", 128) && num_groups <= 256;
+    return tiles ? B200_GEMM_TILE : B200_GEMM_STREAM;
 }
 
 // Grouped GEMM for expert layers: group g multiplies rows [offsets[g], offsets[g] + counts[g]) of
@@ -827,14 +835,11 @@ int launch_grouped_gemm(void* y, const void* x, const void* w, const int32_t* co
     const int n_tiles = div_ceil(n_out, kTileN);
     const int slabs = div_ceil(max_rows_per_group, 256);
     if (num_groups == 0 || slabs == 0 || total_rows == 0) return B200_OK;
-    // A handful of rows per group: weights straight into registers.
-    if (narrow_grouped_takes(x, w, total_rows, max_rows_per_group, num_groups, n_out, K, epilogue)) {
-        if (ring_grouped_takes(x, w, max_rows_per_group, num_groups, n_out, K))
-            return launch_ring_grouped(y, x, w, counts, offsets, num_groups, total_rows, N, K, epilogue, status, stream, act_limit);
-        return launch_narrow_grouped(y, x, w, counts, offsets, num_groups, N, K, epilogue, stream, act_limit);
-    }
-    // Many rows per group on average (prefill batches): tensor-bound, take the tile kernel.
-    if (grouped_on_tiles(total_rows, num_groups))
+    const int kernel_id = grouped_kernel(x, w, total_rows, max_rows_per_group, num_groups, n_out, K, epilogue);
+    if (kernel_id == kGemmRing)
+        return launch_ring_grouped(y, x, w, counts, offsets, num_groups, total_rows, N, K, epilogue, status, stream, act_limit);
+    if (kernel_id == B200_GEMM_NARROW) return launch_narrow_grouped(y, x, w, counts, offsets, num_groups, N, K, epilogue, stream, act_limit);
+    if (kernel_id == B200_GEMM_TILE)
         return launch_grouped_tile_gemm(y, x, w, counts, offsets, num_groups, total_rows, N, K, epilogue, status,
                                         stream, act_limit);
     int nt_max = 32;
@@ -961,31 +966,44 @@ static bool linear_on_tiles(const void* y, int M, int N, int K, int epilogue, bo
     return tile_gemm_us(M, N, K, epilogue) < 0.9f * skinny_gemm_us(M, N, K, epilogue);
 }
 
-int gemm_kernel_of(int64_t rows, int N, int K, int epilogue, int groups, int max_rows, bool normed) {
-    const int n_out = epilogue_is_gated(epilogue) ? N / 2 : N;
-    if (groups == 0) {
-        const int M = static_cast<int>(rows);
-        if (narrow_gemm_takes(nullptr, nullptr, M, N, K, K, epilogue, normed)) return B200_GEMM_NARROW;
-        if (!linear_on_tiles(nullptr, M, N, K, epilogue, false)) return B200_GEMM_STREAM;
-        return tile_gemm_features(M, N, K, epilogue) > 0 ? B200_GEMM_PAIR : B200_GEMM_TILE;
+// The kernel (B200_GEMM_*, kGemmRing; B200_GEMM_TILE for pairs of CTAs as well) of a projection.  narrow: the kernels of a handful of rows may take it; fused: something rides in the
+// weight-streaming kernel; normed: the norm of x rides in the projection.
+static int linear_kernel(const void* y, const void* x, const void* w, int M, int N, int K, int64_t ldx, int epilogue, bool narrow, bool fused,
+                         bool normed) {
+    if (narrow && !fused) {   // weights straight into registers, or of a large W through a ring
+        const bool registers = narrow_gemm_takes(x, w, M, N, K, ldx, epilogue, normed);
+        if (!normed && ring_gemm_takes(x, w, M, N, K, ldx, epilogue, registers)) return kGemmRing;
+        if (registers) return B200_GEMM_NARROW;
     }
-    if (narrow_grouped_takes(nullptr, nullptr, rows, max_rows, groups, n_out, K, epilogue)) return B200_GEMM_NARROW;
-    if (!grouped_on_tiles(rows, groups)) return B200_GEMM_STREAM;
-    return grouped_on_pairs(rows, groups) ? B200_GEMM_PAIR : B200_GEMM_TILE;
+    // Few rows: stream the weights once (swap-AB, split-K).  Many rows: tensor-bound tiles.
+    return linear_on_tiles(y, M, N, K, epilogue, fused) ? B200_GEMM_TILE : B200_GEMM_STREAM;
+}
+
+int gemm_kernel_of(int64_t rows, int N, int K, int epilogue, int groups, int max_rows, bool normed) {
+    const int M = static_cast<int>(rows), n_out = epilogue_is_gated(epilogue) ? N / 2 : N;
+    if (groups == 0) {
+        const int kernel = linear_kernel(nullptr, nullptr, nullptr, M, N, K, K, epilogue, true, false, normed);
+        if (kernel == kGemmRing) return narrow_gemm_takes(nullptr, nullptr, M, N, K, K, epilogue) ? B200_GEMM_NARROW : B200_GEMM_STREAM;
+        return kernel == B200_GEMM_TILE && tile_gemm_features(M, N, K, epilogue) > 0 ? B200_GEMM_PAIR : kernel;
+    }
+    const int kernel = grouped_kernel(nullptr, nullptr, rows, max_rows, groups, n_out, K, epilogue);
+    if (kernel == kGemmRing) return B200_GEMM_NARROW;
+    return kernel == B200_GEMM_TILE && grouped_on_pairs(rows, groups) ? B200_GEMM_PAIR : kernel;
+}
+
+bool gemm_by_ring(int64_t rows, int N, int K, int epilogue, int groups, int max_rows) {
+    const int M = static_cast<int>(rows), n_out = epilogue_is_gated(epilogue) ? N / 2 : N;
+    return kGemmRing == (groups == 0 ? linear_kernel(nullptr, nullptr, nullptr, M, N, K, K, epilogue, true, false, false)
+                                     : grouped_kernel(nullptr, nullptr, rows, max_rows, groups, n_out, K, epilogue));
 }
 
 int launch_linear(void* y, const void* x, const void* w, const void* bias, int M, int N, int K,
                   int64_t ldx, int epilogue, int* status, cudaStream_t stream, const SkinnyFusion* fuse,
                   float act_limit, bool narrow) {
-    // A handful of rows: weights straight into registers, or of a large W through a ring.
-    if (narrow && fuse == nullptr) {
-        const bool registers = narrow_gemm_takes(x, w, M, N, K, ldx, epilogue);
-        if (ring_gemm_takes(x, w, M, N, K, ldx, epilogue, registers))
-            return launch_ring_gemm(y, x, w, bias, M, N, K, ldx, epilogue, status, stream, act_limit, registers);
-        if (registers) return launch_narrow_gemm(y, x, w, bias, M, N, K, ldx, epilogue, status, stream, nullptr, act_limit);
-    }
-    // Few rows: stream the weights once (swap-AB, split-K).  Many rows: tensor-bound tiles.
-    if (linear_on_tiles(y, M, N, K, epilogue, fuse != nullptr)) {
+    const int kernel_id = linear_kernel(y, x, w, M, N, K, ldx, epilogue, narrow, fuse != nullptr, false);
+    if (kernel_id == kGemmRing) return launch_ring_gemm(y, x, w, bias, M, N, K, ldx, epilogue, status, stream, act_limit);
+    if (kernel_id == B200_GEMM_NARROW) return launch_narrow_gemm(y, x, w, bias, M, N, K, ldx, epilogue, status, stream, nullptr, act_limit);
+    if (kernel_id == B200_GEMM_TILE) {
         if (fuse != nullptr) {
             set_last_error("linear: the residual-stream fusions need at most 256 rows");
             return B200_ERR_UNSUPPORTED;
@@ -1022,10 +1040,17 @@ int b200_linear_heads(void* y, const void* x, const void* w, int M, int heads, i
     return b200::launch_linear_heads(y, x, w, M, heads, N, K, status, static_cast<cudaStream_t>(stream));
 }
 
-int b200_gemm_kernel(int64_t rows, int N, int K, int epilogue, int groups, int max_rows, int normed) {
+static bool known_gemm(int64_t rows, int N, int K, int epilogue, int groups, int max_rows) {
     const bool shape = rows > 0 && rows <= INT32_MAX && N > 0 && K > 0 && K % 64 == 0 && groups >= 0 && (groups == 0 || max_rows > 0);
-    const bool known = epilogue >= B200_EPILOGUE_NONE && epilogue <= B200_EPILOGUE_F32;
-    return shape && known ? b200::gemm_kernel_of(rows, N, K, epilogue, groups, max_rows, normed != 0) : 0;
+    return shape && epilogue >= B200_EPILOGUE_NONE && epilogue <= B200_EPILOGUE_F32;
+}
+
+int b200_gemm_kernel(int64_t rows, int N, int K, int epilogue, int groups, int max_rows, int normed) {
+    return known_gemm(rows, N, K, epilogue, groups, max_rows) ? b200::gemm_kernel_of(rows, N, K, epilogue, groups, max_rows, normed != 0) : 0;
+}
+
+int b200_gemm_by_ring(int64_t rows, int N, int K, int epilogue, int groups, int max_rows) {
+    return known_gemm(rows, N, K, epilogue, groups, max_rows) && b200::gemm_by_ring(rows, N, K, epilogue, groups, max_rows) ? 1 : 0;
 }
 
 int b200_linear_act(void* y, const void* x, const void* w, int M, int N, int K, int epilogue, float act_limit, int dtype,

@@ -132,13 +132,14 @@ int launch_narrow_grouped(void* y, const void* x, const void* w, const int32_t* 
 // `narrow`: narrow_gemm_takes the call.
 bool ring_gemm_takes(const void* x, const void* w, int M, int N, int K, int64_t ldx, int epilogue, bool narrow);
 int launch_ring_gemm(void* y, const void* x, const void* w, const void* bias, int M, int N, int K, int64_t ldx, int epilogue, int* status,
-                     cudaStream_t stream, float act_limit, bool narrow);
+                     cudaStream_t stream, float act_limit);
 bool ring_grouped_takes(const void* x, const void* w, int max_rows, int num_groups, int n_out, int K);
 int launch_ring_grouped(void* y, const void* x, const void* w, const int32_t* counts, const int32_t* offsets, int num_groups,
                         int64_t total_rows, int N, int K, int epilogue, int* status, cudaStream_t stream, float act_limit);
 // The kernel (B200_GEMM_*) of launch_linear (groups 0) or launch_grouped_gemm with aligned operands and nothing fused but,
 // where asked for, the norm of the rows of x in a decode step.
 int gemm_kernel_of(int64_t rows, int N, int K, int epilogue, int groups, int max_rows, bool normed);
+bool gemm_by_ring(int64_t rows, int N, int K, int epilogue, int groups, int max_rows);   // the ring kernel in its place
 // The K split launch_linear picks for a slab of this shape (the fusions need it above 1).
 int skinny_gemm_split(int M, int N, int K, int epilogue);
 

@@ -53,6 +53,29 @@ def test_projections_of_a_handful_of_rows(pkg, N, K, epilogue, narrow, not_narro
         assert lib.b200_gemm_kernel(rows, N, K, epilogue, 0, 0, 0) == STREAM, rows
 
 
+@pytest.mark.parametrize("N,K,epilogue,ring,not_ring", [
+    (4096, 1024, PLAIN, (), (1, 8, 16)), (151936, 1024, PLAIN, (), (1, 8, 16)), (4096, 2048, PLAIN, (), (1, 8)), (6144, 2048, PLAIN, (1, 8, 16), (17,)),
+    (2048, 6144, PLAIN, (1, 8, 9, 16), (17,)), (32768, 2048, PLAIN, (1, 4, 8, 16), ()), (4096, 4096, PLAIN, (1, 8, 16), (17,)),
+    (28672, 4096, SWIGLU, (1, 16), (17,)), (1024, 16384, PLAIN, (1, 16), ()), (512, 32768, PLAIN, (1, 16), ()), (512, 4096, PLAIN, (), (1, 8)),
+])
+def test_projections_by_the_ring_kernel(pkg, N, K, epilogue, ring, not_ring):
+    """What runs there is told apart from the kernel whose place it takes."""
+    lib = pkg.load_library()
+    assert [lib.b200_gemm_by_ring(r, N, K, epilogue, 0, 0) for r in ring + not_ring] == [1] * len(ring) + [0] * len(not_ring)
+    assert all(lib.b200_gemm_kernel(r, N, K, epilogue, 0, 0, 0) in (NARROW, STREAM) for r in ring)
+
+
+@pytest.mark.parametrize("experts,per_token,hidden,inter,ring,not_ring", [
+    (64, 4, 2048, 1024, (1, 8, 32, 48), (49, 64)), (32, 2, 2048, 1024, (8, 32, 48), (49, 64)), (31, 2, 2048, 1024, (), (8, 32)),
+    (28, 4, 2048, 1024, (), (1, 8, 16)), (128, 8, 2048, 768, (1, 8), (64,)), (16, 4, 1024, 2048, (), (1, 32)),
+])
+def test_experts_by_the_ring_kernel(pkg, experts, per_token, hidden, inter, ring, not_ring):
+    lib = pkg.load_library()
+    for tokens, want in [(t, 1) for t in ring] + [(t, 0) for t in not_ring]:
+        assert lib.b200_gemm_by_ring(tokens * per_token, 2 * inter, hidden, SWIGLU, experts, tokens) == want, tokens
+        assert lib.b200_gemm_by_ring(tokens * per_token, hidden, inter, PLAIN, experts, tokens) == want, tokens
+
+
 @pytest.mark.parametrize("M,N,K,epilogue,kernel", [
     (64, 6144, 1024, SWIGLU, STREAM), (65, 6144, 1024, SWIGLU, PAIR), (65, 3072, 640, PLAIN, STREAM), (128, 2048, 1024, PLAIN, STREAM),
     (65, 12288, 1024, PLAIN, PAIR), (129, 2048, 1024, PLAIN, PAIR), (129, 1024, 1024, PLAIN, STREAM), (256, 1024, 1024, PLAIN, PAIR),
@@ -78,6 +101,7 @@ def test_expert_tiles(pkg, rows, kernel):
 
 def test_shapes_that_no_kernel_takes(pkg):
     lib = pkg.load_library()
+    assert [lib.b200_gemm_by_ring(*a) for a in [(0, 4096, 4096, 0, 0, 0), (4, 4096, 4000, 0, 0, 0), (4, 4096, 4096, 99, 0, 0), (4, 4096, 4096, 0, 2, 0)]] == [0] * 4
     assert [lib.b200_gemm_kernel(*a) for a in [(0, 64, 64, 0, 0, 0, 0), (4, 64, 96, 0, 0, 0, 0), (4, 64, 64, 99, 0, 0, 0), (4, 64, 64, 0, 2, 0, 0)]] == [0] * 4
 
 

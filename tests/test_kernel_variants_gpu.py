@@ -225,9 +225,13 @@ def test_experts_on_pair_tiles_that_tokens_do_not_choose_alike(L, pkg):
 
 
 @pytest.mark.parametrize("T,E,k,H,I,act", [(32, 16, 4, 2048, 1024, "silu"), (1, 64, 4, 1088, 64, "silu"), (9, 3, 1, 64, 192, "gelu"),
-                                           (24, 16, 4, 1024, 2048, "silu")])
-def test_experts_of_a_handful_of_rows(L, T, E, k, H, I, act):
-    """At most 8 rows per expert on average, some with more and some with none; K of one and of two register buffers."""
+                                           (24, 16, 4, 1024, 2048, "silu"), (64, 32, 2, 1088, 64, "silu")])
+def test_experts_of_a_handful_of_rows(L, pkg, T, E, k, H, I, act):
+    """At most 8 rows per expert on average, some with more and some with none; K of one and of two register buffers.  (Many experts
+    with up to 48 tokens: the ring kernel.)"""
+    lib = pkg.load_library()
+    assert lib.b200_gemm_kernel(T * k, 2 * I, H, pkg.EPILOGUE_SWIGLU, E, T, 0) == NARROW
+    assert lib.b200_gemm_by_ring(T * k, 2 * I, H, pkg.EPILOGUE_SWIGLU, E, T) == (E >= 32 and T <= 48)
     moe_forward(L, T, E, k, H, I, True, act)
 
 
@@ -299,6 +303,7 @@ def test_linear_of_few_rows_of_a_large_w(L, pkg, M, N, K):
     SMs, one and two blocks of tokens."""
     lib = pkg.load_library()
     assert lib.b200_gemm_kernel(M, N, K, pkg.EPILOGUE_NONE, 0, 0, 0) == (STREAM if K > 2048 or M > 8 else NARROW)
+    assert lib.b200_gemm_by_ring(M, N, K, pkg.EPILOGUE_NONE, 0, 0) == (K >= 2048)
     gen = torch.Generator().manual_seed(M + N + K)
     buf, w, b = randn_bf16(gen, M, K + 64), randn_bf16(gen, N, K, std=0.05), randn_bf16(gen, N)
     atol = BIG[0] * (K / 1024) ** 0.5 + BIG[1]
@@ -317,6 +322,7 @@ def test_many_experts_of_few_rows(L, pkg, T, E, k, H, I, alike):
     """The ring kernel's experts: rows of an expert below, at and above the 8 and 16 of one pass, K within a stage and beyond."""
     lib = pkg.load_library()
     assert lib.b200_gemm_kernel(T * k, 2 * I, H, pkg.EPILOGUE_SWIGLU, E, T, 0) == NARROW
+    assert lib.b200_gemm_by_ring(T * k, 2 * I, H, pkg.EPILOGUE_SWIGLU, E, T) == lib.b200_gemm_by_ring(T * k, H, I, pkg.EPILOGUE_NONE, E, T) == 1
     gen = torch.Generator().manual_seed(T + E + H)
     hidden = randn_bf16(gen, T, H)
     logits = torch.randn(T, E, generator=gen).argsort(1).to(torch.bfloat16) / 32   # distinct in every row
