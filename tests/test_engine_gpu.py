@@ -689,10 +689,6 @@ def test_tokens_into_pinned_and_pageable_memory_and_reports_of_steps(pkg, nreq):
     call("b200_engine_step", e._h, ctypes.byref(step), pageable.ctypes.data)   # the same prompts again
     e.synchronize()
     assert np.array_equal(pageable, out.next_tokens_cpu.numpy())
-    odd = torch.full((4 * nreq + 2,), 99, dtype=torch.uint8).pin_memory()   # pinned, but no place for a kernel's words
-    call("b200_engine_step", e._h, ctypes.byref(step), odd.data_ptr() + 1)
-    e.synchronize()
-    assert odd[1:-1].numpy().tobytes() == pageable.tobytes() and odd[0] == odd[-1] == 99
     assert np.array_equal(e.forward_batch_async(0, rows, zeros, lens, none).wait()[0], pageable)
     good = e.read_table("token_pool")[rows[0], :1].tolist()
     e.write_token_pool(rows[:1], [0], [cfg.vocab_size + 3])   # a token that is no token
@@ -706,6 +702,30 @@ def test_tokens_into_pinned_and_pageable_memory_and_reports_of_steps(pkg, nreq):
         e.synchronize()
     e.write_token_pool(rows[:1], [0], good)
     e.forward_batch(0, rows, zeros, lens, none).synchronize()
+    e.close()
+
+
+@pytest.mark.parametrize("nreq", [1, 5])
+def test_tokens_into_pinned_memory_that_holds_no_words(pkg, nreq):
+    """Pinned, but at an address that a kernel's words may not have: a copy, as into other memory."""
+    import ctypes
+
+    from sglang_cpp_b200._lib import StepStruct, call
+
+    cfg = small_cfg("qwen3")
+    pr = Pair(pkg, cfg, 16)
+    rng = np.random.default_rng(nreq)
+    reqs = [pr.hb.add_request(rng.integers(0, cfg.vocab_size, size=9 + i).astype(np.int32), 8) for i in range(nreq)]
+    pr.hb.allocate(reqs)
+    out = pr.hb.prefill(reqs)
+    out.synchronize()
+    e, rows = pr.engine, np.array([r.table_idx for r in reqs], np.int32)
+    zeros, lens, none = np.zeros(nreq, np.int32), np.array([9 + i for i in range(nreq)], np.int32), np.full(nreq, -1, np.int32)
+    step = StepStruct(0, nreq, nreq, rows.ctypes.data, zeros.ctypes.data, lens.ctypes.data, none.ctypes.data, None, None, None, None, 0)
+    odd = torch.full((4 * nreq + 2,), 99, dtype=torch.uint8).pin_memory()
+    call("b200_engine_step", e._h, ctypes.byref(step), odd.data_ptr() + 1)   # the same prompts again
+    e.synchronize()
+    assert odd[1:-1].numpy().tobytes() == out.next_tokens_cpu.numpy().tobytes() and odd[0] == odd[-1] == 99
     e.close()
 
 

@@ -225,13 +225,9 @@ def test_experts_on_pair_tiles_that_tokens_do_not_choose_alike(L, pkg):
 
 
 @pytest.mark.parametrize("T,E,k,H,I,act", [(32, 16, 4, 2048, 1024, "silu"), (1, 64, 4, 1088, 64, "silu"), (9, 3, 1, 64, 192, "gelu"),
-                                           (24, 16, 4, 1024, 2048, "silu"), (64, 32, 2, 1088, 64, "silu")])
-def test_experts_of_a_handful_of_rows(L, pkg, T, E, k, H, I, act):
-    """At most 8 rows per expert on average, some with more and some with none; K of one and of two register buffers.  (Many experts
-    with up to 48 tokens: the ring kernel.)"""
-    lib = pkg.load_library()
-    assert lib.b200_gemm_kernel(T * k, 2 * I, H, pkg.EPILOGUE_SWIGLU, E, T, 0) == NARROW
-    assert lib.b200_gemm_by_ring(T * k, 2 * I, H, pkg.EPILOGUE_SWIGLU, E, T) == (E >= 32 and T <= 48)
+                                           (24, 16, 4, 1024, 2048, "silu")])
+def test_experts_of_a_handful_of_rows(L, T, E, k, H, I, act):
+    """At most 8 rows per expert on average, some with more and some with none; K of one and of two register buffers."""
     moe_forward(L, T, E, k, H, I, True, act)
 
 
@@ -303,7 +299,6 @@ def test_linear_of_few_rows_of_a_large_w(L, pkg, M, N, K):
     SMs, one and two blocks of tokens."""
     lib = pkg.load_library()
     assert lib.b200_gemm_kernel(M, N, K, pkg.EPILOGUE_NONE, 0, 0, 0) == (STREAM if K > 2048 or M > 8 else NARROW)
-    assert lib.b200_gemm_by_ring(M, N, K, pkg.EPILOGUE_NONE, 0, 0) == (K >= 2048)
     gen = torch.Generator().manual_seed(M + N + K)
     buf, w, b = randn_bf16(gen, M, K + 64), randn_bf16(gen, N, K, std=0.05), randn_bf16(gen, N)
     atol = BIG[0] * (K / 1024) ** 0.5 + BIG[1]
@@ -322,7 +317,6 @@ def test_many_experts_of_few_rows(L, pkg, T, E, k, H, I, alike):
     """The ring kernel's experts: rows of an expert below, at and above the 8 and 16 of one pass, K within a stage and beyond."""
     lib = pkg.load_library()
     assert lib.b200_gemm_kernel(T * k, 2 * I, H, pkg.EPILOGUE_SWIGLU, E, T, 0) == NARROW
-    assert lib.b200_gemm_by_ring(T * k, 2 * I, H, pkg.EPILOGUE_SWIGLU, E, T) == lib.b200_gemm_by_ring(T * k, H, I, pkg.EPILOGUE_NONE, E, T) == 1
     gen = torch.Generator().manual_seed(T + E + H)
     hidden = randn_bf16(gen, T, H)
     logits = torch.randn(T, E, generator=gen).argsort(1).to(torch.bfloat16) / 32   # distinct in every row
@@ -335,3 +329,27 @@ def test_many_experts_of_few_rows(L, pkg, T, E, k, H, I, alike):
     assert_close_bf16(moe.forward(hidden.cuda(), logits.cuda()), O.moe_forward(hidden, logits, gu, dn, k, True, "silu", O.store_bf16),
                       2e-2, 4 * 2 ** -7, "experts")
     assert L.read_device_status() == (0, 0)
+
+
+@pytest.mark.parametrize("M", [1, 5, 8, 9, 13, 16])
+@pytest.mark.parametrize("N,K", [(6664, 2112), (3336, 4160), (1000, 14336), (28672, 512)])
+def test_few_rows_of_a_large_w_are_the_ring_kernels(pkg, M, N, K):
+    """What test_linear_of_few_rows_of_a_large_w runs on (the last shape: on its neighbours)."""
+    assert pkg.load_library().b200_gemm_by_ring(M, N, K, pkg.EPILOGUE_NONE, 0, 0) == (K >= 2048)
+
+
+@pytest.mark.parametrize("T", [1, 8, 9, 17, 40])
+@pytest.mark.parametrize("E,k,H,I", [(33, 4, 192, 576), (64, 3, 576, 64), (256, 1, 64, 128)])
+def test_many_experts_of_few_rows_are_the_ring_kernels(pkg, T, E, k, H, I):
+    """What test_many_experts_of_few_rows runs on."""
+    lib = pkg.load_library()
+    assert lib.b200_gemm_by_ring(T * k, 2 * I, H, pkg.EPILOGUE_SWIGLU, E, T) == lib.b200_gemm_by_ring(T * k, H, I, pkg.EPILOGUE_NONE, E, T) == 1
+
+
+def test_many_experts_on_the_narrow_kernel(L, pkg):
+    """More tokens than the ring kernel's experts take, at most 8 rows per expert on average."""
+    T, E, k, H, I = 64, 32, 2, 1088, 64
+    lib = pkg.load_library()
+    assert lib.b200_gemm_kernel(T * k, 2 * I, H, pkg.EPILOGUE_SWIGLU, E, T, 0) == NARROW
+    assert not lib.b200_gemm_by_ring(T * k, 2 * I, H, pkg.EPILOGUE_SWIGLU, E, T)
+    moe_forward(L, T, E, k, H, I, True, "silu")

@@ -341,20 +341,43 @@ def test_generate_command(pkg, tmp_path):
     assert [[int(t) for t in x.split()] for x in r.stdout.splitlines()] == [greedy("mixed", p, 5) for p in prompts]
 
 
-@pytest.mark.parametrize("requests", [1, 8, 9, 16])
-@pytest.mark.parametrize("ff", [6144, 8192])
-def test_steps_whose_kernels_start_early_have_the_bits_of_steps_whose_kernels_do_not(pkg, monkeypatch, requests, ff):
+@pytest.mark.parametrize("requests", [8, 9, 16])
+def test_steps_whose_kernels_start_early_have_the_bits_of_steps_whose_kernels_do_not(pkg, monkeypatch, requests):
     """Layers wide enough for the GEMMs that walk over a large W, of one and two blocks of 8 rows, behind the latents' chain of
-    small kernels.  (6144: the last of a layer lets the next kernels in when it ends; 8192: at once.)"""
-    cfg = C.config([C.latent(16, 64, 64, 128, 768, 512, 0.0884, ff=ff), C.latent(16, 64, 64, 128, 768, 512, 0.0884, kv_from=0, ff=ff)],
+    small kernels."""
+    cfg = C.config([C.latent(16, 64, 64, 128, 768, 512, 0.0884, ff=6144), C.latent(16, 64, 64, 128, 768, 512, 0.0884, kv_from=0, ff=6144)],
                    width=2048, vocab=512)
-    if f"chained{ff}" not in C._models:
-        C._models[f"chained{ff}"] = C.O.random_model(cfg, 5)
+    if "chained" not in C._models:
+        C._models["chained"] = C.O.random_model(cfg, 5)
     prompts = [C.prompt(cfg, 70 + i, 40 + i) for i in range(requests)]
     got = []
     for early in ("0", "1"):
         monkeypatch.setenv("B200_PDL", early)
-        e, hb = engine_for(cfg, C._models[f"chained{ff}"], "bfloat16", pages=2 * requests, live=requests, max_extend=2048)
+        e, hb = engine_for(cfg, C._models["chained"], "bfloat16", pages=2 * requests, live=requests, max_extend=2048)
+        e.capture_graphs([requests])
+        live = [hb.open_request(100) for _ in prompts]
+        hb.extend(live, prompts).synchronize()
+        steps = []
+        for step in range(6):
+            hb.extend(live, [[int(p[step])] for p in prompts]).synchronize()
+            steps.append(e.token_logits(range(requests)))
+        got.append(torch.stack(steps))
+    assert torch.equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("ff,requests", [(6144, 1), (8192, 1), (8192, 8), (8192, 9), (8192, 16)])
+def test_steps_with_early_starts_and_a_wider_mlp_have_the_bits_of_steps_without(pkg, monkeypatch, ff, requests):
+    """The same with a single request, and with a last GEMM of a layer that lets the next kernels in at once (8192; 6144: when it ends)."""
+    cfg = C.config([C.latent(16, 64, 64, 128, 768, 512, 0.0884, ff=ff), C.latent(16, 64, 64, 128, 768, 512, 0.0884, kv_from=0, ff=ff)],
+                   width=2048, vocab=512)
+    if f"chained{ff}" not in C._models:
+        C._models[f"chained{ff}"] = C.O.random_model(cfg, 5)
+    model = C._models[f"chained{ff}"]
+    prompts = [C.prompt(cfg, 70 + i, 40 + i) for i in range(requests)]
+    got = []
+    for early in ("0", "1"):
+        monkeypatch.setenv("B200_PDL", early)
+        e, hb = engine_for(cfg, model, "bfloat16", pages=2 * requests, live=requests, max_extend=2048)
         e.capture_graphs([requests])
         live = [hb.open_request(100) for _ in prompts]
         hb.extend(live, prompts).synchronize()
