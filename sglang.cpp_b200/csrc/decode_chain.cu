@@ -647,6 +647,7 @@ decode_chain_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_consta
                 }
 
                 // ---- this CTA's exchange buffer is free again: arm it for the next unit, then tell the cluster ----
+                fence_proxy_async_smem();   // (read with ordinary loads, filled by the peers' copies: see mbar_release_stage)
                 bar_epilogue();
                 if (et == 0) {
                     int nq = q;
