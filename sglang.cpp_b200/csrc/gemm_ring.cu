@@ -350,10 +350,19 @@ RingParams ring_params(void* y, int N, int K, int epilogue, float act_limit, int
 //   8 x 28672 x 4096 with SwiGLU 41.1, 46.4;  9 rows of it 43.2, 46.4;  8 x 128256 x 4096 155, 167
 // Steps: Llama-3-8B, 1 request 2906 us against 3542, 4 requests 3025 against 3726, 8 requests 3097 against 3745; Saluzen, 12 requests 470
 // against 566, 16 requests 498 against 594.
+//
+// Where the registers' kernel would take the call it is ahead up to 8 rows while the ring's CTAs have one tile each and some a second one,
+// and its warps request their whole share of K at once (K up to 4096): 1 row / 8 rows, programmatic launches, the ring first
+//   3328 x 3840 6.9, 5.7 / 6.9, 6.2;  3584 x 3712 6.7, 5.8 / 6.8, 6.3;  3840 x 3328 6.2, 5.7 / 6.3, 6.2;  4096 x 3264 6.4, 5.7 / 6.6, 6.3
+//   4736 x 2688 (two tiles each) 6.2, 6.2 / 6.2, 6.4;  4800 x 2688 7.4, 8.8 / 7.5, 9.2;  3072 x 4352 8.1, 8.6 / 8.2, 9.0;  9 rows of 3328 x 3840 7.5, 9.0
+// Fewer tiles than SMs are no reason against the ring: 512 x 24576 14.1, 16.0 / 14.1, 16.8; 1024 x 12288 8.5, 10.2 / 8.5, 10.7;
+// 512 x 32768 17.5, 27.2 against the weight-streaming kernel.
 bool ring_gemm_takes(const void* x, const void* w, int M, int N, int K, int64_t ldx, int epilogue, bool narrow) {
     const int n_out = epilogue_is_gated(epilogue) ? N / 2 : N;
-    return M >= 1 && M <= 16 && K >= 2048 && static_cast<int64_t>(N) * K >= (narrow ? 12ll << 20 : 4ll << 20) && n_out % 8 == 0 && K % 64 == 0 && ldx % 8 == 0 &&
-           aligned16(x, w);
+    const int tiles = div_ceil(N, 16);
+    const bool uneven = M <= 8 && K <= 4096 && tiles > sm_count() && tiles < 2 * sm_count();
+    const bool large = narrow ? static_cast<int64_t>(N) * K >= 12ll << 20 && !uneven : static_cast<int64_t>(N) * K >= 4ll << 20;
+    return M >= 1 && M <= 16 && K >= 2048 && large && n_out % 8 == 0 && K % 64 == 0 && ldx % 8 == 0 && aligned16(x, w);
 }
 
 int launch_ring_gemm(void* y, const void* x, const void* w, const void* bias, int M, int N, int K, int64_t ldx, int epilogue, int* status,

@@ -65,6 +65,13 @@ def test_projections_by_the_ring_kernel(pkg, N, K, epilogue, ring, not_ring):
     assert all(lib.b200_gemm_kernel(r, N, K, epilogue, 0, 0, 0) in (NARROW, STREAM) for r in ring)
 
 
+@pytest.mark.parametrize("N,K", [(3072, 4096), (3328, 3840), (3584, 3584), (3840, 3328), (4096, 3264), (4608, 2752)])
+def test_tiles_that_go_round_the_ring_kernels_ctas_unevenly(pkg, N, K):
+    """Up to 8 rows the kernel from memory to registers is the faster one (with 9 rows it is not)."""
+    lib = pkg.load_library()
+    assert [lib.b200_gemm_by_ring(r, N, K, PLAIN, 0, 0) for r in (1, 8, 9, 16)] == [0, 0, 1, 1]
+
+
 def test_shapes_that_the_ring_kernel_does_not_take(pkg):
     lib = pkg.load_library()
     assert [lib.b200_gemm_by_ring(*a) for a in [(0, 4096, 4096, 0, 0, 0), (4, 4096, 4000, 0, 0, 0), (4, 4096, 4096, 99, 0, 0), (4, 4096, 4096, 0, 2, 0)]] == [0] * 4
