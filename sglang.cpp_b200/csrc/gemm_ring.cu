@@ -377,14 +377,26 @@ int launch_ring_gemm(void* y, const void* x, const void* w, const void* bias, in
 }
 
 // Of the calls that narrow_grouped_takes: many groups, and few enough rows that a group with all of them does not take more turns than
-// there.  Layers (us, this kernel against narrow_grouped_kernel; rows spread at random, and all tokens with the same experts):
-//   64 experts of 2 x 1024 x 2048, 4 per token    1 token 36, 43;   8 tokens 77, 86 and 35, 43;   32: 137, 147 and 52, 58;   48: 149, 166 and 70, 70
-//   128 of 2 x 768 x 2048, 8 per token            1 token 45, 60;   8: 115, 129 and 47, 65;   16: 161, 176 and 60, 67
-//   32 of 2 x 1024 x 2048, 2 per token            8: 49, 57 and 27, 31;   32: 83, 88 and 38, 39;   64: 92, 100, but 51, 49
-//   16 of 2 x 2048 x 1024, 4 per token            1 token 33, 31;   32: 77, 67 and 52, 46
-// Steps of 12 such layers (the first kind): 1 request 581 us against 648, 32 requests 2045 against 2264.
-bool ring_grouped_takes(const void* x, const void* w, int max_rows, int num_groups, int n_out, int K) {
-    return num_groups >= 32 && num_groups <= kMaxRingGroups && max_rows <= 48 && n_out % 8 == 0 && K % 64 == 0 && aligned16(x, w);
+// there.  A K of three whole stages and more hides what a tile costs beside its weights (the warps' sums meet, a stage fills only in part);
+// with a shorter one the kernel is ahead only of what a launch of CTAs for groups without rows costs there.  us that this kernel adds to
+// a layer in which narrow_grouped_kernel runs, and the layer with that (one projection at a time; rows spread at random, and all
+// tokens with the same experts, 4 per token unless stated):
+//   64 experts, 2 x 1024 x 2048   1 token -5.0 of 34;   8 -8.8 of 81, -5.8 of 35;   32 -16.3 of 144, -2.4 of 46;   48 -21.3 of 161, 1.3 of 52
+//   32 experts of it              1 token -1.5 of 25;   8 -6.2 of 64, -2.8 of 28;   32 -11.9 of 94, -1.1 of 41;    48 3.5 of 98, 5.3 of 44
+//   32 experts, 2 x 512 x 1536    1 token -0.8 of 20;   16 -3.4 of 45, -0.9 of 22;   32 2.4 of 48, -0.5 of 28
+//   64 experts, 1024 x 2048       8 tokens -2.6 of 77, -2.2 of 36;   32 -8.1 of 158, -0.1 of 45;   48 -9.2 of 181, 2.0 of 49
+//   64 experts, 2048 x 1024       1 token -2.2 of 34;   4 1.3 of 55, -2.8 of 33;   8 3.2 of 81, -3.7 of 35;   32 -1.1 of 144, -2.1 of 46
+//   64 experts, 2048 x 768        1 token -1.3 of 30;   8 4.0 of 69, -4.5 of 33;   32 6.2 of 123, -1.9 of 41
+//   32 experts, 2048 x 256        1 token 0.1 of 18;    8 1.8 of 31, -0.9 of 19;   32 11.7 of 43, 1.3 of 25
+//   128 experts, 2048 x 256       1 token -11 of 35;    8 -5.4 of 48, -13 of 38
+//   128 experts, 1536 x 1024      1 token -8.2 of 46;   8 2.5 of 85, -6.9 of 45;   16 -2.8 of 118, -4.1 of 44
+//   128 experts, 1024 x 512, 8 per token   4 tokens -1.1 of 39, -3.4 of 31;   16 1.2 of 66, -1.2 of 34;   48 1.9 of 93, 0.8 of 44
+//   128 experts, 512 x 1024       1 token -0.2 of 32;   4 1.7 of 34, -0.4 of 32;   32 1.5 of 79, -2.0 of 35
+bool ring_grouped_takes(const void* x, const void* w, int64_t total_rows, int max_rows, int num_groups, int n_out, int K, int epilogue) {
+    const int tiles = epilogue_is_gated(epilogue) ? div_ceil(n_out, 8) : div_ceil(n_out, 16);
+    const bool faster = K >= 3 * kChunk ? total_rows <= (tiles >= 96 ? 4ll : 3ll) * num_groups
+                                        : num_groups >= 64 && tiles >= 64 && total_rows * 4 <= num_groups;
+    return faster && num_groups >= 32 && num_groups <= kMaxRingGroups && max_rows <= 48 && n_out % 8 == 0 && K % 64 == 0 && aligned16(x, w);
 }
 
 int launch_ring_grouped(void* y, const void* x, const void* w, const int32_t* counts, const int32_t* offsets, int num_groups,

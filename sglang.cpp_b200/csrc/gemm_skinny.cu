@@ -816,7 +816,7 @@ constexpr int kGemmRing = 5;
 // many rows per group on average (prompts) are tensor-bound.
 static int grouped_kernel(const void* x, const void* w, int64_t total_rows, int max_rows, int num_groups, int n_out, int K, int epilogue) {
     if (narrow_grouped_takes(x, w, total_rows, max_rows, num_groups, n_out, K, epilogue))
-        return ring_grouped_takes(x, w, max_rows, num_groups, n_out, K) ? kGemmRing : B200_GEMM_NARROW;
+        return ring_grouped_takes(x, w, total_rows, max_rows, num_groups, n_out, K, epilogue) ? kGemmRing : B200_GEMM_NARROW;
     const bool tiles = total_rows >= static_cast<int64_t>(num_groups) * env_int("B200_GROUPED_TILE_MIN_ROWS", 128) && num_groups <= 256;
     return tiles ? B200_GEMM_TILE : B200_GEMM_STREAM;
 }

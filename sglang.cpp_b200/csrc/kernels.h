@@ -133,7 +133,7 @@ int launch_narrow_grouped(void* y, const void* x, const void* w, const int32_t* 
 bool ring_gemm_takes(const void* x, const void* w, int M, int N, int K, int64_t ldx, int epilogue, bool narrow);
 int launch_ring_gemm(void* y, const void* x, const void* w, const void* bias, int M, int N, int K, int64_t ldx, int epilogue, int* status,
                      cudaStream_t stream, float act_limit);
-bool ring_grouped_takes(const void* x, const void* w, int max_rows, int num_groups, int n_out, int K);
+bool ring_grouped_takes(const void* x, const void* w, int64_t total_rows, int max_rows, int num_groups, int n_out, int K, int epilogue);
 int launch_ring_grouped(void* y, const void* x, const void* w, const int32_t* counts, const int32_t* offsets, int num_groups,
                         int64_t total_rows, int N, int K, int epilogue, int* status, cudaStream_t stream, float act_limit);
 // The kernel (B200_GEMM_*) of launch_linear (groups 0) or launch_grouped_gemm with aligned operands and nothing fused but,

@@ -338,16 +338,20 @@ def test_few_rows_of_a_large_w_are_the_ring_kernels(pkg, M, N, K):
     assert pkg.load_library().b200_gemm_by_ring(M, N, K, pkg.EPILOGUE_NONE, 0, 0) == (K >= 2048)
 
 
-@pytest.mark.parametrize("T", [1, 8, 9, 17, 40])
-@pytest.mark.parametrize("E,k,H,I", [(33, 4, 192, 576), (64, 3, 576, 64), (256, 1, 64, 128)])
-def test_many_experts_of_few_rows_are_the_ring_kernels(pkg, T, E, k, H, I):
-    """What test_many_experts_of_few_rows runs on."""
+@pytest.mark.parametrize("T", [1, 8, 9, 16, 17, 33])
+@pytest.mark.parametrize("E,k,H,I,up,down", [(33, 3, 1600, 64, 99, 0), (32, 2, 64, 1600, 0, 96), (128, 2, 64, 512, 32, 0), (128, 2, 1024, 64, 0, 32)])
+@pytest.mark.parametrize("alike", [False, True])
+def test_experts_of_the_ring_kernel(L, pkg, T, E, k, H, I, up, down, alike):
+    """Rows of an expert below, at and above the 8 and 16 of one pass, K of a part of a stage, of whole ones and of three and a part; up to
+    `up` and `down` rows that projection is the ring kernel's."""
     lib = pkg.load_library()
-    assert lib.b200_gemm_by_ring(T * k, 2 * I, H, pkg.EPILOGUE_SWIGLU, E, T) == lib.b200_gemm_by_ring(T * k, H, I, pkg.EPILOGUE_NONE, E, T) == 1
+    assert lib.b200_gemm_by_ring(T * k, 2 * I, H, pkg.EPILOGUE_SWIGLU, E, T) == (T * k <= up)
+    assert lib.b200_gemm_by_ring(T * k, H, I, pkg.EPILOGUE_NONE, E, T) == (T * k <= down)
+    test_many_experts_of_few_rows(L, pkg, T, E, k, H, I, alike)
 
 
 def test_many_experts_on_the_narrow_kernel(L, pkg):
-    """More tokens than the ring kernel's experts take, at most 8 rows per expert on average."""
+    """A K that is too short for the ring kernel, at most 8 rows per expert on average."""
     T, E, k, H, I = 64, 32, 2, 1088, 64
     lib = pkg.load_library()
     assert lib.b200_gemm_kernel(T * k, 2 * I, H, pkg.EPILOGUE_SWIGLU, E, T, 0) == NARROW
