@@ -79,6 +79,7 @@ struct PrefillTc2Params {
     const int32_t* seq_lens;
     const int32_t* qo_indptr;
     int q_heads, kv_heads, group, batch;
+    int group_inverse;       // 65536 / group, rounded up: r / group = r * group_inverse >> 16 for r <= 128
     int blocks;              // of 2 x 128/G query tokens in the longest extension
     int kpc;  // keys of a page in a tile = min(page_size, 128)
     int whole_pages;       // KvMaps::page is there: pages and a cache of 8 slots and more (the map counts groups of 8)
@@ -131,9 +132,10 @@ attention_prefill_tc2_kernel(const __grid_constant__ KvMaps maps, const PrefillT
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     uint8_t* smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
-    const int G = p.group;         // (a power of two)
-    const int g_shift = __ffs(G) - 1;
-    const int QB = kTile >> g_shift;      // query tokens per tile
+    const int G = p.group;
+    auto token_of = [&](int r) { return r * p.group_inverse >> 16; };   // of a tile's row
+    auto head_of = [&](int r) { return r - token_of(r) * G; };
+    const int QB = token_of(kTile);       // query tokens per tile; rows behind them (3 or 5 heads ...) are the next tile's first ones again
     // Blocks of all requests and heads, the last (heaviest) ones of every prompt first: CTAs that start late are short.
     const int heads = p.kv_heads * p.batch;
     const int h = static_cast<int>(blockIdx.x) % heads % p.kv_heads;
@@ -270,8 +272,8 @@ attention_prefill_tc2_kernel(const __grid_constant__ KvMaps maps, const PrefillT
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
             const int r = (sw & 3) * 32 + i * 2 + (lane >> 4);
-            const int tok = t0 + tile * QB + (r >> g_shift);
-            const int head = h * G + (r & (G - 1));
+            const int tok = t0 + tile * QB + token_of(r);
+            const int head = h * G + head_of(r);
             v[i] = make_uint4(0, 0, 0, 0);
             if (tok < t_end)
                 v[i] = reinterpret_cast<const uint4*>(p.q + static_cast<int64_t>(q_begin + tok) * p.q_st +
@@ -382,8 +384,8 @@ attention_prefill_tc2_kernel(const __grid_constant__ KvMaps maps, const PrefillT
         const int tile = (warp >> 2) - 1;         // query tile of this warp
         const int qtr = warp & 3;                 // TMEM lane quarter this warp may read
         const int r = qtr * 32 + lane;            // query row = TMEM lane
-        const int tok = t0 + tile * QB + (r >> g_shift);
-        const int head = h * G + (r & (G - 1));
+        const int tok = t0 + tile * QB + token_of(r);
+        const int head = h * G + head_of(r);
         const int limit = min(pos0 + tok, len - 1);   // last visible key of this row
         const int oldest = WINDOW ? p.w.oldest(limit) : 0;   // keys before it are seen below keep_first only
         const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(qtr * 32) << 16);
@@ -545,12 +547,12 @@ attention_prefill_tc2_kernel(const __grid_constant__ KvMaps maps, const PrefillT
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
                 const int row2 = qtr * 32 + i * 2 + (lane >> 4);
-                const int tok2 = t0 + tile * QB + (row2 >> g_shift);
+                const int at2 = token_of(row2), tok2 = t0 + tile * QB + at2;
                 const uint32_t a = swz128(smem_base + kQOff + (tile * 2 + (lane >> 3 & 1)) * kAtomBytes + row2 * 128, lane & 7);
                 uint4 w;
                 asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w) : "r"(a) : "memory");
-                if (ok && tok2 < t_end)
-                    reinterpret_cast<uint4*>(p.out + (q_begin + tok2) * out_st + (h * G + (row2 & (G - 1))) * kD)[lane & 15] = w;
+                if (ok && at2 < QB && tok2 < t_end)
+                    reinterpret_cast<uint4*>(p.out + (q_begin + tok2) * out_st + (h * G + row2 - at2 * G) * kD)[lane & 15] = w;
             }
         }
     }
@@ -629,6 +631,7 @@ int launch_attention_prefill_tc2(void* out, const void* q, int64_t q_st, int64_t
     p.q_heads = q_heads;
     p.kv_heads = kv_heads;
     p.group = q_heads / kv_heads;
+    p.group_inverse = (65536 + p.group - 1) / p.group;
     p.batch = batch;
     p.kpc = page_size < kTile ? page_size : kTile;
     p.num_slots = num_slots;

@@ -705,6 +705,27 @@ def test_tokens_into_pinned_and_pageable_memory_and_reports_of_steps(pkg, nreq):
     e.close()
 
 
+@pytest.mark.parametrize("q_heads,kv_heads", [(6, 2), (5, 1), (6, 1), (14, 2)])
+def test_prefill_of_heads_that_do_not_fill_the_attention_tiles(pkg, q_heads, kv_heads):
+    """3, 5, 6 and 7 heads per KV head: 128 rows of a tile are whole tokens and a rest.  Two layers, so that every token counts; whole
+    prompts, and one behind what is cached."""
+    cfg = O.ModelConfig(2, 256, q_heads, kv_heads, 128, 512, 1024, 1e-6, 1e6, 512, True, True, True)
+    pr = Pair(pkg, cfg, 16)
+    rng = np.random.default_rng(q_heads)
+    prompts = [rng.integers(0, cfg.vocab_size, size=n).astype(np.int32) for n in (23, 200, 87)]
+    reqs = [pr.hb.add_request(p, 4) for p in prompts]
+    pr.host_tokens = {r.table_idx: list(p) + [0] * 8 for r, p in zip(reqs, prompts)}
+    pr.hb.allocate(reqs)
+    ob, pt = pr.oracle_batch(reqs, True)
+    want = pr.oracle.forward(ob, pr.kv, pt)
+    rows, lens, none = np.array([r.table_idx for r in reqs], np.int32), np.array([23, 200, 87], np.int32), np.full(3, -1, np.int32)
+    pr.hb.prefill(reqs).synchronize()
+    check_logits(pr.engine.logits(3), want, "prompts")
+    pr.engine.forward_batch(0, rows[1:], np.array([70, 30], np.int32), np.array([130, 57], np.int32), none[1:]).synchronize()
+    check_logits(pr.engine.logits(2), want[1:], "prompts behind cached tokens")
+    pr.engine.close()
+
+
 @pytest.mark.parametrize("nreq", [1, 5])
 def test_tokens_into_pinned_memory_that_holds_no_words(pkg, nreq):
     """Pinned, but at an address that a kernel's words may not have: a copy, as into other memory."""
