@@ -337,7 +337,9 @@ attention_prefill_tc2_kernel(const __grid_constant__ KvMaps maps, const PrefillT
                     tc_commit(smem_u32(&s_full[i]));
                 }
                 if (failed) break;
-                tc_commit(smem_u32(&empty[slot]));   // both tiles have read this K tile
+                // both tiles have read this K tile (a slot that is not filled again is not handed back: nobody would wait for that
+                // arrival, and it could still be under way when the block ends)
+                if (kt + kKSlots < ntiles) tc_commit(smem_u32(&empty[slot]));
                 if (++slot == kKSlots) {
                     slot = 0;
                     phase ^= 1;
@@ -371,7 +373,7 @@ attention_prefill_tc2_kernel(const __grid_constant__ KvMaps maps, const PrefillT
                     tc_commit(smem_u32(&pv_done[i]));
                 }
                 if (failed) break;
-                tc_commit(smem_u32(&empty[slot]));   // both tiles have read this V tile
+                if (kt + kVSlots < ntiles) tc_commit(smem_u32(&empty[slot]));   // both tiles have read this V tile
                 if (++slot == kSlots) {
                     slot = kKSlots;
                     phase ^= 1;
