@@ -39,6 +39,7 @@
 //     S and P V from two threads                                           214 / 233 / 65.7 / 14.5
 //     queries and outputs by half warps per row, first K tile early        203 / 227 / 57.6 / 12.4
 //     unmasked tiles without tests, one wait per tile for P V              188 / 215 / 54.1 / 12.3
+// A ring of slots each for K and V and any number of heads, one launch at a time between two events: 195 / 221 / 61 / 14.3.
 // Queries are the LAST extend_len positions of the request, so tiles left of the diagonal need no mask
 // and tiles right of it are never loaded.
 //

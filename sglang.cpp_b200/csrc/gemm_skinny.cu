@@ -812,8 +812,8 @@ int launch_skinny_gemm(void* y, const void* x, const void* w, const void* bias, 
 // What b200_gemm_kernel calls by the name of the kernel that it stands in for.
 constexpr int kGemmRing = 5;
 
-// The kernel (B200_GEMM_*, kGemmRing; B200_GEMM_TILE for pairs of CTAs as well) of the expert projections: a handful of rows per group have two,
-// many rows per group on average (prompts) are tensor-bound.
+// The kernel (B200_GEMM_*, kGemmRing; B200_GEMM_TILE for pairs of CTAs as well) of the expert projections: a handful of rows per group
+// have two, many rows per group on average (prompts) are tensor-bound.
 static int grouped_kernel(const void* x, const void* w, int64_t total_rows, int max_rows, int num_groups, int n_out, int K, int epilogue) {
     if (narrow_grouped_takes(x, w, total_rows, max_rows, num_groups, n_out, K, epilogue))
         return ring_grouped_takes(x, w, total_rows, max_rows, num_groups, n_out, K, epilogue) ? kGemmRing : B200_GEMM_NARROW;
@@ -966,8 +966,8 @@ static bool linear_on_tiles(const void* y, int M, int N, int K, int epilogue, bo
     return tile_gemm_us(M, N, K, epilogue) < 0.9f * skinny_gemm_us(M, N, K, epilogue);
 }
 
-// The kernel (B200_GEMM_*, kGemmRing; B200_GEMM_TILE for pairs of CTAs as well) of a projection.  narrow: the kernels of a handful of rows may take it; fused: something rides in the
-// weight-streaming kernel; normed: the norm of x rides in the projection.
+// The kernel (B200_GEMM_*, kGemmRing; B200_GEMM_TILE for pairs of CTAs as well) of a projection.  narrow: the kernels of a handful of
+// rows may take it; fused: something rides in the weight-streaming kernel; normed: the norm of x rides in the projection.
 static int linear_kernel(const void* y, const void* x, const void* w, int M, int N, int K, int64_t ldx, int epilogue, bool narrow, bool fused,
                          bool normed) {
     if (narrow && !fused) {   // weights straight into registers, or of a large W through a ring
