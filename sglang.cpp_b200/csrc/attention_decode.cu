@@ -257,7 +257,7 @@ attention_decode_kernel(const __grid_constant__ CUtensorMap tmap_k,
             for (int st = it.s_begin; st < it.s_end; ++st, ++it_count) {
                 const uint32_t slot = it_count % kStages;
                 const uint32_t parity = ((it_count / kStages) & 1u) ^ 1u;
-                if (!mbar_wait_bounded(smem_u32(&empty_bar[slot]), parity, p.status, 201)) {
+                if (!mbar_wait_warp(smem_u32(&empty_bar[slot]), parity, p.status, 201)) {
                     failed = true;
                     break;
                 }

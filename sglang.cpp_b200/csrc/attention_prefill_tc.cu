@@ -196,7 +196,7 @@ attention_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k,
 #pragma unroll
             for (int kv = 0; kv < 2; ++kv) {   // 0: K tile, 1: V tile
                 if (kt >= kStages &&
-                    !mbar_wait_bounded(smem_u32(kv == 0 ? &k_empty[slot] : &v_empty[slot]), parity, p.status, 311)) {
+                    !mbar_wait_warp(smem_u32(kv == 0 ? &k_empty[slot] : &v_empty[slot]), parity, p.status, 311)) {
                     failed = true;
                     break;
                 }

@@ -39,7 +39,8 @@
 //     S and P V from two threads                                           214 / 233 / 65.7 / 14.5
 //     queries and outputs by half warps per row, first K tile early        203 / 227 / 57.6 / 12.4
 //     unmasked tiles without tests, one wait per tile for P V              188 / 215 / 54.1 / 12.3
-// A ring of slots each for K and V and any number of heads, one launch at a time between two events: 195 / 221 / 61 / 14.3.
+// A ring of slots each for K and V, any number of heads, waits that lanes agree on; one launch at a time between two events:
+// 198 / 223 / 61 / 14.3.
 // Queries are the LAST extend_len positions of the request, so tiles left of the diagonal need no mask
 // and tiles right of it are never loaded.
 //
@@ -195,12 +196,14 @@ attention_prefill_tc2_kernel(const __grid_constant__ KvMaps maps, const PrefillT
             next[i] = copy < n ? pt_row[k0 + copy * p.kpc] : 0;
         }
     };
-    // K (kv = 0) or V tile kt into `slot`.  A tile whose pages are consecutive slots is fetched with one copy; so
-    // is a page, unless it is smaller than a group or starts inside one.
-    auto load_tile = [&](int kv, int kt, uint32_t slot) {
-        const int ncopies = copies_of(kt);
-        bool whole = kv_end - first_key(kt) >= kTile && p.whole_tile_boxes, groups = p.whole_pages;
-        int sl[4];
+    // How tile kt is copied: a tile whose pages are consecutive slots with one copy; so is a page, unless it is smaller than a group or
+    // starts inside one.  (Before its slot is free.)
+    int sl[4], ncopies = 0;
+    bool whole = false, groups = false;
+    auto plan_tile = [&](int kt) {
+        ncopies = copies_of(kt);
+        whole = kv_end - first_key(kt) >= kTile && p.whole_tile_boxes;
+        groups = p.whole_pages;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             sl[i] = next[i];
@@ -219,12 +222,15 @@ attention_prefill_tc2_kernel(const __grid_constant__ KvMaps maps, const PrefillT
         }
         whole = __all_sync(0xffffffffu, whole);
         groups = __all_sync(0xffffffffu, groups);
+    };
+    // That K (kv = 0) or V tile into `slot`.
+    auto load_tile = [&](int kv, uint32_t slot) {
         const uint32_t bar = smem_u32(&full[slot]);
         const uint32_t base = smem_base + kKVOff + slot * kSlotBytes;
         if (lane == 0) mbar_arrive_expect_tx(bar, static_cast<uint32_t>(ncopies * p.kpc) * kD * 2u);
         __syncwarp();
         if (whole) {
-            if (lane == 0) tma_load_5d(base, &maps.tile[kv], 0, 0, 0, first >> 3, h, bar);
+            if (lane == 0) tma_load_5d(base, &maps.tile[kv], 0, 0, 0, sl[0] >> 3, h, bar);
         } else {
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -245,7 +251,8 @@ attention_prefill_tc2_kernel(const __grid_constant__ KvMaps maps, const PrefillT
     };
     if (warp == 0 || warp == 2) fetch_slots(0);
     if (warp == 0) {   // the first K tile is under way while the others fetch the queries (this warp has made the barriers)
-        load_tile(0, 0, 0);
+        plan_tile(0);
+        load_tile(0, 0);
         if (ntiles > 1) fetch_slots(1);
     }
 
@@ -301,9 +308,10 @@ attention_prefill_tc2_kernel(const __grid_constant__ KvMaps maps, const PrefillT
         const uint32_t ring = kv == 0 ? 0 : kKSlots, ring_end = kv == 0 ? kKSlots : kSlots;
         uint32_t slot = kv == 0 ? 1 : kKSlots, phase = 1;   // (the first waits are for slots that nobody has used)
         for (int kt = kv == 0 ? 1 : 0; kt < ntiles; ++kt) {
-            if (!mbar_wait_mostly_ready(smem_u32(&empty[slot]), phase, p.status, 321)) break;
-            load_tile(kv, kt, slot);
+            plan_tile(kt);
             if (kt + 1 < ntiles) fetch_slots(kt + 1);
+            if (!__all_sync(0xffffffffu, mbar_wait_mostly_ready(smem_u32(&empty[slot]), phase, p.status, 321))) break;   // (see mbar_wait_warp)
+            load_tile(kv, slot);
             if (++slot == ring_end) {
                 slot = ring;
                 phase ^= 1;

@@ -246,6 +246,12 @@ __device__ __forceinline__ bool mbar_wait_mostly_ready(uint32_t bar, uint32_t pa
     return mbar_wait_bounded(bar, parity, status, site);
 }
 
+// The first of them for a whole warp whose lanes go on together (votes, shuffles, tcgen05.ld): a wait that has run out has run out for
+// all.  Every lane reads the timer by itself, and lanes that stop alone would leave the others at their next vote for good.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, int* status, int site) {
+    return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, status, site)) != 0;
+}
+
 // ---- TMA (tiled tensor copies, never multicast) -----------------------------
 
 __device__ __forceinline__ void tma_prefetch_desc(const void* tmap) {

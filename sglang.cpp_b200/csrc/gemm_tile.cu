@@ -305,7 +305,7 @@ tile_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
             const TileAt at = locate(t);
             const int acc = tcount & 1;
             const uint32_t par = static_cast<uint32_t>(tcount >> 1) & 1u;
-            if (!mbar_wait_bounded(smem_u32(&acc_full_bar[acc]), par, p.status, 114)) {
+            if (!mbar_wait_warp(smem_u32(&acc_full_bar[acc]), par, p.status, 114)) {
                 failed = true;
                 break;
             }
@@ -508,7 +508,7 @@ pair_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
             const TileAt at = locate(t);
             const int acc = tcount & 1;
             const uint32_t par = static_cast<uint32_t>(tcount >> 1) & 1u;
-            if (!mbar_wait_bounded(smem_u32(&acc_full_bar[acc]), par, p.status, 124)) {
+            if (!mbar_wait_warp(smem_u32(&acc_full_bar[acc]), par, p.status, 124)) {
                 failed = true;
                 break;
             }
