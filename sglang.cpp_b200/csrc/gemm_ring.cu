@@ -25,7 +25,7 @@ namespace {
 constexpr int kChunk = 512;                        // columns per stage, 64 per warp
 constexpr uint32_t kWBytes = 16 * kChunk * 2, kXBytes = 8 * kChunk * 2;   // of a stage, x per block of 8 tokens
 constexpr int kStages = 6;
-constexpr int kWideStages = 4;                     // GROUPED, where some group has more than 8 rows
+constexpr int kWideStages = 4;                     // GROUPED, where many groups have more than 8 rows
 constexpr uint32_t ring_bytes(int blocks) { return kStages * (kWBytes + blocks * kXBytes); }
 static_assert(kWideStages * (kWBytes + 2 * kXBytes) <= ring_bytes(1), "");
 constexpr int kWarps = 8;                          // that multiply; one more requests
@@ -231,11 +231,22 @@ ring_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     if (GROUPED) {
         pdl_wait_prior();   // (the group table comes from the kernel before this one)
         if (warp == 0) {
-            int most = 0;
-            for (int g = lane; g < p.groups; g += 32) most = max(most, p.counts[g]);
+            // 16 rows per pass where that saves a third of the passes.  (Where one expert with more than 8 rows was enough for it, all the
+            // others paid: 64 experts of 2 x 1024 x 2048, 4 per token, a quarter of 32 tokens with the same experts 144.5 us per layer
+            // against 127.6, all of them 44.7 and 45.2; steps of 12 such layers, 24 requests of a batch of 32 2283 us against 2087.)
+            int narrow_passes = 0, wide_passes = 0;
+            for (int g = lane; g < p.groups; g += 32) {
+                const int rows = max(p.counts[g], 0);
+                narrow_passes += (rows + 7) / 8;
+                wide_passes += (rows + 15) / 16;
+            }
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, o));
-            const int width = most > 8 ? 16 : 8;
+            for (int o = 16; o > 0; o >>= 1) {
+                narrow_passes += __shfl_xor_sync(0xffffffffu, narrow_passes, o);
+                wide_passes += __shfl_xor_sync(0xffffffffu, wide_passes, o);
+            }
+            const bool wide = 2 * narrow_passes >= 3 * wide_passes;
+            const int width = wide ? 16 : 8;
             int total = 0;
             for (int base = 0; base < p.groups; base += 32) {
                 const int g = base + lane;
@@ -252,7 +263,7 @@ ring_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
             }
             if (lane == 0) {
                 s.passes = total;
-                s.wide = most > 8;
+                s.wide = wide;
             }
         }
     }
@@ -377,25 +388,35 @@ int launch_ring_gemm(void* y, const void* x, const void* w, const void* bias, in
 }
 
 // Of the calls that narrow_grouped_takes: many groups, and few enough rows that a group with all of them does not take more turns than
-// there.  A K of three whole stages and more hides what a tile costs beside its weights (the warps' sums meet, a stage fills only in part);
-// with a shorter one the kernel is ahead only of what a launch of CTAs for groups without rows costs there.  us that this kernel adds to
-// a layer in which narrow_grouped_kernel runs, and the layer with that (one projection at a time; rows spread at random, and all
-// tokens with the same experts, 4 per token unless stated):
-//   64 experts, 2 x 1024 x 2048   1 token -5.0 of 34;   8 -8.8 of 81, -5.8 of 35;   32 -16.3 of 144, -2.4 of 46;   48 -21.3 of 161, 1.3 of 52
-//   32 experts of it              1 token -1.5 of 25;   8 -6.2 of 64, -2.8 of 28;   32 -11.9 of 94, -1.1 of 41;    48 3.5 of 98, 5.3 of 44
-//   32 experts, 2 x 512 x 1536    1 token -0.8 of 20;   16 -3.4 of 45, -0.9 of 22;   32 2.4 of 48, -0.5 of 28
-//   64 experts, 1024 x 2048       8 tokens -2.6 of 77, -2.2 of 36;   32 -8.1 of 158, -0.1 of 45;   48 -9.2 of 181, 2.0 of 49
-//   64 experts, 2048 x 1024       1 token -2.2 of 34;   4 1.3 of 55, -2.8 of 33;   8 3.2 of 81, -3.7 of 35;   32 -1.1 of 144, -2.1 of 46
-//   64 experts, 2048 x 768        1 token -1.3 of 30;   8 4.0 of 69, -4.5 of 33;   32 6.2 of 123, -1.9 of 41
-//   32 experts, 2048 x 256        1 token 0.1 of 18;    8 1.8 of 31, -0.9 of 19;   32 11.7 of 43, 1.3 of 25
-//   128 experts, 2048 x 256       1 token -11 of 35;    8 -5.4 of 48, -13 of 38
-//   128 experts, 1536 x 1024      1 token -8.2 of 46;   8 2.5 of 85, -6.9 of 45;   16 -2.8 of 118, -4.1 of 44
-//   128 experts, 1024 x 512, 8 per token   4 tokens -1.1 of 39, -3.4 of 31;   16 1.2 of 66, -1.2 of 34;   48 1.9 of 93, 0.8 of 44
-//   128 experts, 512 x 1024       1 token -0.2 of 32;   4 1.7 of 34, -0.4 of 32;   32 1.5 of 79, -2.0 of 35
+// there.  A K of three whole stages and more hides what a tile costs beside its weights (the warps' sums meet, a stage fills only in
+// part), one of two does where there are many tiles; with a shorter one the kernel is ahead only of what a launch of CTAs for groups without
+// rows costs there.  us that this kernel adds to a layer in which narrow_grouped_kernel runs, and the layer with that (one projection
+// at a time; rows spread at random, and all tokens with the same experts, 4 per token unless stated):
+//   64 experts, 2 x 1024 x 2048   1 token -6.1 of 36;   8 -8.8 of 82, -5.4 of 35;   24 -15.4 of 137, -1.4 of 42;
+//       32 -15.3 of 147, -3.1 of 47;   48 -17.4 of 161, +0.1 of 53
+//   32 experts of it             1 token -1.1 of 26;   8 -3.3 of 61, -2.9 of 28;   24 -9.7 of 88, +2.2 of 37;   32 -8.9 of 92, -1.1 of 42;
+//       48 -8.0 of 98, +4.2 of 49
+//   32 experts, 2 x 512 x 1536   1 token -0.3 of 19;   16 -2.0 of 41, -0.1 of 22;   24 -2.3 of 47, +0.1 of 26;   32 -2.2 of 47, +0.0 of 27
+//   64 experts, 1024 x 2048      1 token -0.2 of 34;   8 -1.1 of 73, -3.7 of 38;   32 -9.1 of 160, +0.7 of 43;   48 -12.1 of 183, +1.0 of 50
+//   64 experts, 2048 x 1024      1 token -3.1 of 36;   8 +3.1 of 82, -3.9 of 35;   16 +1.8 of 109, -5.2 of 42;   32 +1.0 of 147, -1.4 of 47;
+//       48 -0.8 of 161, +2.2 of 53
+//   32 experts of it             1 token -0.1 of 26;   8 +2.2 of 61, -1.7 of 28;   32 +0.3 of 92, -0.3 of 42;   48 +1.4 of 98, +3.0 of 49
+//   64 experts, 2048 x 768       1 token -2.2 of 30;   8 +3.1 of 68, -4.0 of 32;   32 +6.6 of 112, -0.5 of 42
+//   32 experts, 2048 x 256       1 token -1.1 of 19;   8 +1.2 of 30, +0.1 of 17;   32 +1.3 of 43, +0.5 of 27
+//   128 experts, 2048 x 256      1 token -11.4 of 34;   8 -4.8 of 47, -13.1 of 38
+//   128 experts, 1536 x 1024     1 token -6.5 of 45;   8 +2.3 of 84, -9.0 of 47;   16 -0.9 of 114, -7.2 of 50
+//   128 experts, 1024 x 512, 8 per token   4 tokens -1.0 of 38, -3.0 of 30;   16 +0.5 of 66, -1.4 of 30;   48 +2.4 of 94, -0.8 of 49
+//   128 experts, 512 x 1024      1 token +0.2 of 31;   4 +0.5 of 34, -0.1 of 32;   32 +1.2 of 78, -2.6 of 34
+// Steps of 12 layers of 64 experts of 2 x 1024 x 2048, gate and up / down as well: 16 requests 1671, 1648 us; 32 2122, 2092; 8 1218, 1214.
 bool ring_grouped_takes(const void* x, const void* w, int64_t total_rows, int max_rows, int num_groups, int n_out, int K, int epilogue) {
     const int tiles = epilogue_is_gated(epilogue) ? div_ceil(n_out, 8) : div_ceil(n_out, 16);
-    const bool faster = K >= 3 * kChunk ? total_rows <= (tiles >= 96 ? 4ll : 3ll) * num_groups
-                                        : num_groups >= 64 && tiles >= 64 && total_rows * 4 <= num_groups;
+    bool faster;
+    if (K >= 3 * kChunk)
+        faster = total_rows <= (tiles >= 96 ? 4ll : 3ll) * num_groups;
+    else if (K >= 2 * kChunk && tiles >= 128 && num_groups >= 64)
+        faster = total_rows <= 3ll * num_groups;
+    else
+        faster = num_groups >= 64 && tiles >= 64 && total_rows * 4 <= num_groups;
     return faster && num_groups >= 32 && num_groups <= kMaxRingGroups && max_rows <= 48 && n_out % 8 == 0 && K % 64 == 0 && aligned16(x, w);
 }
 

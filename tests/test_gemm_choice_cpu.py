@@ -80,8 +80,9 @@ def test_shapes_that_the_ring_kernel_does_not_take(pkg):
 @pytest.mark.parametrize("experts,per_token,N,K,epilogue,ring,not_ring", [
     (64, 4, 2048, 2048, SWIGLU, (1, 8, 32, 48), (49, 64)), (32, 4, 2048, 2048, SWIGLU, (1, 8, 32), (33, 48)), (32, 4, 1024, 1536, SWIGLU, (1, 24), (25, 32)),
     (64, 4, 1024, 2048, PLAIN, (1, 32, 48), (49,)), (31, 2, 2048, 2048, SWIGLU, (), (1, 32)), (128, 8, 1536, 2048, SWIGLU, (1, 8, 16), (64,)),
-    # short K: only a launch of CTAs for groups without rows is behind
-    (32, 4, 2048, 256, PLAIN, (), (1, 8, 32)), (64, 4, 2048, 1024, PLAIN, (1, 4), (5, 8, 32)), (64, 6, 1024, 512, SWIGLU, (1, 2), (3, 8, 32)),
+    # short K: many tiles of two stages; else only a launch of CTAs for groups without rows is behind
+    (32, 4, 2048, 256, PLAIN, (), (1, 8, 32)), (64, 4, 2048, 1024, PLAIN, (1, 8, 32, 48), (49,)), (32, 4, 2048, 1024, PLAIN, (), (1, 8, 32)), (64, 4, 2032, 1024, PLAIN, (1, 4), (5, 32)),
+    (64, 6, 1024, 512, SWIGLU, (1, 2), (3, 8, 32)),
     (64, 8, 1024, 1024, SWIGLU, (1, 2), (3, 24, 48)), (128, 4, 2048, 256, PLAIN, (1, 8), (9, 16)), (128, 4, 512, 1024, PLAIN, (), (1, 4, 32)), (256, 8, 256, 128, SWIGLU, (), (1, 8)),
 ])
 def test_experts_by_the_ring_kernel(pkg, experts, per_token, N, K, epilogue, ring, not_ring):
